@@ -37,44 +37,12 @@ struct LdSplit {
     }
 };
 
-// value of component c of f at (i,j,k) shifted by s along direction d:
-// periodic axes wrap, y walls mirror with the field's ghost formulas
-template <typename P>
-__device__ __forceinline__ double at(const P &f, const Geo &g, int c, int i, int j, int k, int d, int s)
-{
-    if (d == 0) {
-        i = wrapi(i + s, g.N0);
-    } else if (d == 2) {
-        k = wrapi(k + s, g.N2);
-    } else {
-        const int jj = j + s;
-        if (f.wl.on && (jj < 0 || jj >= g.N1)) {
-            const int side = jj < 0 ? 0 : 1;
-            const int l = side == 0 ? -jj : jj - (g.N1 - 1);
-            const int jm = side == 0 ? l : (g.N1 - 1) - l;
-            return wall_ghost(f.wl, side, c, l, f(c, (long long)i * g.N12 + (long long)jm * g.N2 + k));
-        }
-        j = f.wl.on ? jj : wrapi(jj, g.N1);
-    }
-    return f(c, (long long)i * g.N12 + (long long)j * g.N2 + k);
-}
-
 __device__ __forceinline__ void pt_index(const Geo &g, long long t, int &i, int &j, int &k)
 {
     k = (int)(t % g.N2);
     long long r = t / g.N2;
     j = (int)(r % g.N1);
     i = (int)(r / g.N1);
-}
-
-// first derivative along d of component c with weights a (already metric-scaled)
-template <int H, typename P>
-__device__ __forceinline__ double dd1(const P &f, const Geo &g, int c, int i, int j, int k, int d, const double *a)
-{
-    double r = 0.0;
-#pragma unroll
-    for (int l = 0; l < H; l++) r = fma(a[l], at(f, g, c, i, j, k, d, l + 1) - at(f, g, c, i, j, k, d, -l - 1), r);
-    return r;
 }
 
 __global__ void k_scale(Geo g, int ny, cuDoubleComplex *__restrict__ spec, const double *__restrict__ kx2,
@@ -323,247 +291,6 @@ __global__ void __launch_bounds__(256) k_maxabs_chunks(long long n, const double
     for (long long t = b + threadIdx.x; t < e; t += blockDim.x) m = fmax(m, fabs(s[t]));
     m = block_reduce_max(m, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = m;
-}
-
-// --------------------------------------------------------------- operators --
-// Simple one-thread-per-node kernels for the drop-in ex:: entry points.
-
-template <int H>
-__global__ void k_op_grad_s(Geo g, Walls<double> wa, Coef<double> co, const double *__restrict__ ia, const double *__restrict__ s,
-                            double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 S{s, g.N3, wa};
-    double az[H];
-#pragma unroll
-    for (int l = 0; l < H; l++) az[l] = co.a[2][l] * ia[k];
-    out[t] = dd1<H>(S, g, 0, i, j, k, 0, co.a[0]);
-    out[g.N3 + t] = dd1<H>(S, g, 0, i, j, k, 1, co.a[1]);
-    out[2 * g.N3 + t] = dd1<H>(S, g, 0, i, j, k, 2, az);
-}
-
-// ex::grad(Field<vector>) keeps the reference's stencil c_l/(l+1)/delta*(f(+l) - f(-1-l)) (grad.cpp:82-94)
-template <int H>
-__global__ void k_op_grad_v(Geo g, Walls<double> wa, Coef<double> co, const double *__restrict__ ia, const double *__restrict__ U,
-                            double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 F{U, g.N3, wa};
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            double r = 0.0;
-#pragma unroll
-            for (int l = 0; l < H; l++) {
-                double w = 2.0 * co.a[d][l];  // c_l/(l+1)/delta
-                if (d == 2) w *= ia[k];
-                r = fma(w, at(F, g, c, i, j, k, d, l) - at(F, g, c, i, j, k, d, -1 - l), r);
-            }
-            out[(long long)(3 * c + d) * g.N3 + t] = r;
-        }
-}
-
-// ex::curl = antisymmetric part of ex::grad(vector) (src/ex/curl/curl.cpp:44-50)
-template <int H>
-__global__ void k_op_curl(Geo g, Walls<double> wa, Coef<double> co, const double *__restrict__ ia, const double *__restrict__ U,
-                          double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 F{U, g.N3, wa};
-    auto gv = [&](int c, int d) {
-        double r = 0.0;
-#pragma unroll
-        for (int l = 0; l < H; l++) {
-            double w = 2.0 * co.a[d][l];
-            if (d == 2) w *= ia[k];
-            r = fma(w, at(F, g, c, i, j, k, d, l) - at(F, g, c, i, j, k, d, -1 - l), r);
-        }
-        return r;
-    };
-    out[t] = gv(2, 1) - gv(1, 2);
-    out[g.N3 + t] = gv(0, 2) - gv(2, 0);
-    out[2 * g.N3 + t] = gv(1, 0) - gv(0, 1);
-}
-
-template <int H>
-__global__ void k_op_div_v(Geo g, Walls<double> wa, Coef<double> co, const double *__restrict__ ia, const double *__restrict__ U,
-                           double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 F{U, g.N3, wa};
-    double az[H];
-#pragma unroll
-    for (int l = 0; l < H; l++) az[l] = co.a[2][l] * ia[k];
-    out[t] = dd1<H>(F, g, 0, i, j, k, 0, co.a[0]) + dd1<H>(F, g, 1, i, j, k, 1, co.a[1])
-             + dd1<H>(F, g, 2, i, j, k, 2, az);
-}
-
-// skew div(U, f), f with nc components (src/ex/div/div.hxx:84-172)
-template <int H>
-__global__ void k_op_div_vf(Geo g, Walls<double> wa, Walls<double> wb, Coef<double> co, const double *__restrict__ ia, const double *__restrict__ U,
-                            const double *__restrict__ f, int nc, double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 V{U, g.N3, wa}, F{f, g.N3, wb};
-    double a[3][H];
-#pragma unroll
-    for (int l = 0; l < H; l++) {
-        a[0][l] = co.a[0][l];
-        a[1][l] = co.a[1][l];
-        a[2][l] = co.a[2][l] * ia[k];
-    }
-    double divU = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; d++) divU += dd1<H>(V, g, d, i, j, k, d, a[d]);
-    for (int c = 0; c < nc; c++) {
-        const double f0 = F(c, t);
-        double acc = f0 * divU;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            double dq = 0.0;
-#pragma unroll
-            for (int l = 0; l < H; l++)
-                dq = fma(a[d][l],
-                         at(V, g, d, i, j, k, d, l + 1) * at(F, g, c, i, j, k, d, l + 1)
-                             - at(V, g, d, i, j, k, d, -l - 1) * at(F, g, c, i, j, k, d, -l - 1),
-                         dq);
-            acc += dq + V(d, t) * dd1<H>(F, g, c, i, j, k, d, a[d]);
-        }
-        out[(long long)c * g.N3 + t] = 0.5 * acc;
-    }
-}
-
-// laplacian(nu, f) with the stretched-z term (src/ex/laplacian/laplacian.hxx:130-191)
-template <int H>
-__global__ void k_op_lap(Geo g, Walls<double> wa, Coef<double> co, const double *__restrict__ ia, const double *__restrict__ corr2,
-                         double nu, const double *__restrict__ f, int nc, double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 F{f, g.N3, wa};
-    const double i2 = ia[k] * ia[k];
-    for (int c = 0; c < nc; c++) {
-        const double f0 = F(c, t);
-        double r = 0.0;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const double m = (d == 2) ? i2 : 1.0;
-            double s = 0.0;
-#pragma unroll
-            for (int l = 0; l < H; l++)
-                s = fma(co.b[d][l] * m, at(F, g, c, i, j, k, d, l + 1) + at(F, g, c, i, j, k, d, -l - 1), s);
-            r += fma(-co.b2[d] * m, f0, s);
-        }
-        double az[H];
-#pragma unroll
-        for (int l = 0; l < H; l++) az[l] = co.a[2][l] * ia[k];
-        const double dz = dd1<H>(F, g, c, i, j, k, 2, az);
-        out[(long long)c * g.N3 + t] = nu * fma(-corr2[k], dz, r);
-    }
-}
-
-// ex::div(Field<tensor>) (src/ex/div/div.hxx:258-285) and ex::div(Field<symmTensor>)
-// (div.hxx:222-255; storage xx xy xz yy yz zz): out_c = sum_d D_d T[c*3+d],
-// without the z metric, as in the reference
-template <int H>
-__global__ void k_op_div_t(Geo g, Walls<double> wa, Coef<double> co, const double *__restrict__ T, int symm,
-                           double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 F{T, g.N3, wa};
-    const int S[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-    for (int c = 0; c < 3; c++) {
-        double r = 0.0;
-#pragma unroll
-        for (int d = 0; d < 3; d++) r += dd1<H>(F, g, symm ? S[c * 3 + d] : c * 3 + d, i, j, k, d, co.a[d]);
-        out[(long long)c * g.N3 + t] = r;
-    }
-}
-
-// ex::div(Field<scalar> s, Field<tensor> T) (div.hxx:173-207): sum_d D_d (s T[c*3+d])
-template <int H>
-__global__ void k_op_div_st(Geo g, Walls<double> wa, Walls<double> wb, Coef<double> co, const double *__restrict__ s,
-                            const double *__restrict__ T, double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 Sf{s, g.N3, wa}, F{T, g.N3, wb};
-    for (int c = 0; c < 3; c++) {
-        double r = 0.0;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            double q = 0.0;
-#pragma unroll
-            for (int l = 0; l < H; l++)
-                q = fma(co.a[d][l],
-                        at(Sf, g, 0, i, j, k, d, l + 1) * at(F, g, c * 3 + d, i, j, k, d, l + 1)
-                            - at(Sf, g, 0, i, j, k, d, -l - 1) * at(F, g, c * 3 + d, i, j, k, d, -l - 1),
-                        q);
-            r += q;
-        }
-        out[(long long)c * g.N3 + t] = r;
-    }
-}
-
-// ex::laplacian(Field<scalar> nu, Field<T>) (src/ex/laplacian/laplacian.hxx:64-127):
-// the + neighbour at 1+l weighted by nu at offset l, the - neighbour at -1-l
-// by nu at -1-l, both against the centre; z terms over dzdxi^2 and the
-// stretched-z term -nu(0) D_z f d2zdxi2/dzdxi^3
-template <int H>
-__global__ void k_op_lap_f(Geo g, Walls<double> wa, Walls<double> wb, Coef<double> co, const double *__restrict__ ia,
-                           const double *__restrict__ corr2, const double *__restrict__ nu, const double *__restrict__ f,
-                           int nc, double *__restrict__ out)
-{
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= g.N3) return;
-    int i, j, k;
-    pt_index(g, t, i, j, k);
-    Ld64 NU{nu, g.N3, wa}, F{f, g.N3, wb};
-    const double i2 = ia[k] * ia[k];
-    double az[H];
-#pragma unroll
-    for (int l = 0; l < H; l++) az[l] = co.a[2][l] * ia[k];
-    const double nu0 = NU(0, t);
-    for (int c = 0; c < nc; c++) {
-        const double f0 = F(c, t);
-        double r = 0.0;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const double m = (d == 2) ? i2 : 1.0;
-#pragma unroll
-            for (int l = 0; l < H; l++) {
-                const double np = l == 0 ? nu0 : at(NU, g, 0, i, j, k, d, l);
-                const double nm = at(NU, g, 0, i, j, k, d, -l - 1);
-                const double fp = at(F, g, c, i, j, k, d, l + 1), fm = at(F, g, c, i, j, k, d, -l - 1);
-                r = fma(co.b[d][l] * m, fma(np, fp - f0, nm * (fm - f0)), r);
-            }
-        }
-        const double dz = dd1<H>(F, g, c, i, j, k, 2, az);
-        out[(long long)c * g.N3 + t] = fma(-nu0 * corr2[k], dz, r);
-    }
 }
 
 // ------------------------------------------------------------------ layout --
@@ -852,26 +579,6 @@ void launch_maxabs_noalloc(long long n, const double *s, double *scratch, cudaSt
     const int np = (int)((n + kMaxabsChunk - 1) / kMaxabsChunk);
     k_maxabs_chunks<<<np, 256, 0, st>>>(n, s, scratch);
     k_max_final<<<1, 256, 0, st>>>(scratch, np, scratch + kMaxabsStaticParts);
-}
-
-void launch_op(int op, int h, const Geo &g, const Walls<double> &wa, const Walls<double> &wb, const Coef<double> &co,
-               const double *ia, const double *corr2, const double *a, const double *b, int nc, double nu, double *out,
-               cudaStream_t st)
-{
-    const unsigned nb = nblocks(g.N3, 128);
-    switch (op) {
-    case OP_GRAD_S: NOVA_DISPATCH_H(h, (k_op_grad_s<HH><<<nb, 128, 0, st>>>(g, wa, co, ia, a, out))); break;
-    case OP_GRAD_V: NOVA_DISPATCH_H(h, (k_op_grad_v<HH><<<nb, 128, 0, st>>>(g, wa, co, ia, a, out))); break;
-    case OP_DIV_V: NOVA_DISPATCH_H(h, (k_op_div_v<HH><<<nb, 128, 0, st>>>(g, wa, co, ia, a, out))); break;
-    case OP_CURL: NOVA_DISPATCH_H(h, (k_op_curl<HH><<<nb, 128, 0, st>>>(g, wa, co, ia, a, out))); break;
-    case OP_DIV_VF: NOVA_DISPATCH_H(h, (k_op_div_vf<HH><<<nb, 128, 0, st>>>(g, wa, wb, co, ia, a, b, nc, out))); break;
-    case OP_DIV_T: NOVA_DISPATCH_H(h, (k_op_div_t<HH><<<nb, 128, 0, st>>>(g, wa, co, a, nc == 6, out))); break;
-    case OP_DIV_ST: NOVA_DISPATCH_H(h, (k_op_div_st<HH><<<nb, 128, 0, st>>>(g, wa, wb, co, a, b, out))); break;
-    case OP_LAP_F:
-        NOVA_DISPATCH_H(h, (k_op_lap_f<HH><<<nb, 128, 0, st>>>(g, wa, wb, co, ia, corr2, a, b, nc, out)));
-        break;
-    default: NOVA_DISPATCH_H(h, (k_op_lap<HH><<<nb, 128, 0, st>>>(g, wa, co, ia, corr2, nu, a, nc, out))); break;
-    }
 }
 
 void launch_aos_to_soa(const Geo &g, int h, const int n[3], int nc, const double *aos, double *d64, float *hi,
