@@ -276,13 +276,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-// i-chunk: >= ~4 waves of the one resident block per SM
 int adj_ichunk(const Geo &g)
 {
     const long long tiles = (long long)(g.N2 / kTK) * (g.N1 / TJ);
-    int ch = g.N0;
-    while (ch > 16 && tiles * ((g.N0 + ch - 1) / ch) < 148LL * 4) ch /= 2;
-    return ch;
+    return march_chunk(g.N0, tiles, 1, 2.5);
 }
 
 template <int KIND, int S>

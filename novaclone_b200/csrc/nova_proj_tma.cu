@@ -364,18 +364,14 @@ template <typename T> bool encode_rows(ProjMaps &pm, int ms, const T *f, const G
            encode3(&pm.m[ms + M_RB], f, g, kTK, TJ + kH);
 }
 
-// i-chunk: at least `waves` waves of the 2 resident blocks per SM.  The 2H
-// warm-up planes of a chunk load the queue's tile rows alone; for DIV that is
-// a third of the slot (component 0's tile is in every slot), so its longer
-// chunks (2 waves at 256^3) win, while the correction's p rows and halos make
-// shorter chunks with a smaller last wave pay (4 waves: 156 -> 146 us at 256^3,
-// DIV 115 -> 120 us)
-int proj_ichunk(const Geo &g, int waves)
+// i-chunk.  The 2H warm-up planes of a chunk load the queue's tile rows alone;
+// the correction streams twice the bytes of the divergence per plane and its
+// last blocks are later (256^3: 24 planes 147 us, 64 planes 152 us; 192 x 192 x
+// 384: 20 planes 129 us, 96 planes 140 us)
+int proj_ichunk(const Geo &g, double tail)
 {
     const long long tiles = (long long)(g.N2 / kTK) * ((g.N1 + TJ - 1) / TJ);
-    int ch = g.N0;
-    while (ch > 16 && tiles * ((g.N0 + ch - 1) / ch) < 148LL * 2 * waves) ch /= 2;
-    return ch;
+    return march_chunk(g.N0, tiles, 2, 2.5, g.wallY ? 0.45 : tail);
 }
 
 template <int MODE, bool SPLIT, bool WALLS>
@@ -390,7 +386,7 @@ cudaError_t launch_w(const Geo &g, const Coef<double> &co, const Walls<double> &
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         attr = true;
     }
-    const int ch = proj_ichunk(g, MODE == PROJ_DIV ? 2 : 4);
+    const int ch = proj_ichunk(g, MODE == PROJ_DIV ? 0.15 : 0.3);
     const dim3 grid(g.N2 / kTK, (g.N1 + TJ - 1) / TJ, (g.N0 + ch - 1) / ch);
     kern<<<grid, dim3(kTK, TJ + 1), C::kSmem, st>>>(g, co, wl, ia, a, pm, ch, err);
     return cudaSuccess;

@@ -327,13 +327,10 @@ template <typename T> bool encode(CUtensorMap *m, const T *base, const Geo &g, u
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// i-chunk: >= ~4 waves of the one resident block per SM
 template <typename T> int mhd_ichunk(const Geo &g)
 {
     const long long tiles = (long long)(g.N2 / kTK) * (g.N1 / MhdCfg<T>::TJ);
-    int ch = g.N0;
-    while (ch > 16 && tiles * ((g.N0 + ch - 1) / ch) < 148LL * 4) ch /= 2;
-    return ch;
+    return march_chunk(g.N0, tiles, 1, 2.5);
 }
 
 template <typename T, int PHYS, int STAGE, bool STRETCH, class Args>

@@ -531,15 +531,11 @@ template <typename T> bool encode(CUtensorMap *m, const T *base, const Geo &g, u
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// i-chunk of a TMA stage launch: >= ~4 waves of resident blocks, the 2H-plane
-// warm-up kept small against the chunk length
 template <typename T> int tma_ichunk(const Geo &g)
 {
     using C = TmaCfg<T>;
     const long long tiles = (long long)(g.N2 / kTK) * ((g.N1 + C::TJ - 1) / C::TJ);
-    int ch = g.N0;
-    while (ch > 16 && tiles * ((g.N0 + ch - 1) / ch) < 148LL * C::kBlocksPerSM * 4) ch /= 2;
-    return ch;
+    return march_chunk(g.N0, tiles, C::kBlocksPerSM, 2.5, g.wallY ? 0.45 : 0.15);
 }
 
 template <typename T, int STAGE, bool STRETCH, class Args, bool DIAG = false, bool WALLS = false>

@@ -192,15 +192,11 @@ __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, Til
     tile_march<T, H, NC, WALLS>(g, wl, sm, ld, ib, ie, NoPre{}, body);
 }
 
-// grid shape of a tile march: k tiles x j tiles x i chunks
+// of a tile march (k tiles x j tiles x i chunks)
 inline int pick_ichunk(const Geo &g, int blocks_per_sm)
 {
-    // >= ~4 waves of resident blocks on 148 SMs, with the 2H-plane warm-up
-    // kept small against the chunk length
     const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + kTJ - 1) / kTJ);
-    int ch = g.N0;
-    while (ch > 16 && tiles * ((g.N0 + ch - 1) / ch) < 148LL * blocks_per_sm * 4) ch /= 2;
-    return ch;
+    return march_chunk(g.N0, tiles, blocks_per_sm, 3.0, g.wallY ? 0.45 : 0.15);
 }
 
 inline dim3 tile_grid(const Geo &g, int ch)
