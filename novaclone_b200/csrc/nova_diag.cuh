@@ -55,6 +55,10 @@ __device__ __forceinline__ void curl_terms(const VX &vx, const VY &vy, const VZ 
     half_sq = 0.5 * c2;
 }
 
+// The running maximum of |U| is kept as its square: sqrt is monotone and
+// correctly rounded, so k_diag_final's sqrt of the maximum is the maximum of
+// the square roots.
+//
 // the U terms only (6 running values: the fused stage's register budget),
 // expanded to the kDiagParts layout with zero B terms by part()
 struct DiagAccU {
@@ -65,7 +69,7 @@ struct DiagAccU {
         ek += 0.5 * uu;
         om += q1;
         ens += hs;
-        umax = fmax(umax, sqrt(uu));
+        umax = fmax(umax, uu);
         mdu = fmax(mdu, fabs(divu));
         ux = fmax(ux, u[0]);
     }
@@ -112,7 +116,7 @@ struct DiagAccSm {
         m[0] += 0.5 * uu;
         m[stride] += q1;
         m[2 * stride] += hs;
-        m[3 * stride] = fmax(m[3 * stride], sqrt(uu));
+        m[3 * stride] = fmax(m[3 * stride], uu);
         m[4 * stride] = fmax(m[4 * stride], fabs(divu));
         m[5 * stride] = fmax(m[5 * stride], u[0]);
     }
@@ -126,51 +130,6 @@ struct DiagAccSm {
         a.mdu = m[4 * stride];
         a.ux = m[5 * stride];
         return a;
-    }
-};
-
-// running per-thread values of the kDiagParts partials (layout in nova_internal.cuh)
-struct DiagAcc {
-    double v[kDiagParts];
-    __device__ DiagAcc()
-    {
-#pragma unroll
-        for (int q = 0; q < kDiagParts; q++) v[q] = 0.0;
-    }
-    // the U terms of a node: u the vector, divu its divergence, q1/hs its curl
-    // terms; unique = the node is one of the unique nodes the means cover
-    __device__ __forceinline__ void add_u(const double (&u)[3], double divu, double q1, double hs, bool unique)
-    {
-        const double uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
-        if (unique) {
-            v[DP_EK] += 0.5 * uu;
-            v[DP_OMEGA] += q1;
-            v[DP_ENSU] += hs;
-            v[DP_UMAX] = fmax(v[DP_UMAX], sqrt(uu));
-        }
-        v[DP_DIVU] = fmax(v[DP_DIVU], fabs(divu));
-        v[DP_UX] = fmax(v[DP_UX], u[0]);
-    }
-    __device__ __forceinline__ void add_b(const double (&b)[3], double divb, double q1, double hs, bool unique)
-    {
-        if (unique) {
-            v[DP_EM] += 0.5 * (b[0] * b[0] + b[1] * b[1] + b[2] * b[2]);
-            v[DP_JAV] += q1;
-            v[DP_ENSB] += hs;
-            v[DP_JMAX] = fmax(v[DP_JMAX], q1);
-        }
-        v[DP_DIVB] = fmax(v[DP_DIVB], fabs(divb));
-    }
-    // warp reduction (fixed order); the result is valid in lane 0
-    __device__ __forceinline__ void warp_reduce()
-    {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int q = 0; q < kDiagParts; q++) {
-                const double x = __shfl_down_sync(0xffffffffu, v[q], o);
-                v[q] = q >= DP_DIVU ? fmax(v[q], x) : v[q] + x;
-            }
     }
 };
 

@@ -165,48 +165,68 @@ constexpr int kRedThreads = 256;
 // does (the stored north-wall row is the reference's last node and is skipped);
 // the divergence maxima and U_x cover every stored node (tools::maximum,
 // src/Tools/Tools.h:19-36; tools::CFL, src/Tools/Tools.cpp:15-25).
-template <int H, int NC, class LD, bool WALLS>
-__global__ void __launch_bounds__(kThreads, NC == 3 ? 2 : 1) k_diag_tiled(Geo g, Walls<double> wl, Coef<double> co,
-                                                         const double *__restrict__ ia, LD U, LD B, int ichunk,
-                                                         double *__restrict__ part)
+// One field per block: blocks of the upper half of grid.z take B, whose terms
+// share no operand with U's (both fields in one block took 241 registers, one
+// block of 8 warps per SM).
+template <int H, class LD, bool WALLS>
+__global__ void __launch_bounds__(kThreads, 2) k_diag_tiled(Geo g, Walls<double> wlU, Walls<double> wlB,
+                                                            Coef<double> co, const double *__restrict__ ia, LD U, LD B,
+                                                            int ichunk, int nchunk, double *__restrict__ part)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    auto &sm = *reinterpret_cast<TileSmem<double, H, NC> *>(smraw);
-    __shared__ double red[kDiagParts][kThreads / 32];
-    const int ib = blockIdx.z * ichunk;
+    auto &sm = *reinterpret_cast<TileSmem<double, H, 3> *>(smraw);
+    __shared__ double red[6][kThreads / 32];
+    const bool isB = (int)blockIdx.z >= nchunk;
+    const LD &F = isB ? B : U;
+    const Walls<double> &wl = isB ? wlB : wlU;
+    const int ib = ((int)blockIdx.z - (isB ? nchunk : 0)) * ichunk;
     const int ie = min(ib + ichunk, g.N0);
     const int kw = wrapi(blockIdx.x * kTK + threadIdx.x, g.N2);
     double az[H];
 #pragma unroll
     for (int l = 0; l < H; l++) az[l] = co.a[2][l] * ia[kw];
-    const int rows_e = g.N1 - g.wallY;
-    DiagAcc acc;
-    auto ld = [&](int c, long long o) -> double { return c < 3 ? U(c, o) : B(c - 3, o); };
-    tile_march<double, H, NC, WALLS>(g, wl, sm, ld, ib, ie, [&](long long idx, auto &q, const auto &vx, const auto &vy,
-                                                          const auto &vz) {
-        const int j = (int)((idx % g.N12) / g.N2);
-        const bool ce = j < rows_e;
+    const bool ce = (int)(blockIdx.y * kTJ + threadIdx.y) < g.N1 - g.wallY;
+    double en = 0.0, om = 0.0, ens = 0.0, mdiv = 0.0, top = 0.0, ux = 0.0;  // top: max |U|^2, or max |curl B|
+    tile_march<double, H, 3, WALLS>(g, wl, sm, F, ib, ie, [&](long long, auto &q, const auto &vx, const auto &vy,
+                                                              const auto &vz) {
         const double u[3] = {q[H][0], q[H][1], q[H][2]};
         const double du = d1<double, H>(vx, 0, co.a[0]) + d1<double, H>(vy, 1, co.a[1]) + d1<double, H>(vz, 2, az);
         double q1, hs;
         curl_terms<H>(vx, vy, vz, 0, co.a[0], co.a[1], az, 1.0, q1, hs);
-        acc.add_u(u, du, q1, hs, ce);
-        if constexpr (NC == 6) {
-            const double b[3] = {q[H][3], q[H][4], q[H][5]};
-            const double db = d1<double, H>(vx, 3, co.a[0]) + d1<double, H>(vy, 4, co.a[1]) + d1<double, H>(vz, 5, az);
-            curl_terms<H>(vx, vy, vz, 3, co.a[0], co.a[1], az, 1.0, q1, hs);
-            acc.add_b(b, db, q1, hs, ce);
+        if (ce) {
+            const double uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+            en += 0.5 * uu;
+            om += q1;
+            ens += hs;
+            top = fmax(top, isB ? q1 : uu);
         }
+        mdiv = fmax(mdiv, fabs(du));
+        ux = fmax(ux, u[0]);
     });
     const int tid = threadIdx.y * kTK + threadIdx.x, lane = tid & 31, w = tid >> 5;
-    acc.warp_reduce();
-    if (lane == 0)
 #pragma unroll
-        for (int q = 0; q < kDiagParts; q++) red[q][w] = acc.v[q];
+    for (int o = 16; o > 0; o >>= 1) {
+        en += __shfl_down_sync(0xffffffffu, en, o);
+        om += __shfl_down_sync(0xffffffffu, om, o);
+        ens += __shfl_down_sync(0xffffffffu, ens, o);
+        mdiv = fmax(mdiv, __shfl_down_sync(0xffffffffu, mdiv, o));
+        top = fmax(top, __shfl_down_sync(0xffffffffu, top, o));
+        ux = fmax(ux, __shfl_down_sync(0xffffffffu, ux, o));
+    }
+    if (lane == 0) {
+        const double v[6] = {en, om, ens, mdiv, top, ux};
+#pragma unroll
+        for (int q = 0; q < 6; q++) red[q][w] = v[q];
+    }
     __syncthreads();
     if (tid < kDiagParts) {
+        // the value of partial tid among the six of this block's field, -1: the other field's (0)
+        const int mapU[kDiagParts] = {0, -1, 1, -1, 2, -1, 3, -1, -1, 4, 5, -1};
+        const int mapB[kDiagParts] = {-1, 0, -1, 1, -1, 2, -1, 3, 4, -1, -1, -1};
+        const int q = isB ? mapB[tid] : mapU[tid];
         double a = 0.0;
-        for (int x = 0; x < kThreads / 32; x++) a = tid >= DP_DIVU ? fmax(a, red[tid][x]) : a + red[tid][x];
+        if (q >= 0)
+            for (int x = 0; x < kThreads / 32; x++) a = q >= 3 ? fmax(a, red[q][x]) : a + red[q][x];
         const long long blk = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         part[blk * kDiagParts + tid] = a;
     }
@@ -215,18 +235,33 @@ __global__ void __launch_bounds__(kThreads, NC == 3 ? 2 : 1) k_diag_tiled(Geo g,
 // std::max(a, b) of the reference: b only when a < b
 __device__ __forceinline__ double ref_max(double a, double b) { return a < b ? b : a; }
 
-__global__ void k_diag_final(const double *__restrict__ part, int nblk, DiagFinal fin, double *__restrict__ row,
-                             int *__restrict__ flag)
+// kFinalRows threads per partial, consecutive threads on consecutive partials,
+// so that every load is coalesced; then one thread per partial over the rows in
+// order.  Latency-bound (one block): 2048 blocks of partials 18 -> 7 us,
+// 128 blocks 7.1 -> 4.2 us against twelve block reductions in a row.
+constexpr int kFinalRows = 64, kFinalThreads = kFinalRows * kDiagParts;
+__global__ void __launch_bounds__(kFinalThreads) k_diag_final(const double *__restrict__ part, int nblk, DiagFinal fin,
+                                                              double *__restrict__ row, int *__restrict__ flag)
 {
-    __shared__ double sh[32];
-    double tot[kDiagParts];
-#pragma unroll
-    for (int q = 0; q < kDiagParts; q++) {
-        double a = 0.0;
-        for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-            a = q >= DP_DIVU ? fmax(a, part[(long long)b * kDiagParts + q]) : a + part[(long long)b * kDiagParts + q];
-        tot[q] = q >= DP_DIVU ? block_reduce_max(a, sh) : block_reduce_sum(a, sh);
+    __shared__ double sh[kFinalRows][kDiagParts];
+    __shared__ double tot[kDiagParts];
+    const int q = threadIdx.x % kDiagParts, r = threadIdx.x / kDiagParts;
+    const bool mx = q >= DP_DIVU;
+    double a = 0.0;
+#pragma unroll 8
+    for (int b = r; b < nblk; b += kFinalRows) {
+        const double v = part[(long long)b * kDiagParts + q];
+        a = mx ? fmax(a, v) : a + v;
     }
+    sh[r][q] = a;
+    __syncthreads();
+    if (threadIdx.x < kDiagParts) {
+        double t = 0.0;
+#pragma unroll 16
+        for (int x = 0; x < kFinalRows; x++) t = mx ? fmax(t, sh[x][q]) : t + sh[x][q];
+        tot[q] = q == DP_UMAX ? sqrt(t) : t;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         const double n = fin.invN3;
         const double om = tot[DP_OMEGA] * n, jav = tot[DP_JAV] * n;
@@ -477,11 +512,22 @@ cudaError_t launch_correct(int h, const Geo &g, const Walls<double> &pw, const C
     return cudaSuccess;
 }
 
+// i-chunk of the diagnostics kernel over nf fields
+static int diag_chunk(const Geo &g, int nf)
+{
+    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + kTJ - 1) / kTJ) * nf;
+    return march_chunk(g.N0, tiles, 2, 3.0, g.wallY ? 0.45 : 0.15);
+}
+
 int diag_blocks(const Geo &g)
 {
-    const dim3 gr = tile_grid(g, pick_ichunk(g, 2));
-    const long long tiled = (long long)gr.x * gr.y * gr.z;
-    return (int)(tiled > 1184 ? tiled : 1184);
+    long long most = 1184;
+    for (int nf = 1; nf <= 2; nf++) {
+        const dim3 gr = tile_grid(g, diag_chunk(g, nf));
+        const long long nb = (long long)nf * gr.x * gr.y * gr.z;
+        most = nb > most ? nb : most;
+    }
+    return (int)most;
 }
 
 DiagFinal diag_final_of(const Geo &g, const DiagPhys &ph, double step, double time, const double *U64,
@@ -512,38 +558,41 @@ void launch_diag(int h, const Geo &g, const Walls<double> &wl, const Coef<double
                  const float *Blo, int hasB, double *part, double step, double time, double *row, int *flag,
                  cudaStream_t st, const DiagPhys &ph)
 {
-    const int ch = pick_ichunk(g, 2);
-    const dim3 grid = tile_grid(g, ch), block(kTK, kTJ);
+    const int ch = diag_chunk(g, hasB ? 2 : 1);
+    dim3 grid = tile_grid(g, ch);
+    const dim3 block(kTK, kTJ);
+    const int nchunk = (int)grid.z;
+    if (hasB) grid.z *= 2;
     const int nb = (int)(grid.x * grid.y * grid.z);
-#define NOVA_DIAG(NC, LDT, UU, BB, W)                                                                     \
+    // the walls of U's components, then of B's
+    Walls<double> wlB = wl;
+    for (int side = 0; side < 2; side++)
+        for (int c = 0; c < 3; c++) {
+            wlB.dir[side][c] = wl.dir[side][3 + c];
+            wlB.val[side][c] = wl.val[side][3 + c];
+        }
+#define NOVA_DIAG(LDT, UU, BB)                                                                            \
     NOVA_DISPATCH_H(h, {                                                                                  \
-        constexpr size_t sb = tile_smem_bytes<double, HH, NC>();                                          \
-        if (sb > 48 * 1024)                                                                               \
-            cudaFuncSetAttribute(k_diag_tiled<HH, NC, LDT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb); \
-        k_diag_tiled<HH, NC, LDT, W><<<grid, block, sb, st>>>(g, wl, co, ia, UU, BB, ch, part);            \
+        constexpr size_t sb = tile_smem_bytes<double, HH, 3>();                                           \
+        if (wl.on)                                                                                        \
+            k_diag_tiled<HH, LDT, true><<<grid, block, sb, st>>>(g, wl, wlB, co, ia, UU, BB, ch, nchunk, part);  \
+        else                                                                                              \
+            k_diag_tiled<HH, LDT, false><<<grid, block, sb, st>>>(g, wl, wlB, co, ia, UU, BB, ch, nchunk, part); \
     })
     if (U64) {
-        Ld64 U{U64, g.N3, wl}, B{hasB ? B64 : U64, g.N3, wl};
-        if (hasB) {
-            if (wl.on) { NOVA_DIAG(6, Ld64, U, B, true); } else { NOVA_DIAG(6, Ld64, U, B, false); }
-        } else {
-            if (wl.on) { NOVA_DIAG(3, Ld64, U, B, true); } else { NOVA_DIAG(3, Ld64, U, B, false); }
-        }
+        Ld64 U{U64, g.N3, wl}, B{hasB ? B64 : U64, g.N3, wlB};
+        NOVA_DIAG(Ld64, U, B);
     } else {
-        LdSplit U{Uhi, Ulo, g.N3, wl}, B{hasB ? Bhi : Uhi, hasB ? Blo : Ulo, g.N3, wl};
-        if (hasB) {
-            if (wl.on) { NOVA_DIAG(6, LdSplit, U, B, true); } else { NOVA_DIAG(6, LdSplit, U, B, false); }
-        } else {
-            if (wl.on) { NOVA_DIAG(3, LdSplit, U, B, true); } else { NOVA_DIAG(3, LdSplit, U, B, false); }
-        }
+        LdSplit U{Uhi, Ulo, g.N3, wl}, B{hasB ? Bhi : Uhi, hasB ? Blo : Ulo, g.N3, wlB};
+        NOVA_DIAG(LdSplit, U, B);
     }
 #undef NOVA_DIAG
-    k_diag_final<<<1, 256, 0, st>>>(part, nb, diag_final_of(g, ph, step, time, U64, Uhi, Ulo), row, flag);
+    k_diag_final<<<1, kFinalThreads, 0, st>>>(part, nb, diag_final_of(g, ph, step, time, U64, Uhi, Ulo), row, flag);
 }
 
 void launch_diag_final(const double *part, int nb, const DiagFinal &fin, double *row, int *flag, cudaStream_t st)
 {
-    k_diag_final<<<1, 256, 0, st>>>(part, nb, fin, row, flag);
+    k_diag_final<<<1, kFinalThreads, 0, st>>>(part, nb, fin, row, flag);
 }
 
 void launch_maxabs(const Geo &g, const double *s, double *part, double *out, cudaStream_t st)
