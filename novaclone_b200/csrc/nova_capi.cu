@@ -123,10 +123,15 @@ struct nova_ctx {
     double *d_kx2 = nullptr, *d_ky2 = nullptr, *d_kz2 = nullptr;
     cufftHandle plan_f = 0, plan_b = 0;
     bool plans = false;
-    // periodic meshes with N0 = 64 or 256: plan_f/plan_b are batched 2-D (j, k)
-    // transforms and the i direction runs fused with the scale (k_pois_i)
+    // N0 a length of nova_spec.cuh: the i direction runs fused with the scale
+    // (k_pois_i) between transforms of the (j, k) planes: by the library's own
+    // line kernels where N1 and N2/2 are such lengths too (own_jk), else by
+    // plan_f/plan_b, batched 2-D cuFFT plans.  NOVA_FFT=cufft keeps the plans.
     bool pois_i = false;
-    double *d_twN = nullptr;  // W_N0^m, m = 0..N0-1 (re, im)
+    bool own_jk = false;
+    bool fft_plans = false;
+    double *d_twN = nullptr;               // W_N0^m, m = 0..N0-1 (re, im)
+    double *d_twR = nullptr, *d_twC = nullptr;  // W_N2^m and W_N1^m
     // N1 = N2 = 256 as well and NOVA_FFT=cluster: the (j, k) planes by the
     // one-pass cluster kernels (nova_fft2d.cu) instead of the cuFFT plans
     bool fft2 = false;
@@ -142,6 +147,7 @@ struct nova_ctx {
     // rows and k_pois_dct (DCT-I along y); NOVA_DCT=extend keeps the even extension
     cufftHandle dct2_f = 0, dct2_b = 0;
     bool dct2_plans = false;
+    bool dct2_own = false;  // the (i, k) transforms by the line kernels
     bool dct_extend = false;
     void *d_spec3 = nullptr;
     double *d_t512 = nullptr;
@@ -389,6 +395,17 @@ std::vector<double> twiddles(int N)
     return tw;
 }
 
+// the twiddle table W_N on the device
+nova_status twiddle_table(nova_ctx *ctx, double **d, int N)
+{
+    if (*d) return NOVA_OK;
+    const std::vector<double> tw = twiddles(N);
+    const nova_status s = dalloc(ctx, d, tw.size());
+    if (s != NOVA_OK) return s;
+    CK(cudaMemcpy(*d, tw.data(), sizeof(double) * tw.size(), cudaMemcpyHostToDevice));
+    return NOVA_OK;
+}
+
 nova_status ensure_fft(nova_ctx *ctx)
 {
     if (ctx->fft_ready) return NOVA_OK;
@@ -413,10 +430,15 @@ nova_status ensure_fft(nova_ctx *ctx)
     // which with walls are the first N[1] of the N[1]+1 stored rows
     const int ny = ctx->md.N[1];
     const bool pi = pois_i_fits(g);
-    if (pi) {
-        std::vector<double> tw = twiddles(g.N0);
-        if ((s = dalloc(ctx, &ctx->d_twN, tw.size())) != NOVA_OK) return s;
-        CK(cudaMemcpy(ctx->d_twN, tw.data(), sizeof(double) * tw.size(), cudaMemcpyHostToDevice));
+    if (pi && (s = twiddle_table(ctx, &ctx->d_twN, g.N0)) != NOVA_OK) return s;
+    const size_t nspec = (size_t)g.N0 * ny * (g.N2 / 2 + 1);
+    if (pi && !ctx->fft_plans && spec_cols_fit(ny) && spec_rows_fit(g.N2)) {
+        if ((s = twiddle_table(ctx, &ctx->d_twR, g.N2)) != NOVA_OK) return s;
+        if ((s = twiddle_table(ctx, &ctx->d_twC, ny)) != NOVA_OK) return s;
+        if ((s = dalloc(ctx, (double **)&ctx->d_spec, 2 * nspec)) != NOVA_OK) return s;
+        if ((s = dalloc(ctx, &ctx->d_rhs, (size_t)g.N3)) != NOVA_OK) return s;
+        ctx->pois_i = ctx->own_jk = ctx->fft_ready = true;
+        return NOVA_OK;
     }
     // 3-D transform, or for k_pois_i the (j, k) planes batched over i; both
     // give the half spectrum [i][j][kz]
@@ -436,7 +458,6 @@ nova_status ensure_fft(nova_ctx *ctx)
     }
     ctx->plans = true;
     ctx->pois_i = pi;
-    const size_t nspec = (size_t)g.N0 * ny * (g.N2 / 2 + 1);
     if ((s = dalloc(ctx, (double **)&ctx->d_spec, 2 * nspec)) != NOVA_OK) return s;
     if ((s = dalloc(ctx, &ctx->d_rhs, (size_t)g.N3)) != NOVA_OK) return s;
     ctx->fft_ready = true;
@@ -479,6 +500,18 @@ nova_status poisson_device(nova_ctx *ctx, const double *rhs, double *p)
         CKL("cluster FFT / k_pois_i");
         return NOVA_OK;
     }
+    if (ctx->own_jk) {
+        const int ny = ctx->md.N[1], nzh = ctx->g.N2 / 2 + 1;
+        launch_rows_fwd(ctx->g.N0, ny, ctx->g.N12, ctx->g.N2, rhs, ctx->d_spec, ctx->d_twR, ctx->stream);
+        launch_cols_j(ctx->g.N0, ny, nzh, false, ctx->d_spec, ctx->d_twC, ctx->stream);
+        launch_pois_i(ctx->g, ny, ctx->d_spec, ctx->d_twN, ctx->d_kx2, ctx->d_ky2, ctx->d_kz2, 1.0 / (double)nuniq,
+                      ctx->pois_direct ? nullptr : ctx->d_flag + 1, ctx->stream);
+        launch_cols_j(ctx->g.N0, ny, nzh, true, ctx->d_spec, ctx->d_twC, ctx->stream);
+        launch_rows_inv(ctx->g.N0, ny, ctx->g.N12, ctx->g.N2, ctx->d_spec, p, ctx->d_twR, ctx->stream);
+        ctx->launches += 5;
+        CKL("line transforms / k_pois_i");
+        return NOVA_OK;
+    }
     cufftSetStream(ctx->plan_f, ctx->stream);
     cufftSetStream(ctx->plan_b, ctx->stream);
     if ((s = fft_check(ctx, cufftExecD2Z(ctx->plan_f, (cufftDoubleReal *)rhs, (cufftDoubleComplex *)ctx->d_spec),
@@ -517,7 +550,13 @@ nova_status poisson_device_dct1(nova_ctx *ctx, const double *rhs, double *p)
     const Geo &g = ctx->g;
     const int ny = ctx->md.N[1], nzh = g.N2 / 2 + 1;
     nova_status s;
-    if (!ctx->dct2_plans) {
+    const bool own = !ctx->fft_plans && spec_rows_fit(g.N2) && spec_cols_fit(g.N0);
+    if (own && !ctx->dct2_own) {
+        if ((s = twiddle_table(ctx, &ctx->d_twR, g.N2)) != NOVA_OK) return s;
+        if ((s = twiddle_table(ctx, &ctx->d_twN, g.N0)) != NOVA_OK) return s;
+        ctx->dct2_own = true;
+    }
+    if (!own && !ctx->dct2_plans) {
         // element (i, j, k) of a batch-j plane at j N2 + i N1 N2 + k; spectrum at (i N1 + j) nzh + kz
         int n[2] = {g.N0, g.N2}, rin[2] = {g.N0, (int)g.N12}, cin[2] = {g.N0, g.N1 * nzh};
         if ((s = fft_check(ctx, cufftPlanMany(&ctx->dct2_f, 2, n, rin, 1, g.N2, cin, 1, nzh, CUFFT_D2Z, g.N1),
@@ -529,12 +568,11 @@ nova_status poisson_device_dct1(nova_ctx *ctx, const double *rhs, double *p)
             return s;
         }
         ctx->dct2_plans = true;
+    }
+    if (!ctx->d_t512 || !ctx->d_ky2e || !ctx->d_spec3) {
         if ((s = dalloc(ctx, (double **)&ctx->d_spec3, 2 * (size_t)g.N0 * g.N1 * nzh)) != NOVA_OK) return s;
-        const std::vector<double> t256 = twiddles(256), t512 = twiddles(512), ky2e = ky2_walls(ctx);
-        if (!ctx->d_tw256) {
-            if ((s = dalloc(ctx, &ctx->d_tw256, t256.size())) != NOVA_OK) return s;
-            CK(cudaMemcpy(ctx->d_tw256, t256.data(), sizeof(double) * t256.size(), cudaMemcpyHostToDevice));
-        }
+        const std::vector<double> t512 = twiddles(512), ky2e = ky2_walls(ctx);
+        if ((s = twiddle_table(ctx, &ctx->d_tw256, 256)) != NOVA_OK) return s;
         if ((s = dalloc(ctx, &ctx->d_t512, 512)) != NOVA_OK) return s;  // W_512^n, n < 256
         CK(cudaMemcpy(ctx->d_t512, t512.data(), sizeof(double) * 512, cudaMemcpyHostToDevice));
         if (!ctx->d_ky2e) {
@@ -543,13 +581,26 @@ nova_status poisson_device_dct1(nova_ctx *ctx, const double *rhs, double *p)
         }
     }
     ProfScope ps(ctx, NOVA_K_FFT);
+    const double scale = 1.0 / ((double)g.N0 * 2.0 * ny * g.N2);
+    if (own) {
+        const long long per_plane = (long long)g.N1 * nzh;
+        launch_rows_fwd(g.N0, g.N1, g.N12, g.N2, rhs, ctx->d_spec3, ctx->d_twR, ctx->stream);
+        launch_cols_i(g.N0, per_plane, false, ctx->d_spec3, ctx->d_twN, ctx->stream);
+        launch_pois_dct(g, ctx->d_spec3, ctx->d_tw256, ctx->d_t512, ctx->d_kx2, ctx->d_ky2e, ctx->d_kz2, scale,
+                        ctx->stream);
+        launch_cols_i(g.N0, per_plane, true, ctx->d_spec3, ctx->d_twN, ctx->stream);
+        launch_rows_inv(g.N0, g.N1, g.N12, g.N2, ctx->d_spec3, p, ctx->d_twR, ctx->stream);
+        ctx->launches += 5;
+        CKL("wall poisson (DCT-I)");
+        return NOVA_OK;
+    }
     cufftSetStream(ctx->dct2_f, ctx->stream);
     cufftSetStream(ctx->dct2_b, ctx->stream);
     if ((s = fft_check(ctx, cufftExecD2Z(ctx->dct2_f, const_cast<double *>(rhs), (cufftDoubleComplex *)ctx->d_spec3),
                        "cufftExecD2Z")) != NOVA_OK)
         return s;
-    launch_pois_dct(g, ctx->d_spec3, ctx->d_tw256, ctx->d_t512, ctx->d_kx2, ctx->d_ky2e, ctx->d_kz2,
-                    1.0 / ((double)g.N0 * 2.0 * ny * g.N2), ctx->stream);
+    launch_pois_dct(g, ctx->d_spec3, ctx->d_tw256, ctx->d_t512, ctx->d_kx2, ctx->d_ky2e, ctx->d_kz2, scale,
+                    ctx->stream);
     if ((s = fft_check(ctx, cufftExecZ2D(ctx->dct2_b, (cufftDoubleComplex *)ctx->d_spec3, p), "cufftExecZ2D")) !=
         NOVA_OK)
         return s;
@@ -646,7 +697,10 @@ extern "C" nova_status nova_create(const nova_mesh_desc *md, nova_ctx **out)
         if (!std::strcmp(impl, "march")) ctx->stage_impl = STAGE_MARCH;
         if (!std::strcmp(impl, "tma")) ctx->stage_impl = STAGE_TMA;
     }
-    if (const char *f = std::getenv("NOVA_FFT")) ctx->fft_cluster = !std::strcmp(f, "cluster");
+    if (const char *f = std::getenv("NOVA_FFT")) {
+        ctx->fft_cluster = !std::strcmp(f, "cluster");
+        ctx->fft_plans = !std::strcmp(f, "cufft");
+    }
     if (const char *f = std::getenv("NOVA_POIS_I")) ctx->pois_direct = !std::strcmp(f, "direct");
     if (const char *f = std::getenv("NOVA_DCT")) ctx->dct_extend = !std::strcmp(f, "extend");
     for (int a = 0; a < 3; a++) ctx->local_n[a] = md->N[a] + 1 + md->m;
@@ -737,7 +791,7 @@ extern "C" nova_status nova_destroy(nova_ctx *ctx)
     void *ptrs[] = {ctx->d_ia64, ctx->d_corr64, ctx->d_ia32, ctx->d_corr32, ctx->d_kx2, ctx->d_ky2, ctx->d_kz2,
                     ctx->d_spec, ctx->d_rhs, ctx->w64[0], ctx->w64[1], ctx->w64[2], ctx->w32[0], ctx->w32[1],
                     ctx->w32[2], ctx->d_part, ctx->d_scalar, ctx->d_flag, ctx->d_hist, ctx->d_stage, ctx->adj_pool, ctx->d_row, ctx->d_ext, ctx->d_ky2e, ctx->d_spec2, ctx->d_twN, ctx->d_tw256,
-                    ctx->d_spec3, ctx->d_t512};
+                    ctx->d_spec3, ctx->d_t512, ctx->d_twR, ctx->d_twC};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     ctx->bufs->close();

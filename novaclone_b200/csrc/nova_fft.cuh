@@ -1,7 +1,8 @@
 // Register-resident DFT building blocks of the spectral Poisson solve
-// (nova_pois_i.cu, nova_fft2d.cu): complex products, and R-point DFTs (R = 4,
-// 8, 16) in natural order with twiddles W_R^m read from a table of W_N^m
-// (N a multiple of R) at compile-time indices.
+// (nova_spec.cuh, nova_pois_i.cu, nova_pois_dct.cu, nova_fft2d.cu): complex
+// products, and R-point DFTs (R = 4, 5, 6, 8, 9, 10, 12, 15, 16) in natural order with
+// twiddles W_R^m read from a table of W_N^m (N a multiple of R) at
+// compile-time indices.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -109,11 +110,107 @@ template <int N, bool INV> __device__ __forceinline__ void dft16(double2 (&v)[16
     for (int k = 0; k < 16; k++) v[k] = o[k];
 }
 
+// 2-, 3- and 5-point DFTs in place (strided registers a[0], a[S], a[2 S], ...)
+template <int S> __device__ __forceinline__ void dft2s(double2 *a)
+{
+    const double2 t = a[S];
+    a[S] = make_double2(a[0].x - t.x, a[0].y - t.y);
+    a[0] = make_double2(a[0].x + t.x, a[0].y + t.y);
+}
+
+template <int S, bool INV> __device__ __forceinline__ void dft3s(double2 *a)
+{
+    const double h = 0.86602540378443864676;  // sqrt(3)/2
+    const double2 t = make_double2(a[S].x + a[2 * S].x, a[S].y + a[2 * S].y);
+    const double2 d = make_double2(h * (a[S].x - a[2 * S].x), h * (a[S].y - a[2 * S].y));
+    const double2 u = make_double2(fma(-0.5, t.x, a[0].x), fma(-0.5, t.y, a[0].y));
+    a[0] = make_double2(a[0].x + t.x, a[0].y + t.y);
+    // u -+ i d
+    a[S] = INV ? make_double2(u.x - d.y, u.y + d.x) : make_double2(u.x + d.y, u.y - d.x);
+    a[2 * S] = INV ? make_double2(u.x + d.y, u.y - d.x) : make_double2(u.x - d.y, u.y + d.x);
+}
+
+template <int S, bool INV> __device__ __forceinline__ void dft5s(double2 *a)
+{
+    // cos and sin of 2 pi / 5 and 4 pi / 5
+    const double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;
+    const double s1 = 0.95105651629515357212, s2 = 0.58778525229247312917;
+    const double2 p1 = make_double2(a[S].x + a[4 * S].x, a[S].y + a[4 * S].y);
+    const double2 p2 = make_double2(a[2 * S].x + a[3 * S].x, a[2 * S].y + a[3 * S].y);
+    const double2 m1 = make_double2(a[S].x - a[4 * S].x, a[S].y - a[4 * S].y);
+    const double2 m2 = make_double2(a[2 * S].x - a[3 * S].x, a[2 * S].y - a[3 * S].y);
+    const double2 e1 = make_double2(fma(c1, p1.x, fma(c2, p2.x, a[0].x)), fma(c1, p1.y, fma(c2, p2.y, a[0].y)));
+    const double2 e2 = make_double2(fma(c2, p1.x, fma(c1, p2.x, a[0].x)), fma(c2, p1.y, fma(c1, p2.y, a[0].y)));
+    const double2 o1 = make_double2(fma(s1, m1.x, s2 * m2.x), fma(s1, m1.y, s2 * m2.y));
+    const double2 o2 = make_double2(fma(s2, m1.x, -s1 * m2.x), fma(s2, m1.y, -s1 * m2.y));
+    a[0] = make_double2(a[0].x + p1.x + p2.x, a[0].y + p1.y + p2.y);
+    const double g = INV ? -1.0 : 1.0;  // X_k = e - i o (forward)
+    a[S] = make_double2(fma(g, o1.y, e1.x), fma(-g, o1.x, e1.y));
+    a[4 * S] = make_double2(fma(-g, o1.y, e1.x), fma(g, o1.x, e1.y));
+    a[2 * S] = make_double2(fma(g, o2.y, e2.x), fma(-g, o2.x, e2.y));
+    a[3 * S] = make_double2(fma(-g, o2.y, e2.x), fma(g, o2.x, e2.y));
+}
+
+template <int P, int S, bool INV> __device__ __forceinline__ void dft_prime(double2 *a)
+{
+    if constexpr (P == 2)
+        dft2s<S>(a);
+    else if constexpr (P == 3)
+        dft3s<S, INV>(a);
+    else if constexpr (P == 4)
+        dft4<INV>(a[0], a[S], a[2 * S], a[3 * S]);
+    else
+        dft5s<S, INV>(a);
+}
+
+// R = A x B (n = B n1 + n2, k = k1 + A k2), A and B in 2..5: A-point DFTs over
+// n1, the twiddles W_R^(n2 k1), B-point DFTs over n2, then the index transpose
+template <int A, int B, int N, bool INV> __device__ __forceinline__ void dft_ab(double2 (&v)[A * B], const double2 *tw)
+{
+    constexpr int R = A * B;
+#pragma unroll
+    for (int n2 = 0; n2 < B; n2++) dft_prime<A, B, INV>(&v[n2]);
+#pragma unroll
+    for (int n2 = 1; n2 < B; n2++)
+#pragma unroll
+        for (int k1 = 1; k1 < A; k1++) {
+            double2 &x = v[B * k1 + n2];
+            if (4 * n2 * k1 == R)
+                x = INV ? make_double2(-x.y, x.x) : make_double2(x.y, -x.x);
+            else
+                x = cmul(x, INV ? conj2(tw[n2 * k1 * (N / R)]) : tw[n2 * k1 * (N / R)]);
+        }
+#pragma unroll
+    for (int k1 = 0; k1 < A; k1++) dft_prime<B, 1, INV>(&v[B * k1]);
+    double2 o[R];
+#pragma unroll
+    for (int k1 = 0; k1 < A; k1++)
+#pragma unroll
+        for (int k2 = 0; k2 < B; k2++) o[k1 + A * k2] = v[B * k1 + k2];
+#pragma unroll
+    for (int k = 0; k < R; k++) v[k] = o[k];
+}
+
 template <int R, int N, bool INV> __device__ __forceinline__ void dft(double2 (&v)[R], const double2 *tw)
 {
-    static_assert(R == 8 || R == 16, "R-point DFTs of 8 or 16 points");
+    static_assert(R == 4 || R == 5 || R == 6 || R == 8 || R == 9 || R == 10 || R == 12 || R == 15 || R == 16,
+                  "register DFT lengths");
     if constexpr (R == 16)
         dft16<N, INV>(v, tw);
+    else if constexpr (R == 4)
+        dft4<INV>(v[0], v[1], v[2], v[3]);
+    else if constexpr (R == 5)
+        dft5s<1, INV>(&v[0]);
+    else if constexpr (R == 6)
+        dft_ab<2, 3, N, INV>(v, tw);
+    else if constexpr (R == 9)
+        dft_ab<3, 3, N, INV>(v, tw);
+    else if constexpr (R == 15)
+        dft_ab<3, 5, N, INV>(v, tw);
+    else if constexpr (R == 10)
+        dft_ab<2, 5, N, INV>(v, tw);
+    else if constexpr (R == 12)
+        dft_ab<4, 3, N, INV>(v, tw);
     else
         dft_radix2<R, N, INV>(v, tw);
 }

@@ -33,9 +33,23 @@ cudaError_t launch_div_proj(int h, const Geo &g, const Walls<double> &wl, const 
 void launch_scale(const Geo &g, int ny, void *spec, const double *kx2, const double *ky2, const double *kz2,
                   double invN3, cudaStream_t st);
 // the i direction of the periodic spectral solve fused with the scale
-// (nova_pois_i.cu): in place on the half spectrum [i][j][kz] of the 2-D
-// (j, k) transforms; twN = W_N0^m, m = 0..N0-1 (interleaved re, im)
+// (nova_pois_i.cu): in place on the half spectrum [i][j][kz] of the (j, k)
+// transforms; twN = W_N0^m, m = 0..N0-1 (interleaved re, im)
 bool pois_i_fits(const Geo &g);
+// real transforms along k (nova_spec_row.cu): rows of n2 reals, ny of each of
+// `planes` planes (plane: reals between them), to and from the half spectrum
+// [plane][row][n2/2 + 1]; twN = W_n2^m, m < n2
+bool spec_rows_fit(int n2);
+void launch_rows_fwd(int planes, int ny, long long plane, int n2, const double *x, void *spec, const double *twN,
+                     cudaStream_t st);
+void launch_rows_inv(int planes, int ny, long long plane, int n2, const void *spec, double *x, const double *twN,
+                     cudaStream_t st);
+// complex transforms of the half spectrum [i][j][kz] in place (nova_spec_col.cu):
+// along j (ny values, nzh kz each), and along i (n0 values, per_plane = rows
+// times kz); twL = W_L^m, m < L
+bool spec_cols_fit(int L);
+void launch_cols_j(int n0, int ny, int nzh, bool inv, void *spec, const double *twL, cudaStream_t st);
+void launch_cols_i(int n0, long long per_plane, bool inv, void *spec, const double *twL, cudaStream_t st);
 // the (j, k) plane transforms in one pass each (nova_fft2d.cu, clusters of
 // eight CTAs): periodic y, N1 = N2 = 256, and the device can hold a cluster;
 // x real [i][j][k] <-> spec [i][j][kz] (kz < 129), unnormalised like cuFFT's

@@ -4,29 +4,29 @@
 //   rhs^ = FFT_i FFT_j FFT_k rhs,  rhs^ = -rhs^ / k'^2 / (N0 N1 N2)  (0 where k'^2 < 1e-16),
 //   p = IFFT_k IFFT_j IFFT_i rhs^
 //
-// cuFFT runs the (j, k) planes as batched 2-D transforms (D2Z before, Z2D
-// after); this kernel does FFT_i, the scale and IFFT_i of every (j, kz)
-// column of the half spectrum [i][j][kz] in one pass over HBM, where a 3-D
-// cuFFT plan needs an i pass on either side and the scale a pass of its own.
+// The (j, k) planes are transformed before and after (nova_spec_row.cu and
+// nova_spec_col.cu, or cuFFT's batched 2-D D2Z and Z2D); this kernel does
+// FFT_i, the scale and IFFT_i of every (j, kz) column of the half spectrum
+// [i][j][kz] in one pass over HBM, where a 3-D cuFFT plan needs an i pass on
+// either side and the scale a pass of its own.
 //
-// Length N0 = R * R, two-step decomposition with n = R n1 + n2, k = k1 + R k2:
-//   X[k1 + R k2] = sum_n2 W_R^(n2 k2) W_N^(n2 k1) sum_n1 x[R n1 + n2] W_R^(n1 k1)
-// and the inverse with the roles of the two indices exchanged.  A block owns
-// kCols consecutive kz columns of one j; thread (col, t) loads its R values
-// x[R n1 + t] straight from HBM, runs R-point DFTs in registers, and one
-// shared-memory transpose joins the two steps.  The twiddles W_N^m are a
-// host-computed table; the scale is k_scale's up to the rounding of one
-// reciprocal (within an ulp or two of its two divisions).
+// Length N0 = R1 R2 (nova_spec.cuh).  A block owns kSpecCols consecutive
+// (j, kz) columns; a thread loads its values straight from HBM, runs the
+// forward steps, the scale and the inverse steps with the indices' roles
+// exchanged.  The twiddles W_N^m are a host-computed table; the scale is
+// k_scale's up to the rounding of one reciprocal (within an ulp or two of its
+// two divisions).
 //
 // N0 = 256 with N2 % 16 == 0 and N1 % 8 == 0 runs k_pois_tma instead: the
 // same arithmetic on tiles of 8 columns, fed by bulk tensor loads into a
 // double-buffered shared-memory tile (the next tile lands while the block
-// transforms the current one), in a persistent grid.  k_pois_i loads, computes
-// and stores in turn, so with two blocks per SM the memory pipe idles while
-// both compute (96 us at 256^3 against a 41 us byte floor).
+// transforms the current one), in a persistent grid: 70 us at 256^3, k_pois_i 96
+// us, byte floor 41 us (k_pois_i loads, computes and stores in turn, so with two
+// blocks per SM the memory pipe idles while both compute).
 #include "nova_fft.cuh"
 #include "nova_internal.cuh"
 #include "nova_ops.cuh"
+#include "nova_spec.cuh"
 #include "nova_tma.cuh"
 
 #include <algorithm>
@@ -36,86 +36,71 @@ namespace nova {
 
 namespace {
 
-constexpr int kCols = 16;  // kz columns per block: 16 x 16 B = 256 contiguous bytes per i row
-
-template <int R>
-__global__ void __launch_bounds__(kCols *R, R == 16 ? 2 : 4)
-    k_pois_i(int ny, int nzh, double2 *__restrict__ spec, const double2 *__restrict__ twN,
+template <int R1, int R2>
+__global__ void __launch_bounds__(column_threads<R1, R2>(), column_blocks<R1, R2>())
+    k_pois_i(int nzh, long long ncol, double2 *__restrict__ spec, const double2 *__restrict__ twN,
              const double *__restrict__ kx2, const double *__restrict__ ky2, const double *__restrict__ kz2,
              double invN3)
 {
-    constexpr int N = R * R;
+    constexpr int N = R1 * R2, T = Line<R1, R2>::T, U = Line<R1, R2>::U;
     extern __shared__ __align__(16) unsigned char smraw[];
     double2 *tw = reinterpret_cast<double2 *>(smraw);  // W_N^m, m = 0..N-1
-    double2 *S = tw + N;                               // transpose buffer [R][R][kCols]
+    double2 *S = tw + N;                               // transpose buffer [R1][R2][kSpecCols]
     const int tid = threadIdx.x;
-    const int col = tid % kCols, t = tid / kCols;
-    const int j = blockIdx.y;
-    const int kz = blockIdx.x * kCols + col;
-    const bool valid = kz < nzh;
-    for (int m = tid; m < N; m += kCols * R) tw[m] = twN[m];
-    // element (i, j, kz) of the half spectrum; this thread's rows are i = t + R m
-    const long long rowstride = (long long)ny * nzh;
-    double2 *col_t = spec + (long long)t * rowstride + (long long)j * nzh + (valid ? kz : 0);
-    const long long step = R * rowstride;
-
-    double2 v[R];
+    const int col = tid % kSpecCols, t = tid / kSpecCols;
+    const long long c = blockIdx.x * (long long)kSpecCols + col;  // column j nzh + kz
+    const bool valid = c < ncol;
+    double2 *p = spec + (valid ? c : 0);  // element i at p[i ncol]
+    double2 v[U][R1], w[R2];
 #pragma unroll
-    for (int n1 = 0; n1 < R; n1++) v[n1] = valid ? col_t[n1 * step] : make_double2(0.0, 0.0);
-    __syncthreads();  // the twiddle table
-
-    // forward, step 1 (thread = n2 = t): DFT over n1, twiddle W_N^(t k1)
-    dft<R, N, false>(v, tw);
+    for (int u = 0; u < U; u++)
 #pragma unroll
-    for (int k1 = 0; k1 < R; k1++) S[(k1 * R + t) * kCols + col] = k1 == 0 ? v[0] : cmul(v[k1], tw[(t * k1) % N]);
+        for (int n1 = 0; n1 < R1; n1++) v[u][n1] = valid ? p[(R2 * n1 + t + T * u) * ncol] : make_double2(0.0, 0.0);
+    const double kyz = ky2[valid ? c / nzh : 0], kzz = kz2[valid ? c % nzh : 0];
+    for (int m = tid; m < N; m += column_threads<R1, R2>()) tw[m] = twN[m];
     __syncthreads();
-    // forward, step 2 (thread = k1 = t): DFT over n2 -> X[t + R k2]
-#pragma unroll
-    for (int n2 = 0; n2 < R; n2++) v[n2] = S[(t * R + n2) * kCols + col];
-    __syncthreads();  // S is rewritten below
-    dft<R, N, false>(v, tw);
-
+    column_fft<R1, R2, false>(v, w, S, tw, t, col);
     // scale: -1 / k'^2 / (N0 N1 N2), 0 where k'^2 < 1e-16 (k'^2 summed in
     // k_scale's order; one reciprocal per element instead of two divisions)
-    const double kyz = ky2[j], kzz = valid ? kz2[kz] : 0.0;
+    if (T == R1 || t < R1) {
 #pragma unroll
-    for (int k2 = 0; k2 < R; k2++) {
-        const double k2v = (kx2[t + R * k2] + kyz) + kzz;
-        const double f = k2v < 1.0e-16 ? 0.0 : -invN3 * recip(k2v);
-        v[k2] = make_double2(v[k2].x * f, v[k2].y * f);
+        for (int k2 = 0; k2 < R2; k2++) {
+            const double k2v = (kx2[t + R1 * k2] + kyz) + kzz;
+            const double f = k2v < 1.0e-16 ? 0.0 : -invN3 * recip(k2v);
+            w[k2] = make_double2(w[k2].x * f, w[k2].y * f);
+        }
+        // inverse, step 1 (thread = k1 = t): DFT over k2, twiddle W_N^-(n2 t)
+        dft<R2, N, true>(w, tw);
     }
-
-    // inverse, step 1 (thread = k1 = t): DFT over k2, twiddle W_N^-(n1 t)
-    dft<R, N, true>(v, tw);
+    __syncthreads();  // S is rewritten
+    if (T == R1 || t < R1)
 #pragma unroll
-    for (int n1 = 0; n1 < R; n1++)
-        S[(n1 * R + t) * kCols + col] = n1 == 0 ? v[0] : cmul(v[n1], conj2(tw[(t * n1) % N]));
+        for (int n2 = 0; n2 < R2; n2++)
+            S[(t * R2 + n2) * kSpecCols + col] = n2 == 0 ? w[0] : cmul(w[n2], conj2(tw[t * n2]));
     __syncthreads();
-    // inverse, step 2 (thread = n1 = t): DFT over k1 -> x[t + R n2]
+    // inverse, step 2 (thread = n2): DFT over k1 -> x[n2 + R2 n1]
 #pragma unroll
-    for (int k1 = 0; k1 < R; k1++) v[k1] = S[(t * R + k1) * kCols + col];
-    dft<R, N, true>(v, tw);
-    if (valid) {
+    for (int u = 0; u < U; u++) {
+        const int n2 = t + T * u;
 #pragma unroll
-        for (int n2 = 0; n2 < R; n2++) col_t[n2 * step] = v[n2];
+        for (int k1 = 0; k1 < R1; k1++) v[u][k1] = S[(k1 * R2 + n2) * kSpecCols + col];
+        dft<R1, N, true>(v[u], tw);
+        if (valid)
+#pragma unroll
+            for (int n1 = 0; n1 < R1; n1++) p[(n2 + R2 * n1) * ncol] = v[u][n1];
     }
 }
 
-template <int R>
+template <int R1, int R2>
 void launch_r(const Geo &g, int ny, void *spec, const double *twN, const double *kx2, const double *ky2,
               const double *kz2, double invN3, cudaStream_t st)
 {
-    constexpr int N = R * R;
-    constexpr size_t smem = sizeof(double2) * ((size_t)N + (size_t)R * R * kCols);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_pois_i<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
+    constexpr size_t smem = column_smem<R1, R2>();
+    NOVA_SPEC_SMEM((k_pois_i<R1, R2>), smem);
     const int nzh = g.N2 / 2 + 1;
-    const dim3 grid((nzh + kCols - 1) / kCols, ny);
-    k_pois_i<R><<<grid, kCols * R, smem, st>>>(ny, nzh, (double2 *)spec, (const double2 *)twN, kx2, ky2, kz2,
-                                               invN3);
+    const long long ncol = (long long)ny * nzh;
+    k_pois_i<R1, R2><<<(unsigned)((ncol + kSpecCols - 1) / kSpecCols), column_threads<R1, R2>(), smem, st>>>(
+        nzh, ncol, (double2 *)spec, (const double2 *)twN, kx2, ky2, kz2, invN3);
 }
 
 // ---- N0 = 256 on a TMA-fed, double-buffered tile ----
@@ -136,7 +121,7 @@ struct PoisMaps {
 // Tasks t < nmain: j = t / nch, kz = 8 (t % nch) + col (nch = (nzh - 1) / 8);
 // tasks t >= nmain: j = 8 (t - nmain) + col, kz = nzh - 1.  Block b takes
 // tasks b, b + gridDim.x, ...; the load of the next one is issued when the
-// current one starts.  Arithmetic, order and twiddles are k_pois_i<16>'s.
+// current one starts.  Arithmetic, order and twiddles are k_pois_i<16, 16>'s.
 __global__ void __launch_bounds__(kTThreads, 3)
     k_pois_tma(int ny, int nzh, double2 *__restrict__ spec, const double2 *__restrict__ twN,
                const double *__restrict__ kx2, const double *__restrict__ ky2, const double *__restrict__ kz2,
@@ -276,16 +261,20 @@ bool launch_pois_tma(const Geo &g, int ny, void *spec, const double *twN, const 
 
 }  // namespace
 
-bool pois_i_fits(const Geo &g) { return !g.wallY && (g.N0 == 64 || g.N0 == 256); }
+bool pois_i_fits(const Geo &g) { return fft_length(g.N0); }
 
 void launch_pois_i(const Geo &g, int ny, void *spec, const double *twN, const double *kx2, const double *ky2,
                    const double *kz2, double invN3, int *err, cudaStream_t st)
 {
-    if (g.N0 == 256) {
-        if (err && pois_tma_fits(g, ny) && launch_pois_tma(g, ny, spec, twN, kx2, ky2, kz2, invN3, err, st)) return;
-        launch_r<16>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st);
-    } else {
-        launch_r<8>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st);
+    if (g.N0 == 256 && err && pois_tma_fits(g, ny) &&
+        launch_pois_tma(g, ny, spec, twN, kx2, ky2, kz2, invN3, err, st))
+        return;
+    switch (g.N0) {
+#define NOVA_X(l, r1, r2) \
+    case l: launch_r<r1, r2>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st); break;
+        NOVA_FFT_LENGTHS(NOVA_X)
+#undef NOVA_X
+    default: break;
     }
 }
 
