@@ -35,6 +35,14 @@ struct LdSplit {
     {
         return (double)hi[(long long)c * n3 + o] + (double)lo[(long long)c * n3 + o];
     }
+    // the tile march keeps the pair until the value is used: a join at the load
+    // waited for it there (diagnostics at 256^3 447 -> 308 us)
+    using Raw = float2;
+    __device__ __forceinline__ float2 raw(int c, long long o) const
+    {
+        return make_float2(hi[(long long)c * n3 + o], lo[(long long)c * n3 + o]);
+    }
+    static __device__ __forceinline__ double join(float2 v) { return (double)v.x + (double)v.y; }
 };
 
 __device__ __forceinline__ void pt_index(const Geo &g, long long t, int &i, int &j, int &k)

@@ -19,6 +19,8 @@
 
 #include "nova_internal.cuh"
 
+#include <type_traits>
+
 // unroll factor of the plane loop (2H+1 would turn the queue rotation into
 // register renaming, but the extra live ranges cost more than the moves)
 #ifndef NOVA_MARCH_UNROLL
@@ -37,6 +39,20 @@ template <typename T, int H, int NC> constexpr size_t tile_smem_bytes() { return
 
 struct NoPre {
     __device__ void operator()(long long, bool) const {}
+};
+
+// How a march holds a loaded value until it is used: as T, or as the loader's
+// own Raw (two floats of a split field), joined where the value enters the
+// queue or the tile.  A loader without Raw returns T.
+template <typename T, class Ld, class = void> struct MarchLd {
+    using Raw = T;
+    static __device__ __forceinline__ Raw load(const Ld &ld, int c, long long o) { return ld(c, o); }
+    static __device__ __forceinline__ T join(Raw v) { return v; }
+};
+template <typename T, class Ld> struct MarchLd<T, Ld, std::void_t<typename Ld::Raw>> {
+    using Raw = typename Ld::Raw;
+    static __device__ __forceinline__ Raw load(const Ld &ld, int c, long long o) { return ld.raw(c, o); }
+    static __device__ __forceinline__ T join(Raw v) { return Ld::join(v); }
 };
 
 // ld(c, o) returns component c at linear node index o.
@@ -110,8 +126,9 @@ __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, Til
         }
         hoff[s] = (long long)jg * g.N2 + wrapi(k0 + col - H, g.N2);
     }
-    auto hload = [&](int s, int c, long long plane) -> T {
-        const T v = ld(c, plane + hoff[s]);
+    using ML = MarchLd<T, Ld>;
+    auto hval = [&](int s, int c, typename ML::Raw r) -> T {
+        const T v = ML::join(r);
         if constexpr (!WALLS) {
             return v;
         } else {
@@ -125,20 +142,20 @@ __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, Til
     for (int s = 0; s < 2 * H; s++) {
         const long long p = (long long)wrapi(ib - H + s, g.N0) * g.N12 + colOff;
 #pragma unroll
-        for (int c = 0; c < NC; c++) q[s + 1][c] = ld(c, p);
+        for (int c = 0; c < NC; c++) q[s + 1][c] = ML::join(ML::load(ld, c, p));
     }
     // plane index of the queue head, kept wrapped incrementally
     int lead = wrapi(ib + H, g.N0);
-    T qn[NC], hn[HS][NC];
+    typename ML::Raw qn[NC], hn[HS][NC];
     {
         const long long p = (long long)lead * g.N12 + colOff;
         const long long plane = (long long)ib * g.N12;
 #pragma unroll
-        for (int c = 0; c < NC; c++) qn[c] = ld(c, p);
+        for (int c = 0; c < NC; c++) qn[c] = ML::load(ld, c, p);
 #pragma unroll
         for (int s = 0; s < HS; s++)
 #pragma unroll
-            for (int c = 0; c < NC; c++) hn[s][c] = hon[s] ? hload(s, c, plane) : T(0);
+            for (int c = 0; c < NC; c++) hn[s][c] = hon[s] ? ML::load(ld, c, plane + hoff[s]) : typename ML::Raw{};
         if (valid) pre(plane + colOff, true);
     }
 
@@ -151,7 +168,7 @@ __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, Til
             for (int c = 0; c < NC; c++) q[s][c] = q[s + 1][c];
 #pragma unroll
         for (int c = 0; c < NC; c++) {
-            q[2 * H][c] = qn[c];
+            q[2 * H][c] = ML::join(qn[c]);
             if constexpr (WALLS)
                 sm.v[b][c][ty + H][tx + H] = (tside < 0) ? q[H][c] : wall_ghost(wl, 1, c, tl, q[H][c]);
             else
@@ -161,7 +178,7 @@ __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, Til
         for (int s = 0; s < HS; s++)
             if (hon[s])
 #pragma unroll
-                for (int c = 0; c < NC; c++) sm.v[b][c][hrow[s]][hcol[s]] = hn[s][c];
+                for (int c = 0; c < NC; c++) sm.v[b][c][hrow[s]][hcol[s]] = hval(s, c, hn[s][c]);
         __syncthreads();
         const bool more = i + 1 < ie;
         const long long nplane = (long long)(i + 1) * g.N12;
@@ -169,12 +186,12 @@ __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, Til
             lead = (lead + 1 == g.N0) ? 0 : lead + 1;
             const long long p = (long long)lead * g.N12 + colOff;
 #pragma unroll
-            for (int c = 0; c < NC; c++) qn[c] = ld(c, p);
+            for (int c = 0; c < NC; c++) qn[c] = ML::load(ld, c, p);
 #pragma unroll
             for (int s = 0; s < HS; s++)
                 if (hon[s])
 #pragma unroll
-                    for (int c = 0; c < NC; c++) hn[s][c] = hload(s, c, nplane);
+                    for (int c = 0; c < NC; c++) hn[s][c] = ML::load(ld, c, nplane + hoff[s]);
         }
         if (!valid) continue;
         pre(nplane + colOff, more);
