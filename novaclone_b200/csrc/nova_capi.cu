@@ -1265,7 +1265,7 @@ nova_status evolve(nova_ctx *ctx, const nova_run_desc *rd, int phys, nova_field 
                 ProfScope ps(ctx, NOVA_K_STAGE);
                 if (f64)
                     e = launch_stage64(phys, 5, str, g, sw64, ctx->co64, ctx->d_ia64, ctx->d_corr64, rd->dt, visc,
-                                       StageArgs64{Y->d64, X ? X->d64 : nullptr, Old64, nullptr, Us64, kShearW[rk]},
+                                       StageArgs64{Y->d64, X ? X->d64 : nullptr, Old64, nullptr, nullptr, Us64, kShearW[rk]},
                                        st, ex);
                 else {
                     StageArgs32 a{Y->hi, X ? X->hi : nullptr, Oh, Ol, nullptr, nullptr, nullptr, nullptr,
@@ -1338,18 +1338,18 @@ nova_status evolve(nova_ctx *ctx, const nova_run_desc *rd, int phys, nova_field 
             }
         };
         if (lit) {
-            run64(4, StageArgs64{Y->d64, X ? X->d64 : nullptr, nullptr, nullptr, ctx->w64[1]});
+            run64(4, StageArgs64{Y->d64, X ? X->d64 : nullptr, nullptr, nullptr, nullptr, ctx->w64[1]});
             Ustar = ctx->w64[1];
         } else {
-            double *w0 = ctx->w64[0], *w1 = ctx->w64[1], *A = ctx->w64[2];
+            double *w0 = ctx->w64[0], *w1 = ctx->w64[1], *w2 = ctx->w64[2];
             const double *Xp = X ? X->d64 : nullptr;
-            run64(0, StageArgs64{Y->d64, Xp, nullptr, A, w0});
+            run64(0, StageArgs64{Y->d64, Xp, nullptr, nullptr, nullptr, w0});
             fix64(w0);
-            run64(1, StageArgs64{w0, Xp, Y->d64, A, w1});
+            run64(1, StageArgs64{w0, Xp, Y->d64, nullptr, nullptr, w1});
             fix64(w1);
-            run64(2, StageArgs64{w1, Xp, Y->d64, A, w0});
-            fix64(w0);
-            run64(3, StageArgs64{w0, Xp, nullptr, A, Y->d64});
+            run64(2, StageArgs64{w1, Xp, Y->d64, nullptr, nullptr, w2});
+            fix64(w2);
+            run64(3, StageArgs64{w2, Xp, Y->d64, w0, w1, Y->d64});
             Ustar = Y->d64;
         }
         fix64(Ustar);
@@ -1555,8 +1555,8 @@ extern "C" nova_status nova_advance(nova_ctx *ctx, const nova_run_desc *rd, nova
 namespace {
 
 // One classical RK4 loop of the evolved FP64 field Yin with the frozen field X
-// (physics phys, viscosity visc), stage states into S2, S3, S4 (S4 may alias
-// S2); with `full` the stage-3 result and its projection (rhs divisor and
+// (physics phys, viscosity visc), stage states into S2, S3, S4 (three arrays);
+// with `full` the stage-3 result and its projection (rhs divisor and
 // correction scale `div`) into out (may alias Yin).  Without `full` only the
 // stage states are produced.
 nova_status rk_loop64(nova_ctx *ctx, const nova_run_desc *rd, int phys, double visc, double div, const double *Yin,
@@ -1564,7 +1564,6 @@ nova_status rk_loop64(nova_ctx *ctx, const nova_run_desc *rd, int phys, double v
 {
     const Geo &g = ctx->g;
     cudaStream_t st = ctx->stream;
-    double *A = ctx->w64[2];
     const bool str = ctx->md.hyperbolic_z != 0;
     nova_status sst = NOVA_OK;
     auto run = [&](int stage, const StageArgs64 &a) {
@@ -1575,15 +1574,15 @@ nova_status rk_loop64(nova_ctx *ctx, const nova_run_desc *rd, int phys, double v
         if (e != cudaSuccess && sst == NOVA_OK) sst = stage_fail(ctx, e);
         ctx->launches += 1;
     };
-    run(0, StageArgs64{Yin, X, nullptr, A, S2});
-    run(1, StageArgs64{S2, X, Yin, A, S3});
-    run(2, StageArgs64{S3, X, Yin, A, S4});
+    run(0, StageArgs64{Yin, X, nullptr, nullptr, nullptr, S2});
+    run(1, StageArgs64{S2, X, Yin, nullptr, nullptr, S3});
+    run(2, StageArgs64{S3, X, Yin, nullptr, nullptr, S4});
     if (!full) {
         if (sst != NOVA_OK) return sst;
         CKL("stage kernel");
         return NOVA_OK;
     }
-    run(3, StageArgs64{S4, X, nullptr, A, out});
+    run(3, StageArgs64{S4, X, Yin, S2, S3, out});
     if (sst != NOVA_OK) return sst;
     CKL("stage kernel");
     cudaError_t e = launch_div_proj(ctx->h, g, Walls<double>{}, ctx->co64, ctx->d_ia64, out, nullptr, nullptr, div,
@@ -1652,7 +1651,7 @@ nova_status rk_loop32(nova_ctx *ctx, const nova_run_desc *rd, int phys, double v
 }
 
 // One classical RK4 step + projection of an FP64 Navier-Stokes state:
-// Uin -> Uout (may alias), stage states into Y2, Y3, Y4 (Y4 may alias Y2).
+// Uin -> Uout (may alias), stage states into Y2, Y3, Y4.
 // Without `full` only the stage states are produced.
 nova_status fwd_step64(nova_ctx *ctx, const nova_run_desc *rd, const double *Uin, double *Y2, double *Y3, double *Y4,
                        double *Uout, bool full)
@@ -1782,7 +1781,7 @@ extern "C" nova_status nova_adjoint_grad(nova_ctx *ctx, const nova_adj_desc *ad,
             continue;
         }
         const double *src = (n % K == 0) ? ck + V * (n / K) : mu;
-        if ((s = fwd_step64(ctx, rd, src, ctx->w64[0], ctx->w64[1], ctx->w64[0], mu, true)) != NOVA_OK) return s;
+        if ((s = fwd_step64(ctx, rd, src, ctx->w64[0], ctx->w64[1], ctx->w64[2], mu, true)) != NOVA_OK) return s;
         if ((n + 1) % K == 0 && n + 1 < N)
             CK(cudaMemcpyAsync(ck + V * ((n + 1) / K), mu, sizeof(double) * V, cudaMemcpyDeviceToDevice, st));
     }
@@ -1887,7 +1886,7 @@ nova_status adjoint_mhd(nova_ctx *ctx, const nova_adj_desc *ad, const nova_state
     auto St = [&](int t) { return slot(t, 0); };
     auto SB = [&](int t) { return slot(t, 4); };
     cudaStream_t st = ctx->stream;
-    double *w0 = ctx->w64[0], *w1 = ctx->w64[1];
+    double *w0 = ctx->w64[0], *w1 = ctx->w64[1], *w2 = ctx->w64[2];
     double *runU = mu, *runB = Lam;  // running state of the forward pass
 
     // one step; the B loop is projected only when bout is set
@@ -1934,7 +1933,7 @@ nova_status adjoint_mhd(nova_ctx *ctx, const nova_adj_desc *ad, const nova_state
             continue;
         }
         const bool ck = n % K == 0;
-        if ((s = step(ck ? ckU + V * (n / K) : runU, ck ? ckB + V * (n / K) : runB, w0, w1, w0, runU, w0, w1, w0,
+        if ((s = step(ck ? ckU + V * (n / K) : runU, ck ? ckB + V * (n / K) : runB, w0, w1, w2, runU, w0, w1, w2,
                       runB)) != NOVA_OK)
             return s;
         if ((n + 1) % K == 0 && n + 1 < N) {

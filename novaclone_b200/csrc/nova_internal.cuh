@@ -176,8 +176,8 @@ __device__ __forceinline__ T lsum(const V &v, int c, const T *b)
 struct StageArgs64 {
     const double *Y;   // halo'd stage state (3 comps)
     const double *X;   // second halo'd field (MHD), else nullptr
-    const double *U0;  // RK base (stages 1, 2, 5)
-    double *A;         // RK accumulator
+    const double *U0;  // RK base (stages 1, 2, 3, 5)
+    const double *Y1, *Y2;  // the states after stages 0 and 1 (stage 3)
     double *Ynext;     // next stage state, or U* after the last stage (stage 5: U*)
     double w;          // stage 5: the stage's weight
 };

@@ -20,11 +20,11 @@
 // the Mesh::dzdxi_ metric (src/Mesh/Mesh.cpp:147-179).
 //
 // Epilogue (stage s of the classical RK4 of src/settings/settings.cpp:44-51,
-// association order of app/TG_Piosson/RKLoop.H:24-28 kept):
-//   s=0: Y1 = U0 + dU*1/2   A = U0 + dU*1/6
-//   s=1: Y2 = U0 + dU*1/2   A = A  + dU*1/3
-//   s=2: Y3 = U0 + dU       A = A  + dU*1/3
-//   s=3: U* = A  + dU*1/6
+// app/TG_Piosson/RKLoop.H:24-28; rk_store64 and rk_store32):
+//   s=0: Y1 = U0 + dU*1/2
+//   s=1: Y2 = U0 + dU*1/2
+//   s=2: Y3 = U0 + dU
+//   s=3: U* = U0 + the weighted increments
 //   s=4 (the reference loop as written, U not refreshed between stages, so
 //        all four dU are equal): U* = (((U0 + dU/6) + dU/3) + dU/3) + dU/6
 //   s=5 (app/shearLayer/UEqn.H:28-29): U* = U0 + dU*w, w the stage's weight
@@ -76,33 +76,41 @@ __global__ void __launch_bounds__(kThreads, (stage_minb<T, PHYS>())) k_stage(Geo
 #pragma unroll
     for (int c = 0; c < NC; c++) src[c] = ((c < 3) ? args.Y : args.X) + (long long)(c % 3) * g.N3;
 
-    // pointwise epilogue operands (base, accumulator): prefetched one plane
-    // ahead in FP64 and in the FP32 shear-layer stage (5: base hi and lo, the
-    // latter in the accumulator's place); the other FP32 stages load them at
-    // the start of the plane (measured faster there: fewer live registers)
-    constexpr bool kSplit5 = !std::is_same<T, double>::value && STAGE == 5;
-    constexpr bool kE0 = (STAGE == 1 || STAGE == 2 || STAGE == 5) || (!std::is_same<T, double>::value && STAGE == 3);
-    constexpr bool kE1 = (STAGE >= 1 && STAGE <= 3) || kSplit5;
-    constexpr bool kAhead = std::is_same<T, double>::value || kSplit5;
-    const T *e0p = nullptr, *e1p = nullptr;
-    if constexpr (std::is_same<T, double>::value) {
+    // pointwise epilogue operands: FP64 the base (stages 1, 2, 3, 5) and, in the
+    // last stage, Y1 and Y2; split the base and the accumulator.  Prefetched one
+    // plane ahead where they are few (FP64 but the last stage; split in the
+    // shear-layer stage, 5: base hi and lo, the
+    // latter in the accumulator's place), else loaded at the start of the plane
+    // (measured faster there: fewer live registers)
+    constexpr bool kF64 = std::is_same<T, double>::value;
+    constexpr bool kSplit5 = !kF64 && STAGE == 5;
+    constexpr bool kE0 = STAGE == 1 || STAGE == 2 || STAGE == 3 || STAGE == 5;
+    constexpr bool kE1 = kF64 ? STAGE == 3 : ((STAGE >= 1 && STAGE <= 3) || kSplit5);
+    constexpr bool kE2 = kF64 && STAGE == 3;
+    constexpr bool kAhead = (kF64 && STAGE != 3) || kSplit5;
+    const T *e0p = nullptr, *e1p = nullptr, *e2p = nullptr;
+    if constexpr (kF64) {
         e0p = args.U0;
-        e1p = args.A;
+        e1p = args.Y1;
+        e2p = args.Y2;
     } else {
         e0p = args.U0hi;
         e1p = kSplit5 ? args.U0lo : args.A;
     }
-    T e0[3] = {0, 0, 0}, e1[3] = {0, 0, 0}, e0n[3] = {0, 0, 0}, e1n[3] = {0, 0, 0};
+    T e0[3] = {0, 0, 0}, e1[3] = {0, 0, 0}, e2[3] = {0, 0, 0};
+    T e0n[3] = {0, 0, 0}, e1n[3] = {0, 0, 0}, e2n[3] = {0, 0, 0};
     auto pre = [&](long long nidx, bool load) {
         if constexpr (kAhead) {
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 e0[c] = e0n[c];
                 e1[c] = e1n[c];
+                e2[c] = e2n[c];
                 if (load) {
                     const long long o = (long long)c * g.N3 + nidx;
                     if constexpr (kE0) e0n[c] = e0p[o];
                     if constexpr (kE1) e1n[c] = e1p[o];
+                    if constexpr (kE2) e2n[c] = e2p[o];
                 }
             }
         }
@@ -117,6 +125,7 @@ __global__ void __launch_bounds__(kThreads, (stage_minb<T, PHYS>())) k_stage(Geo
                     const long long o = (long long)c * g.N3 + idx;
                     if constexpr (kE0) e0[c] = e0p[o];
                     if constexpr (kE1) e1[c] = e1p[o];
+                    if constexpr (kE2) e2[c] = e2p[o];
                 }
             }
             T rhs[3], divu;
@@ -138,7 +147,7 @@ __global__ void __launch_bounds__(kThreads, (stage_minb<T, PHYS>())) k_stage(Geo
             if constexpr (std::is_same<T, double>::value) {
 #pragma unroll
                 for (int c = 0; c < 3; c++)
-                    rk_store64<STAGE>(args, (long long)c * g.N3 + idx, q[H][c], e0[c], e1[c], dt * rhs[c]);
+                    rk_store64<STAGE>(args, (long long)c * g.N3 + idx, q[H][c], e0[c], e1[c], e2[c], dt * rhs[c]);
             } else {
 #pragma unroll
                 for (int c = 0; c < 3; c++) {

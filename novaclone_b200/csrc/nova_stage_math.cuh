@@ -185,49 +185,41 @@ __device__ __forceinline__ void mhd_rhs(const VX &vx, const VY &vy, const VZ &vz
 }
 
 // Stage update of one component at node o (classical RK4 of
-// src/settings/settings.cpp:44-51 in the association order of
-// app/TG_Piosson/RKLoop.H:24-28; STAGE 4 = the loop as written, one dU):
-//   s=0: Y1 = U0 + dU*1/2   A = U0 + dU*1/6
-//   s=1: Y2 = U0 + dU*1/2   A = A  + dU*1/3
-//   s=2: Y3 = U0 + dU       A = A  + dU*1/3
-//   s=3: U* = A  + dU*1/6
+// src/settings/settings.cpp:44-51, app/TG_Piosson/RKLoop.H:24-28; STAGE 4 = the
+// loop as written, one dU):
+//   s=0: Y1 = U0 + dU*1/2
+//   s=1: Y2 = U0 + dU*1/2
+//   s=2: Y3 = U0 + dU
+//   s=3: U* = U0 + [(Y1 - U0) + 2 (Y2 - U0) + (Y3 - U0)]*1/3 + dU*1/6
 //   s=5: U* = U0 + dU*w   (app/shearLayer/UEqn.H:28-29, w = RK4[rk] of the stage)
-// y0: the stage state at the node; e0: U0 (stages 1, 2, 5); e1: A (stages 1-3)
-// (every product-sum an explicit fma and the stage-2 sum unfused, so the
-// result does not depend on the compiler's contraction choices)
-template <int STAGE> struct RK64 {
-    // the (Ynext, A) values of one node
-    __device__ __forceinline__ static void eval(const StageArgs64 &a, double y0, double e0, double e1, double du,
-                                                double &yn, double &an)
-    {
-        const double w6 = 1.0 / 6.0, w3 = 1.0 / 3.0;
-        if constexpr (STAGE == 5) {
-            yn = fma(du, a.w, e0);
-        } else if constexpr (STAGE == 4) {
-            yn = fma(du, w6, fma(du, w3, fma(du, w3, fma(du, w6, y0))));
-        } else if constexpr (STAGE == 0) {
-            yn = fma(du, 0.5, y0);
-            an = fma(du, w6, y0);
-        } else if constexpr (STAGE == 1) {
-            yn = fma(du, 0.5, e0);
-            an = fma(du, w3, e1);
-        } else if constexpr (STAGE == 2) {
-            yn = __dadd_rn(e0, du);  // not contracted with du = dt * rhs
-            an = fma(du, w3, e1);
-        } else {
-            yn = fma(du, w6, e1);
-        }
-    }
-    static constexpr bool kA = STAGE <= 2;  // the stage writes the accumulator
-};
-
+// The stage states carry the increments dU = 2 (Y1 - U0), 2 (Y2 - U0), Y3 - U0,
+// so no running sum is kept: 312 instead of 384 bytes per node and step (the
+// sum was written by stages 0-2 and read by stages 1-3), and one rounding each
+// of Y1, Y2, Y3 and U* instead of four of the sum.
+// y0: the stage state at the node; e0: U0 (stages 1, 2, 3, 5); e1, e2: Y1, Y2 (stage 3)
+// (every product-sum an explicit fma and the stage-2 and last sums unfused, so
+// the result does not depend on the compiler's contraction choices)
 template <int STAGE>
-__device__ __forceinline__ void rk_store64(const StageArgs64 &a, long long o, double y0, double e0, double e1, double du)
+__device__ __forceinline__ void rk_store64(const StageArgs64 &a, long long o, double y0, double e0, double e1,
+                                           double e2, double du)
 {
-    double yn, an;
-    RK64<STAGE>::eval(a, y0, e0, e1, du, yn, an);
+    const double w6 = 1.0 / 6.0, w3 = 1.0 / 3.0;
+    double yn;
+    if constexpr (STAGE == 5) {
+        yn = fma(du, a.w, e0);
+    } else if constexpr (STAGE == 4) {
+        yn = fma(du, w6, fma(du, w3, fma(du, w3, fma(du, w6, y0))));
+    } else if constexpr (STAGE == 0) {
+        yn = fma(du, 0.5, y0);
+    } else if constexpr (STAGE == 1) {
+        yn = fma(du, 0.5, e0);
+    } else if constexpr (STAGE == 2) {
+        yn = __dadd_rn(e0, du);  // not contracted with du = dt * rhs
+    } else {
+        const double inc = fma(2.0, e2 - e0, (e1 - e0) + (y0 - e0));
+        yn = __dadd_rn(e0, fma(du, w6, __dmul_rn(inc, w3)));
+    }
     a.Ynext[o] = yn;
-    if constexpr (RK64<STAGE>::kA) a.A[o] = an;
 }
 
 // FP32-split: A is an FP32 sum of increments; the last stage (3, 4, or the

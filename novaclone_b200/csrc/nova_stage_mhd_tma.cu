@@ -39,7 +39,7 @@ template <typename T> struct MhdCfg {
     static constexpr int kWarps = TJ;
     static constexpr int kThreads = kTK * (TJ + 1);
     static constexpr int kRing = 7;
-    static constexpr int kERing = 3;
+    template <int NE> static constexpr int kERing = (sizeof(T) == 8 && NE == 3) ? 2 : 3;
     static constexpr int kTcbE = (TJ + 2 * kH) * kRowE;  // one field's halo'd rows
     static constexpr int kLRE = 3 * TJ * 4;              // one field's k halo, one side
     static constexpr int kFieldE = kTcbE + 2 * kLRE;
@@ -49,12 +49,12 @@ template <typename T> struct MhdCfg {
 };
 
 // epilogue operands per stage, in load order (as nova_stage_tma.cu):
-//   FP64:  s=1,2: U0, A   s=3: A
+//   FP64:  s=1,2: U0   s=3: U0, Y1, Y2
 //   split: s=1,2: U0hi, A   s=3: U0hi, A, U0lo   s=4: U0lo
 template <typename T, int STAGE> __host__ __device__ constexpr int mhd_epi_fields()
 {
     if constexpr (sizeof(T) == 8)
-        return (STAGE == 1 || STAGE == 2) ? 2 : (STAGE == 3 ? 1 : 0);
+        return (STAGE == 1 || STAGE == 2) ? 1 : (STAGE == 3 ? 3 : 0);
     else
         return (STAGE == 1 || STAGE == 2) ? 2 : (STAGE == 3 ? 3 : (STAGE == 4 ? 1 : 0));
 }
@@ -62,8 +62,8 @@ template <typename T, int STAGE> __host__ __device__ constexpr int mhd_epi_field
 template <typename T, int NE> constexpr size_t mhd_smem_bytes()
 {
     using C = MhdCfg<T>;
-    return ((size_t)C::kRing * C::kSlotE + (size_t)C::kERing * NE * C::kEpiE) * sizeof(T) +
-           8 * (2 * C::kRing + 2 * C::kERing);
+    constexpr int ering = C::template kERing<NE>;
+    return ((size_t)C::kRing * C::kSlotE + (size_t)ering * NE * C::kEpiE) * sizeof(T) + 8 * (2 * C::kRing + 2 * ering);
 }
 
 struct MhdMaps {
@@ -76,17 +76,14 @@ struct MhdMaps {
 template <typename T, int STAGE, int EPI_E>
 __device__ __forceinline__ void mhd_epi_read(const T *se, int c, T &e0, T &e1, T &lo)
 {
+    // lo: the third operand (split: U0lo, FP64: Y2)
     if constexpr (STAGE == 1 || STAGE == 2) {
         e0 = se[c * kTK];
-        e1 = se[EPI_E + c * kTK];
+        if constexpr (sizeof(T) == 4) e1 = se[EPI_E + c * kTK];
     } else if constexpr (STAGE == 3) {
-        if constexpr (sizeof(T) == 8) {
-            e1 = se[c * kTK];
-        } else {
-            e0 = se[c * kTK];
-            e1 = se[EPI_E + c * kTK];
-            lo = se[2 * EPI_E + c * kTK];
-        }
+        e0 = se[c * kTK];
+        e1 = se[EPI_E + c * kTK];
+        lo = se[2 * EPI_E + c * kTK];
     } else if constexpr (STAGE == 4 && sizeof(T) == 4) {
         lo = se[c * kTK];
     }
@@ -98,9 +95,9 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
               T visc, Args args, const __grid_constant__ MhdMaps maps, int ichunk, int *err)
 {
     using C = MhdCfg<T>;
-    constexpr int H = kH, TJ = C::TJ, kRing = C::kRing, kERing = C::kERing;
-    constexpr int kTcbE = C::kTcbE, kLRE = C::kLRE, kFieldE = C::kFieldE, kSlotE = C::kSlotE, kEpiE = C::kEpiE;
     constexpr int NE = mhd_epi_fields<T, STAGE>();
+    constexpr int H = kH, TJ = C::TJ, kRing = C::kRing, kERing = C::template kERing<NE>;
+    constexpr int kTcbE = C::kTcbE, kLRE = C::kLRE, kFieldE = C::kFieldE, kSlotE = C::kSlotE, kEpiE = C::kEpiE;
     constexpr uint32_t kSlotBytes = kSlotE * sizeof(T), kRowBytes = kRowE * sizeof(T), kEpiBytes = kEpiE * sizeof(T);
     constexpr uint32_t kLRBoxBytes = 3 * kLRB * 4 * sizeof(T), kFieldBytes = kFieldE * sizeof(T);
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -278,7 +275,7 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
         for (int c = 0; c < 3; c++) {
             const long long o = (long long)c * g.N3 + idx;
             if constexpr (sizeof(T) == 8)
-                rk_store64<STAGE>(args, o, y0[c], e0[c], e1[c], dt * rhs[c]);
+                rk_store64<STAGE>(args, o, y0[c], e0[c], e1[c], lo[c], dt * rhs[c]);
             else
                 rk_store32<STAGE>(args, o, y0[c], e0[c], e1[c], lo[c], dt * rhs[c]);
         }
@@ -401,11 +398,10 @@ cudaError_t launch_mhd_tma64(int phys, int stage, bool stretch, const Geo &g, co
                              cudaStream_t st)
 {
     const double *ef[3] = {nullptr, nullptr, nullptr};
-    if (stage == 1 || stage == 2) {
-        ef[0] = a.U0;
-        ef[1] = a.A;
-    } else if (stage == 3) {
-        ef[0] = a.A;
+    if (stage >= 1 && stage <= 3) ef[0] = a.U0;
+    if (stage == 3) {
+        ef[1] = a.Y1;
+        ef[2] = a.Y2;
     }
     return launch_mhd_any<double>(phys, stage, stretch, g, co, ia, corr2, dt, visc, a, a.X, ef, err, st);
 }

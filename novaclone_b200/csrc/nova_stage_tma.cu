@@ -58,7 +58,8 @@ template <typename T> struct TmaCfg {
     static constexpr int kThreads = kTK * (kWarps + 1);          // plus the producer warp
     static constexpr int kBlocksPerSM = sizeof(T) == 8 ? 1 : 3;
     static constexpr int kRing = 7;   // stencil slots: the queue head runs kRing - 2H - 1 planes behind the loads
-    static constexpr int kERing = 3;  // epilogue slots
+    // epilogue slots (two for the FP64 last stage, whose three fields leave no room for a third)
+    template <int NE> static constexpr int kERing = (sizeof(T) == 8 && NE == 3) ? 2 : 3;
     static constexpr int kTcbE = (TJ + 2 * kH) * kRowE;
     static constexpr int kLRE = 3 * TJ * 4;           // the k-halo boxes of one side
     static constexpr int kSlotE = kTcbE + 2 * kLRE;   // elements per stencil slot
@@ -68,12 +69,12 @@ template <typename T> struct TmaCfg {
 };
 
 // epilogue operands per stage, in load order
-//   FP64:  s=1,2: U0, A   s=3: A   s=5: U0
+//   FP64:  s=1,2,5: U0   s=3: U0, Y1, Y2
 //   split: s=1,2: U0hi, A   s=3: U0hi, A, U0lo   s=4: U0lo   s=5: U0hi, U0lo
 template <typename T, int STAGE> __host__ __device__ constexpr int epi_fields()
 {
     if constexpr (sizeof(T) == 8)
-        return (STAGE == 1 || STAGE == 2) ? 2 : ((STAGE == 3 || STAGE == 5) ? 1 : 0);
+        return (STAGE == 1 || STAGE == 2 || STAGE == 5) ? 1 : (STAGE == 3 ? 3 : 0);
     else
         return (STAGE == 1 || STAGE == 2 || STAGE == 5) ? 2 : (STAGE == 3 ? 3 : (STAGE == 4 ? 1 : 0));
 }
@@ -84,8 +85,8 @@ template <typename T, int STAGE> __host__ __device__ constexpr int epi_fields()
 template <typename T, int NE, bool DIAG = false> constexpr size_t tma_smem_bytes()
 {
     using C = TmaCfg<T>;
-    return ((size_t)C::kRing * C::kSlotE + (size_t)C::kERing * NE * C::kEpiE) * sizeof(T) +
-           8 * (2 * C::kRing + 2 * C::kERing) + (DIAG ? 8 * (kDiagParts + 6 * kTK) * C::kWarps : 0);
+    constexpr int ering = C::template kERing<NE>;
+    return ((size_t)C::kRing * C::kSlotE + (size_t)ering * NE * C::kEpiE) * sizeof(T) + 8 * (2 * C::kRing + 2 * ering) + (DIAG ? 8 * (kDiagParts + 6 * kTK) * C::kWarps : 0);
 }
 
 struct StageMaps {
@@ -95,24 +96,14 @@ struct StageMaps {
     CUtensorMap e[3];              // epilogue operands
 };
 
-template <typename T, int STAGE, int EPI_E>
-__device__ __forceinline__ void epi_read(const T *se, int c, T &e0, T &e1, T &lo)
+// FP64: the operands of component c, in load order
+template <int STAGE, int EPI_E>
+__device__ __forceinline__ void epi_read(const double *se, int c, double &e0, double &e1, double &e2)
 {
-    if constexpr (STAGE == 1 || STAGE == 2) {
-        e0 = se[c * kTK];
+    e0 = se[c * kTK];
+    if constexpr (STAGE == 3) {
         e1 = se[EPI_E + c * kTK];
-    } else if constexpr (STAGE == 3) {
-        if constexpr (sizeof(T) == 8) {
-            e1 = se[c * kTK];
-        } else {
-            e0 = se[c * kTK];
-            e1 = se[EPI_E + c * kTK];
-            lo = se[2 * EPI_E + c * kTK];
-        }
-    } else if constexpr (STAGE == 4 && sizeof(T) == 4) {
-        lo = se[c * kTK];
-    } else if constexpr (STAGE == 5 && sizeof(T) == 8) {
-        e0 = se[c * kTK];
+        e2 = se[2 * EPI_E + c * kTK];
     }
 }
 
@@ -137,9 +128,9 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
     static_assert(!(DIAG && WALLS), "diagnostics on periodic meshes");
     static_assert(!WALLS || sizeof(T) == 4, "FP64 wall stages run the register-queue march");
     using C = TmaCfg<T>;
-    constexpr int H = kH, TJ = C::TJ, kRing = C::kRing, kERing = C::kERing;
-    constexpr int kTcbE = C::kTcbE, kLRE = C::kLRE, kSlotE = C::kSlotE, kEpiE = C::kEpiE;
     constexpr int NE = epi_fields<T, STAGE>();
+    constexpr int H = kH, TJ = C::TJ, kRing = C::kRing, kERing = C::template kERing<NE>;
+    constexpr int kTcbE = C::kTcbE, kLRE = C::kLRE, kSlotE = C::kSlotE, kEpiE = C::kEpiE;
     constexpr uint32_t kSlotBytes = kSlotE * sizeof(T), kRowBytes = kRowE * sizeof(T), kEpiBytes = kEpiE * sizeof(T);
     constexpr uint32_t kLRBoxBytes = 3 * kLRB * 4 * sizeof(T);
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -310,7 +301,7 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
             }
             release(empty(cur % kRing));  // the slot's values are in registers
 
-            T e0[3] = {0, 0, 0}, e1[3] = {0, 0, 0}, lo[3] = {0, 0, 0};
+            T e0[3] = {0, 0, 0}, e1[3] = {0, 0, 0}, e2[3] = {0, 0, 0};
             if constexpr (NE > 0) {
                 ok = mbar_wait(efull(p % kERing), (p / kERing) & 1, err);
                 if (!__all_sync(0xffffffffu, ok)) {
@@ -319,17 +310,14 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
                 }
                 const T *se = ering + (p % kERing) * NE * kEpiE + ty * kRowE + tx;
 #pragma unroll
-                for (int c = 0; c < 3; c++) epi_read<T, STAGE, kEpiE>(se, c, e0[c], e1[c], lo[c]);
+                for (int c = 0; c < 3; c++) epi_read<STAGE, kEpiE>(se, c, e0[c], e1[c], e2[c]);
                 release(eempty(p % kERing));
             }
             const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 const long long o = (long long)c * g.N3 + idx;
-                if constexpr (sizeof(T) == 8)
-                    rk_store64<STAGE>(args, o, q[H][c], e0[c], e1[c], dt * rhs[c]);
-                else
-                    rk_store32<STAGE>(args, o, q[H][c], e0[c], e1[c], lo[c], dt * rhs[c]);
+                rk_store64<STAGE>(args, o, q[H][c], e0[c], e1[c], e2[c], dt * rhs[c]);
             }
         }
     } else {
@@ -621,13 +609,10 @@ cudaError_t launch_stage_tma64(int stage, bool stretch, const Geo &g, const Wall
                                int *err, cudaStream_t st, const StageDiag *dg, bool *dg_done)
 {
     const double *ef[3] = {nullptr, nullptr, nullptr};
-    if (stage == 1 || stage == 2) {
-        ef[0] = a.U0;
-        ef[1] = a.A;
-    } else if (stage == 3) {
-        ef[0] = a.A;
-    } else if (stage == 5) {
-        ef[0] = a.U0;
+    if (stage == 1 || stage == 2 || stage == 3 || stage == 5) ef[0] = a.U0;
+    if (stage == 3) {
+        ef[1] = a.Y1;
+        ef[2] = a.Y2;
     }
     if (dg && !stretch && !wl.on && (stage == 0 || stage == 4)) {
         using Cf = TmaCfg<double>;
