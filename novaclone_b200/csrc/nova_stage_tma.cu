@@ -46,7 +46,8 @@ constexpr int kRowE = 3 * kTK;  // one halo'd row, three components
 constexpr int kLRB = 8;         // rows of one k-halo box
 
 // Tile and ring configuration per precision.  FP64: a 32 x 16 tile, one block
-// per SM, one consumer warp per tile row.  FP32: a 32 x 8 tile, three blocks
+// per SM, one consumer warp per tile row and a warpgroup of which one warp
+// produces.  FP32: a 32 x 8 tile, three blocks
 // per SM, one consumer warp per two tile rows (a half-warp per row, each lane
 // two adjacent k nodes in the paired f32x2 arithmetic).  Each block also has
 // one producer warp, whose elected lane issues the loads in the order the
@@ -55,7 +56,7 @@ constexpr int kLRB = 8;         // rows of one k-halo box
 template <typename T> struct TmaCfg {
     static constexpr int TJ = sizeof(T) == 8 ? 16 : 8;
     static constexpr int kWarps = sizeof(T) == 8 ? TJ : TJ / 2;  // consumer warps
-    static constexpr int kThreads = kTK * (kWarps + 1);          // plus the producer warp
+    static constexpr int kThreads = kTK * (kWarps + (sizeof(T) == 8 ? 4 : 1));  // plus the producer warp (FP64: its warpgroup)
     static constexpr int kBlocksPerSM = sizeof(T) == 8 ? 1 : 3;
     static constexpr int kRing = 7;   // stencil slots: the queue head runs kRing - 2H - 1 planes behind the loads
     // epilogue slots (two for the FP64 last stage, whose three fields leave no room for a third)
@@ -163,8 +164,9 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
     __syncthreads();
 
     // ---- producer warp: lane 0 issues every load of the block ----
-    if (ty == C::kWarps) {
-        if (lane != 0) return;
+    if (ty >= C::kWarps) {
+        if constexpr (sizeof(T) == 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        if (ty > C::kWarps || lane != 0) return;
         const bool jlo = j0 < H, jhi = j0 + TJ + H > g.N1;
         const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + kTK == g.N2) ? 0 : k0 + kTK;
         auto issue_s = [&](int n) -> bool {  // stencil load n: plane ib - H + n
@@ -238,17 +240,22 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
     };
 
     // i-stencil queue of the centre values of planes cur-3 .. cur+3.
-    // FP64: the queue shifts by one plane per step (q[s] = logical s); the
-    // unrolled form below exceeds the FP64 kernel's 96-register budget.
-    // FP32: plane ib - H + x lives in q[x % 7], so logical plane s (0..2H,
-    // centre H) of step p is q[(p + s) % 7]; the loop is unrolled by 7
-    // (= 2H + 1 = kRing) so that the rotation is register renaming and every
-    // ring slot index is a compile-time constant of the unrolled step.
+    // Plane ib - H + x lives in q[x % 7], so logical plane s (0..2H, centre H)
+    // of step p is q[(p + s) % 7]; the loop is unrolled by 7 (= 2H + 1 = kRing)
+    // so that the rotation is register renaming and every ring slot index is a
+    // compile-time constant of the unrolled step.  FP64 needs more than the 96
+    // registers of a block of 17 warps for it: the producer sits in a warpgroup
+    // of its own that hands its registers to the consumers (96 -> 112; at 96 the
+    // unrolled loop spilled).  256^3, stages 0-3: 254, 277, 277, 317 us with the
+    // queue shifted by moves, 231, 247, 247, 315 us unrolled (byte floors 123,
+    // 184, 184, 307); with the diagnostics in stage 0: 525 -> 439 us.
     // DIAG: the running diagnostics in shared memory (the registers hold the queue)
     double *dred = reinterpret_cast<double *>(smraw + (bar0 - s0) + 8 * (2 * kRing + 2 * kERing));
     DiagAccSm dacc{dred + kDiagParts * C::kWarps + ty * kTK + tx, C::kWarps * kTK};
     if constexpr (DIAG) dacc.init();
     if constexpr (sizeof(T) == 8) {
+        // 16 x 32 x 112 + 4 x 32 x 24 = 60416 registers of the 20 x 32 x 96 = 61440 at launch
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
         const int kw = k0 + tx;
         const T iak = ia[kw];
         const T c2k = STRETCH ? corr2[kw] : T(0);
@@ -264,34 +271,30 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
             }
             const T *sl = ring + (n % kRing) * kSlotE;
 #pragma unroll
-            for (int c = 0; c < 3; c++) q[n + 1][c] = sl[cen + c * kTK];
+            for (int c = 0; c < 3; c++) q[n][c] = sl[cen + c * kTK];
             if (n < H || n >= H + nout) release(empty(n % kRing));  // queue-only plane
         }
-
-        for (int p = 0; p < nout && ok; p++) {
-            const int hd = p + 2 * H;  // queue head: plane ib + p + 3
-            ok = mbar_wait(full(hd % kRing), (hd / kRing) & 1, err);
-            if (!__all_sync(0xffffffffu, ok)) {
-                ok = false;
-                break;
-            }
-#pragma unroll
-            for (int s = 0; s < 2 * H; s++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) q[s][c] = q[s + 1][c];
+        int es = 0, eph = 0;  // epilogue ring slot and phase of step p
+        long long idx = (long long)ib * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
+        // step p = 7 m + R: queue head plane p + 2H, centre plane p + H
+        auto step = [&](auto Rc, int m, int p) -> bool {
+            constexpr int R = decltype(Rc)::value;
+            const int hd = p + 2 * H;
+            constexpr int sHd = (R + 2 * H) % kRing, sCur = (R + H) % kRing;
+            if (!__all_sync(0xffffffffu, mbar_wait(full(sHd), (m + (R + 2 * H) / kRing) & 1, err))) return false;
             {
-                const T *sh = ring + (hd % kRing) * kSlotE;
+                constexpr int kQ = (R + 2 * H) % (2 * H + 1);
+                const T *sh = ring + sHd * kSlotE;
 #pragma unroll
-                for (int c = 0; c < 3; c++) q[2 * H][c] = sh[cen + c * kTK];
-                if (hd >= H + nout) release(empty(hd % kRing));
+                for (int c = 0; c < 3; c++) q[kQ][c] = sh[cen + c * kTK];
+                if (hd >= H + nout) release(empty(sHd));
             }
-
-            const int cur = p + H;
-            const T *sl = ring + (cur % kRing) * kSlotE;
-            auto vx = [&](int c, int s) -> T { return q[H + s][c]; };
+            const T *sl = ring + sCur * kSlotE;
+            constexpr int kC = (R + H) % (2 * H + 1);
+            auto vx = [&](int c, int s) -> T { return q[(R + H + s + 2 * H + 1) % (2 * H + 1)][c]; };
             auto vy = [&](int c, int s) -> T { return sl[cen + s * kRowE + c * kTK]; };
             auto vz = [&](int c, int s) -> T { return sl[zoff(s) + c * kTK]; };
-            const T u0[3] = {q[H][0], q[H][1], q[H][2]};
+            const T u0[3] = {q[kC][0], q[kC][1], q[kC][2]};
             T rhs[3], divu;
             ns_rhs<T, H, STRETCH>(vx, vy, vz, u0, co, sc, iak, c2k, visc, rhs, divu);
             if constexpr (DIAG) {
@@ -299,26 +302,38 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
                 curl_terms<H>(vx, vy, vz, 0, co.a[0], co.a[1], co.a[2], iak, q1, hs);
                 dacc.add(u0, divu, q1, hs);
             }
-            release(empty(cur % kRing));  // the slot's values are in registers
+            release(empty(sCur));  // the slot's values are in registers
 
             T e0[3] = {0, 0, 0}, e1[3] = {0, 0, 0}, e2[3] = {0, 0, 0};
             if constexpr (NE > 0) {
-                ok = mbar_wait(efull(p % kERing), (p / kERing) & 1, err);
-                if (!__all_sync(0xffffffffu, ok)) {
-                    ok = false;
-                    break;
-                }
-                const T *se = ering + (p % kERing) * NE * kEpiE + ty * kRowE + tx;
+                if (!__all_sync(0xffffffffu, mbar_wait(efull(es), eph, err))) return false;
+                const T *se = ering + es * NE * kEpiE + ty * kRowE + tx;
 #pragma unroll
                 for (int c = 0; c < 3; c++) epi_read<STAGE, kEpiE>(se, c, e0[c], e1[c], e2[c]);
-                release(eempty(p % kERing));
+                release(eempty(es));
+                if (++es == kERing) {
+                    es = 0;
+                    eph ^= 1;
+                }
             }
-            const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
 #pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const long long o = (long long)c * g.N3 + idx;
-                rk_store64<STAGE>(args, o, q[H][c], e0[c], e1[c], e2[c], dt * rhs[c]);
-            }
+            for (int c = 0; c < 3; c++)
+                rk_store64<STAGE>(args, (long long)c * g.N3 + idx, u0[c], e0[c], e1[c], e2[c], dt * rhs[c]);
+            idx += g.N12;
+            return true;
+        };
+        using I0 = std::integral_constant<int, 0>;
+        using I1 = std::integral_constant<int, 1>;
+        using I2 = std::integral_constant<int, 2>;
+        using I3 = std::integral_constant<int, 3>;
+        using I4 = std::integral_constant<int, 4>;
+        using I5 = std::integral_constant<int, 5>;
+        using I6 = std::integral_constant<int, 6>;
+        for (int m = 0, p = 0; ok && p < nout; m++, p += kRing) {
+            ok = step(I0{}, m, p) && (p + 1 >= nout || (step(I1{}, m, p + 1) && (p + 2 >= nout ||
+                 (step(I2{}, m, p + 2) && (p + 3 >= nout || (step(I3{}, m, p + 3) && (p + 4 >= nout ||
+                 (step(I4{}, m, p + 4) && (p + 5 >= nout || (step(I5{}, m, p + 5) && (p + 6 >= nout ||
+                 step(I6{}, m, p + 6))))))))))));
         }
     } else {
         // FP32: warp ty computes tile rows 2 ty and 2 ty + 1 (one per half-warp),
@@ -549,7 +564,7 @@ cudaError_t launch_tma(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     }
     const int ch = tma_ichunk<T>(g);
     const dim3 grid(g.N2 / kTK, (g.N1 + Cf::TJ - 1) / Cf::TJ, (g.N0 + ch - 1) / ch);
-    kern<<<grid, dim3(kTK, Cf::kWarps + 1), smem, st>>>(g, co, stage_coef(co, visc), wl, ia, corr2, dt, visc, a, maps,
+    kern<<<grid, dim3(kTK, Cf::kThreads / kTK), smem, st>>>(g, co, stage_coef(co, visc), wl, ia, corr2, dt, visc, a, maps,
                                                      ch, err, dpart);
     return cudaSuccess;
 }
