@@ -39,7 +39,11 @@ namespace {
 constexpr int kH = 3;
 constexpr int TJ = 8;                        // tile rows: one consumer warp per row
 constexpr int kWarps = TJ;
-constexpr int kThreads = kTK * (TJ + 1);     // plus the producer warp
+// plus the producer's warpgroup, which hands its registers to the consumers:
+// 8 x 32 x 232 + 4 x 32 x 24 = 62464 of 12 x 32 x 168 = 64512 at launch (at 168 the
+// unrolled loop spilled 100 B; 256^3, s = 4..1: 579, 705, 716, 655 -> 493, 557, 571,
+// 565 us; MHD pieces at 128^3 100-105 -> 83-90 us)
+constexpr int kThreads = kTK * (TJ + 4);
 constexpr int kRing = 7;
 constexpr int kERing = 3;
 constexpr int kLRB = 8;                      // rows of the k-halo box
@@ -107,8 +111,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
 
     // ---- producer warp: lane 0 issues every load of the block ----
-    if (ty == TJ) {
-        if (lane != 0) return;
+    if (ty >= TJ) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        if (ty > TJ || lane != 0) return;
         const bool jlo = j0 < H, jhi = j0 + TJ + H > g.N1;
         const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + kTK == g.N2) ? 0 : k0 + kTK;
         auto issue_s = [&](int n) -> bool {  // stencil load n: plane ib - H + n
@@ -160,6 +165,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 
     // ---- consumer warps ----
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
     auto release = [&](uint32_t bar) {
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
@@ -309,7 +315,7 @@ cudaError_t launch_adj_s(const Geo &g, const Coef<double> &co, const double *ia,
     }
     const int ch = adj_ichunk(g);
     const dim3 grid(g.N2 / kTK, g.N1 / TJ, (g.N0 + ch - 1) / ch);
-    k_adj_tma<KIND, S><<<grid, dim3(kTK, TJ + 1), smem, st>>>(g, co, ia, dt, nu, a, acc, maps, ch, err);
+    k_adj_tma<KIND, S><<<grid, dim3(kTK, kThreads / kTK), smem, st>>>(g, co, ia, dt, nu, a, acc, maps, ch, err);
     return cudaGetLastError();
 }
 

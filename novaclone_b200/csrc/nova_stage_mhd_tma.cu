@@ -15,7 +15,7 @@
 // as two boxes.  Every mbarrier wait is bounded (nova_tma.cuh).
 //
 // FP64: TJ = 8 (a slot of the two fields is 24 KB, 209 KB with the epilogue
-// ring; one block of 9 warps per SM, up to 224 registers a thread); FP32:
+// ring; one block per SM, 8 consumer warps of 232 registers); FP32:
 // TJ = 16 (20 KB slots, 195 KB; one block of 17 warps).
 #include "nova_internal.cuh"
 #include "nova_stage_math.cuh"
@@ -37,7 +37,10 @@ constexpr int kLRB = 8;         // rows of one k-halo box
 template <typename T> struct MhdCfg {
     static constexpr int TJ = sizeof(T) == 8 ? 8 : 16;
     static constexpr int kWarps = TJ;
-    static constexpr int kThreads = kTK * (TJ + 1);
+    // the producer has a warpgroup of its own, which hands its registers to the
+    // consumers: FP64 8 x 32 x 232 + 4 x 32 x 24 = 62464 of 12 x 32 x 168 = 64512
+    // at launch, FP32 16 x 32 x 112 + 4 x 32 x 24 = 60416 of 20 x 32 x 96 = 61440
+    static constexpr int kThreads = kTK * (TJ + 4);
     static constexpr int kRing = 7;
     template <int NE> static constexpr int kERing = (sizeof(T) == 8 && NE == 3) ? 2 : 3;
     static constexpr int kTcbE = (TJ + 2 * kH) * kRowE;  // one field's halo'd rows
@@ -130,8 +133,9 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
     __syncthreads();
 
     // ---- producer warp: lane 0 issues every load of the block ----
-    if (ty == TJ) {
-        if (lane != 0) return;
+    if (ty >= TJ) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        if (ty > TJ || lane != 0) return;
         const bool jlo = j0 < H, jhi = j0 + TJ + H > g.N1;
         const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + kTK == g.N2) ? 0 : k0 + kTK;
         auto issue_s = [&](int n) -> bool {  // stencil load n: plane ib - H + n, both fields
@@ -204,6 +208,11 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
     const T iak = ia[kw];
     const T c2k = STRETCH ? corr2[kw] : T(0);
 
+    if constexpr (sizeof(T) == 8)
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    else
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+
     // slot offsets within a field: centre, and the k neighbour at s (inside the
     // row box or in the left/right halo boxes); component stride kTK in both
     const int cen = (H + ty) * kRowE + tx;
@@ -215,6 +224,13 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
     // component c (0-2 the stage field, 3-5 the frozen one) within a slot
     auto fc = [](int c) -> int { return (c / 3) * kFieldE + (c % 3) * kTK; };
 
+    // i-stencil queue: plane ib - H + x lives in q[x % 7], so logical plane s of
+    // step p is q[(p + s) % 7]; the loop is unrolled by the queue period, which
+    // makes the rotation register renaming and every ring slot a compile-time
+    // constant.  128^3, B loop stages 0-3: 76, 84, 83, 88 us with the queue shifted
+    // by moves, 71, 77, 77, 83 us unrolled; jet 192 x 192 x 384 FP32: 266, 287, 287,
+    // 306 -> 249, 274, 273, 286 us (FP64 at 168 registers spilled: 100 us)
+    static_assert(kRing == 2 * H + 1, "queue rotation and ring slots share one period");
     T q[2 * H + 1][6];
     bool ok = true;
     for (int n = 0; n < 2 * H; n++) {  // queue: planes ib-3 .. ib+2
@@ -225,52 +241,48 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
         }
         const T *sl = ring + (n % kRing) * kSlotE;
 #pragma unroll
-        for (int c = 0; c < 6; c++) q[n + 1][c] = sl[cen + fc(c)];
+        for (int c = 0; c < 6; c++) q[n][c] = sl[cen + fc(c)];
         if (n < H || n >= H + nout) release(empty(n % kRing));  // queue-only plane
     }
 
-    for (int p = 0; p < nout && ok; p++) {
-        const int hd = p + 2 * H;  // queue head: plane ib + p + 3
-        ok = mbar_wait(full(hd % kRing), (hd / kRing) & 1, err);
-        if (!__all_sync(0xffffffffu, ok)) {
-            ok = false;
-            break;
-        }
-#pragma unroll
-        for (int s = 0; s < 2 * H; s++)
-#pragma unroll
-            for (int c = 0; c < 6; c++) q[s][c] = q[s + 1][c];
+    int es = 0, eph = 0;  // epilogue ring slot and phase of step p
+    long long idx = (long long)ib * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
+    // step p = 7 m + R: queue head plane p + 2H, centre plane p + H
+    auto step = [&](auto Rc, int m, int p) -> bool {
+        constexpr int R = decltype(Rc)::value;
+        constexpr int sHd = (R + 2 * H) % kRing, sCur = (R + H) % kRing;
+        const int hd = p + 2 * H;
+        if (!__all_sync(0xffffffffu, mbar_wait(full(sHd), (m + (R + 2 * H) / kRing) & 1, err))) return false;
         {
-            const T *sh = ring + (hd % kRing) * kSlotE;
+            constexpr int kQ = (R + 2 * H) % (2 * H + 1);
+            const T *sh = ring + sHd * kSlotE;
 #pragma unroll
-            for (int c = 0; c < 6; c++) q[2 * H][c] = sh[cen + fc(c)];
-            if (hd >= H + nout) release(empty(hd % kRing));
+            for (int c = 0; c < 6; c++) q[kQ][c] = sh[cen + fc(c)];
+            if (hd >= H + nout) release(empty(sHd));
         }
-
-        const int cur = p + H;
-        const T *sl = ring + (cur % kRing) * kSlotE;
-        auto vx = [&](int c, int s) -> T { return q[H + s][c]; };
+        const T *sl = ring + sCur * kSlotE;
+        constexpr int kC = (R + H) % (2 * H + 1);
+        auto vx = [&](int c, int s) -> T { return q[(R + H + s + 2 * H + 1) % (2 * H + 1)][c]; };
         auto vy = [&](int c, int s) -> T { return sl[cen + s * kRowE + fc(c)]; };
         auto vz = [&](int c, int s) -> T { return sl[zoff(s) + fc(c)]; };
-        const T y0[3] = {q[H][0], q[H][1], q[H][2]};
-        const T x0[3] = {q[H][3], q[H][4], q[H][5]};
+        const T y0[3] = {q[kC][0], q[kC][1], q[kC][2]};
+        const T x0[3] = {q[kC][3], q[kC][4], q[kC][5]};
         T rhs[3];
         mhd_rhs<T, H, STRETCH, PHYS == PHYS_MHD_U>(vx, vy, vz, y0, x0, co, sc, iak, c2k, visc, rhs);
-        release(empty(cur % kRing));  // the slot's values are in registers
+        release(empty(sCur));  // the slot's values are in registers
 
         T e0[3] = {0, 0, 0}, e1[3] = {0, 0, 0}, lo[3] = {0, 0, 0};
         if constexpr (NE > 0) {
-            ok = mbar_wait(efull(p % kERing), (p / kERing) & 1, err);
-            if (!__all_sync(0xffffffffu, ok)) {
-                ok = false;
-                break;
-            }
-            const T *se = ering + (p % kERing) * NE * kEpiE + ty * kRowE + tx;
+            if (!__all_sync(0xffffffffu, mbar_wait(efull(es), eph, err))) return false;
+            const T *se = ering + es * NE * kEpiE + ty * kRowE + tx;
 #pragma unroll
             for (int c = 0; c < 3; c++) mhd_epi_read<T, STAGE, kEpiE>(se, c, e0[c], e1[c], lo[c]);
-            release(eempty(p % kERing));
+            release(eempty(es));
+            if (++es == kERing) {
+                es = 0;
+                eph ^= 1;
+            }
         }
-        const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             const long long o = (long long)c * g.N3 + idx;
@@ -279,6 +291,21 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
             else
                 rk_store32<STAGE>(args, o, y0[c], e0[c], e1[c], lo[c], dt * rhs[c]);
         }
+        idx += g.N12;
+        return true;
+    };
+    using I0 = std::integral_constant<int, 0>;
+    using I1 = std::integral_constant<int, 1>;
+    using I2 = std::integral_constant<int, 2>;
+    using I3 = std::integral_constant<int, 3>;
+    using I4 = std::integral_constant<int, 4>;
+    using I5 = std::integral_constant<int, 5>;
+    using I6 = std::integral_constant<int, 6>;
+    for (int m = 0, p = 0; ok && p < nout; m++, p += kRing) {
+        ok = step(I0{}, m, p) && (p + 1 >= nout || (step(I1{}, m, p + 1) && (p + 2 >= nout ||
+             (step(I2{}, m, p + 2) && (p + 3 >= nout || (step(I3{}, m, p + 3) && (p + 4 >= nout ||
+             (step(I4{}, m, p + 4) && (p + 5 >= nout || (step(I5{}, m, p + 5) && (p + 6 >= nout ||
+             step(I6{}, m, p + 6))))))))))));
     }
 }
 
@@ -356,7 +383,7 @@ cudaError_t launch_mhd(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     }
     const int ch = mhd_ichunk<T>(g);
     const dim3 grid(g.N2 / kTK, g.N1 / Cf::TJ, (g.N0 + ch - 1) / ch);
-    kern<<<grid, dim3(kTK, Cf::TJ + 1), smem, st>>>(g, co, stage_coef(co, visc), ia, corr2, dt, visc, a, maps, ch, err);
+    kern<<<grid, dim3(kTK, Cf::kThreads / kTK), smem, st>>>(g, co, stage_coef(co, visc), ia, corr2, dt, visc, a, maps, ch, err);
     return cudaSuccess;
 }
 
