@@ -68,7 +68,7 @@ template <int NE> constexpr size_t adj_smem_bytes()
 }
 
 struct AdjMaps {
-    CUtensorMap f[2][4];  // per field: rows TJ+6, 3, TJ+3, k halos
+    CUtensorMap f[2][5];  // per field: rows TJ+6, 3, TJ+3, k halos, the last j tile's rows and the H before them
     CUtensorMap e[2];     // mu, Lam (or the accumulated adjoint)
 };
 
@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int k0 = blockIdx.x * kTK, j0 = blockIdx.y * TJ;
     const int ib = blockIdx.z * ichunk, ie = min(ib + ichunk, g.N0);
     const int nout = ie - ib, nld = nout + 2 * H;
+    const int w = min(kTK, g.N2 - k0), hrows = min(TJ, g.N1 - j0);  // valid columns and rows of the tile
 
     if (ty == TJ && lane == 0) {
         for (int r = 0; r < kRing; r++) {
@@ -114,13 +115,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (ty >= TJ) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
         if (ty > TJ || lane != 0) return;
-        const bool jlo = j0 < H, jhi = j0 + TJ + H > g.N1;
-        const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + kTK == g.N2) ? 0 : k0 + kTK;
+        const bool jlo = j0 < H, jhi = j0 + TJ >= g.N1;
+        const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + w == g.N2) ? 0 : k0 + kTK;
+        const uint32_t slot_bytes = kSlotBytes - (jhi ? 2 * (TJ - hrows) * kRowBytes : 0);
         auto issue_s = [&](int n) -> bool {  // stencil load n: plane ib - H + n
             const int r = n % kRing;
             if (n >= kRing && !mbar_wait(empty(r), ((n / kRing) + 1) & 1, err)) return false;
             const uint32_t bar = full(r);
-            mbar_expect_tx(bar, kSlotBytes);
+            mbar_expect_tx(bar, slot_bytes);
             const int plane = wrapi(ib - H + n, g.N0);
 #pragma unroll
             for (int f = 0; f < 2; f++) {
@@ -130,8 +132,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                     tma_load_4d(dst, &m[1], bar, k0, 0, g.N1 - H, plane);
                     tma_load_4d(dst + H * kRowBytes, &m[2], bar, k0, 0, 0, plane);
                 } else if (jhi) {
-                    tma_load_4d(dst, &m[2], bar, k0, 0, j0 - H, plane);
-                    tma_load_4d(dst + (TJ + H) * kRowBytes, &m[1], bar, k0, 0, 0, plane);
+                    tma_load_4d(dst, &m[4], bar, k0, 0, j0 - H, plane);
+                    tma_load_4d(dst + (hrows + H) * kRowBytes, &m[1], bar, k0, 0, 0, plane);
                 } else {
                     tma_load_4d(dst, &m[0], bar, k0, 0, j0 - H, plane);
                 }
@@ -170,16 +172,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
     };
-    const int kw = k0 + tx;
+    const bool on = tx < w && ty < hrows;
+    const int txc = min(tx, w - 1);  // lanes past the valid columns read the last one and store nothing
     double az[H], bz[H], bsum;
-    adj_zweights<double, H>(co, ia[kw], az, bz, bsum);
+    adj_zweights<double, H>(co, ia[k0 + txc], az, bz, bsum);
 
     // slot offsets within a field: centre, and the k neighbour at s (row box
     // or the left/right halo boxes, [c][8 rows][4]); component stride kTK in both
-    const int cen = (H + ty) * kRowE + tx;
+    const int cen = (H + ty) * kRowE + txc;
     auto zoff = [&](int s) -> int {
-        const int x = tx + s;
-        return x < 0 ? kTcbE + ty * 4 + 4 + x : (x >= kTK ? kTcbE + kLRE + ty * 4 + (x - kTK) : cen + s);
+        const int x = txc + s;
+        return x < 0 ? kTcbE + ty * 4 + 4 + x : (x >= w ? kTcbE + kLRE + ty * 4 + (x - w) : cen + s);
     };
     auto fo = [](int c) { return (c / 3) * kFieldE + (c % 3) * kTK; };  // field and component offset
 
@@ -256,9 +259,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int c = 0; c < 3; c++) e0[c] = g0[c];  // mu: the g field at s = 4
         }
-        const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
+        const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + ty) * g.N2 + k0 + tx;
 #pragma unroll
         for (int e = 0; e < 3; e++) {
+            if (!on) break;
             const long long o = (long long)e * g.N3 + idx;
             if constexpr (kRec)
                 adj_store<double, S>(args, o, e0[e], e1[e], r[e]);
@@ -284,7 +288,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 int adj_ichunk(const Geo &g)
 {
-    const long long tiles = (long long)(g.N2 / kTK) * (g.N1 / TJ);
+    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + TJ - 1) / TJ);
     return march_chunk(g.N0, tiles, 1, 2.5);
 }
 
@@ -300,7 +304,8 @@ cudaError_t launch_adj_s(const Geo &g, const Coef<double> &co, const double *ia,
     for (int f = 0; f < 2; f++)
         ok = ok && tma_encode_field(&maps.f[f][0], fld[f], g, TJ + 2 * kH) &&
              tma_encode_field(&maps.f[f][1], fld[f], g, kH) && tma_encode_field(&maps.f[f][2], fld[f], g, TJ + kH) &&
-             tma_encode_field(&maps.f[f][3], fld[f], g, 0);
+             tma_encode_field(&maps.f[f][3], fld[f], g, 0) &&
+             tma_encode_field(&maps.f[f][4], fld[f], g, (g.N1 - 1) % TJ + 1 + kH);
     if (KIND == ADJ_NS || KIND == ADJ_BB) {
         if (NE > 0) ok = ok && tma_encode_field(&maps.e[0], a.mu, g, TJ) && tma_encode_field(&maps.e[1], a.Lam, g, TJ);
     } else {
@@ -314,7 +319,7 @@ cudaError_t launch_adj_s(const Geo &g, const Coef<double> &co, const double *ia,
         attr = true;
     }
     const int ch = adj_ichunk(g);
-    const dim3 grid(g.N2 / kTK, g.N1 / TJ, (g.N0 + ch - 1) / ch);
+    const dim3 grid((g.N2 + kTK - 1) / kTK, (g.N1 + TJ - 1) / TJ, (g.N0 + ch - 1) / ch);
     k_adj_tma<KIND, S><<<grid, dim3(kTK, kThreads / kTK), smem, st>>>(g, co, ia, dt, nu, a, acc, maps, ch, err);
     return cudaGetLastError();
 }
@@ -333,7 +338,7 @@ cudaError_t launch_adj_k(int s, const Geo &g, const Coef<double> &co, const doub
 
 }  // namespace
 
-bool adj_tma_fits(const Geo &g) { return !g.wallY && g.N2 % kTK == 0 && g.N1 % TJ == 0 && g.N1 >= 2 * TJ; }
+bool adj_tma_fits(const Geo &g) { return !g.wallY && tma_mesh_fits(g, 2, TJ); }
 
 cudaError_t launch_adj_tma64(int kind, int s, const Geo &g, const Coef<double> &co, const double *ia, double dt,
                              double nu, const AdjArgs &a, double *acc, int *err, cudaStream_t st)

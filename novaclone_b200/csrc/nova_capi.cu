@@ -478,7 +478,7 @@ nova_status stage_fail(nova_ctx *ctx, cudaError_t e)
 {
     if (e == cudaErrorNotSupported)
         return fail(ctx, NOVA_E_UNSUPPORTED,
-                    "NOVA_STAGE_IMPL=tma: the TMA stage kernel needs N2 % 32 == 0 and N1 at least twice the tile height (16 rows FP64, 8 FP32), with periodic y a multiple of it; walls in y only in FP32");
+                    "NOVA_STAGE_IMPL=tma: the TMA stage kernel needs N2 >= 32 with whole 16-byte rows and no one or two columns beyond a 32-column tile, and N1 at least twice the tile height (16 rows FP64, 8 FP32) with, for periodic y, no one or two rows beyond a tile; walls in y only in FP32");
     if (e == cudaErrorInvalidValue) return fail(ctx, NOVA_E_CUDA, "stage kernel: cuTensorMapEncodeTiled failed");
     return cuda_check(ctx, e, "stage kernel");
 }

@@ -238,7 +238,7 @@ struct AdjArgs {
     double *LamOut;     // updated running sum (s > 1)
 };
 // err: the pipeline error word; with it, meshes that fit the TMA adjoint
-// (nova_adj_tma.cu: periodic, N2 % 32 == 0, N1 a multiple of 8 and >= 16) run it
+// (nova_adj_tma.cu: periodic, tma_mesh_fits with tiles of 8 rows) run it
 cudaError_t launch_adj_stage64(int s, const Geo &g, const Coef<double> &co, const double *ia, double dt, double nu,
                                const AdjArgs &a, cudaStream_t st, int *err = nullptr);
 bool adj_tma_fits(const Geo &g);
@@ -275,18 +275,28 @@ void launch_dot(long long n, const double *x, const double *y, double scale, dou
                 cudaStream_t st);
 
 // Which kernel runs the Navier-Stokes stage: STAGE_AUTO = the TMA pipeline
-// (nova_stage_tma.cu) where the mesh fits it (stage_tma_fits: N2 % 32 == 0,
-// N1 at least twice the tile height 16 (FP64) or 8 (FP32), and with periodic y
-// a multiple of it; FP32 walls in y take ragged last tiles), else the
-// register-queue march (nova_stage.cu); STAGE_MARCH / STAGE_TMA force one
-// (STAGE_TMA on a mesh that does not fit is an error).  err: device word
-// raised by a pipeline wait that timed out.
+// (nova_stage_tma.cu) where the mesh fits it (stage_tma_fits: tma_mesh_fits with
+// tiles of 16 rows (FP64) or 8 (FP32)), else the register-queue march
+// (nova_stage.cu); STAGE_MARCH / STAGE_TMA force one (STAGE_TMA on a mesh that
+// does not fit, or on FP64 wall stages, is an error).  err: device word raised
+// by a pipeline wait that timed out.
 enum StageImpl { STAGE_AUTO = 0, STAGE_MARCH = 1, STAGE_TMA = 2 };
 struct StageExec {
     int impl;
     int *err;
 };
 bool stage_tma_fits(const Geo &g, bool fp64);
+// Meshes the TMA-fed kernels take: rows a multiple of 16 bytes (N2 a multiple of
+// `align` elements: the bulk copies' strides, and the wrapped start of the left
+// k halo), at least one whole tile along k and two (tj rows) along j.  The last
+// tile of either direction may be ragged, but holds at least the H = 3 nodes
+// the tile before it reads as its halo (in j only where y is periodic).
+inline bool tma_mesh_fits(const Geo &g, int align, int tj)
+{
+    const int wk = g.N2 % kTK, hj = g.N1 % tj;
+    if (g.N2 < kTK || g.N2 % align || wk == 1 || wk == 2) return false;
+    return g.N1 >= 2 * tj && (g.wallY || (hj != 1 && hj != 2));
+}
 // tensor map of a 3-component FP64 field [c][i][j][k] (nova_stage_tma.cu):
 // rows > 0: box kTK(k) x 3(c) x rows(j) x 1(i), landing [row][c][k];
 // rows = 0: the 4-wide k-halo box 4(k) x 8(j) x 3(c) x 1(i), landing [c][j][k]
@@ -327,8 +337,7 @@ cudaError_t launch_stage_tma64(int stage, bool stretch, const Geo &g, const Wall
                                const double *ia, const double *corr2, double dt, double visc, const StageArgs64 &a,
                                int *err, cudaStream_t st, const StageDiag *dg = nullptr, bool *dg_done = nullptr);
 // MHD stage kernels on the TMA pipeline (nova_stage_mhd_tma.cu): periodic y,
-// N2 % 32 == 0, N1 a multiple of the tile height 8 (FP64) or 16 (FP32) and at
-// least twice it; a.X is the frozen field
+// tma_mesh_fits with tiles of 8 rows (FP64) or 16 (FP32); a.X is the frozen field
 bool mhd_tma_fits(const Geo &g, bool fp64);
 cudaError_t launch_mhd_tma64(int phys, int stage, bool stretch, const Geo &g, const Coef<double> &co, const double *ia,
                              const double *corr2, double dt, double visc, const StageArgs64 &a, int *err,

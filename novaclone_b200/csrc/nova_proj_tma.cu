@@ -50,12 +50,13 @@ enum {
     M_RB = 3,
     M_C2 = 4,   // DIV: component 2 tile
     M_LR = 5,   // k halo boxes (4 x 8) (DIV: component 2, CORR: p)
-    M_SET = 6,  // maps per field set (DIV split: hi set, then lo set)
-    M_EPI = 12  // CORR: U* (box 32 x 3 x TJ), U*lo at M_EPI + 1
+    M_RR = 6,   // the last j tile's rows and the H before them
+    M_SET = 7,  // maps per field set (DIV split: hi set, then lo set)
+    M_EPI = 14  // CORR: U* (box 32 x 3 x TJ), U*lo at M_EPI + 1
 };
 
 struct ProjMaps {
-    CUtensorMap m[14];
+    CUtensorMap m[16];
 };
 
 template <int MODE, bool SPLIT> struct ProjCfg {
@@ -81,7 +82,7 @@ struct ProjArgs {
     float *hi, *lo;             // CORR output (split)
 };
 
-template <int MODE, bool SPLIT, bool WALLS>
+template <int MODE, bool SPLIT, bool WALLS, bool WHOLE>
 __global__ void __launch_bounds__(kThreads, 2)
     k_proj_tma(Geo g, Coef<double> co, const Walls<double> wl, const double *__restrict__ ia, ProjArgs a,
                const __grid_constant__ ProjMaps maps, int ichunk, int *err)
@@ -106,6 +107,8 @@ __global__ void __launch_bounds__(kThreads, 2)
     const int k0 = blockIdx.x * kTK, j0 = blockIdx.y * TJ;
     const int ib = blockIdx.z * ichunk, ie = min(ib + ichunk, g.N0);
     const int nout = ie - ib, nld = nout + 2 * H;
+    // valid columns and rows of the tile (WHOLE: the mesh has no ragged tile)
+    const int w = WHOLE ? kTK : min(kTK, g.N2 - k0), hrows = WHOLE ? TJ : min(TJ, g.N1 - j0);
 
     if (ty == TJ && lane == 0) {
         for (int r = 0; r < kRing; r++) {
@@ -123,8 +126,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     // ---- producer warp ----
     if (ty == TJ) {
         if (lane != 0) return;
-        const bool jlo = j0 < H, jhi = j0 + TJ + H > g.N1;
-        const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + kTK == g.N2) ? 0 : k0 + kTK;
+        const bool jlo = j0 < H, jhi = j0 + TJ >= g.N1;
+        const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + w == g.N2) ? 0 : k0 + kTK;
+        const uint32_t slot_bytes = C::kSlotBytes - (!WALLS && jhi ? C::kSets * (TJ - hrows) * kRowBytes : 0);
         // rows with j halos of map set `ms` into dst
         auto rows = [&](int ms, uint32_t dst, uint32_t bar, int plane) {
             if (WALLS) {
@@ -133,8 +137,8 @@ __global__ void __launch_bounds__(kThreads, 2)
                 tma_load_3d(dst, &maps.m[ms + M_R3], bar, k0, g.N1 - H, plane);
                 tma_load_3d(dst + H * kRowBytes, &maps.m[ms + M_RB], bar, k0, 0, plane);
             } else if (jhi) {
-                tma_load_3d(dst, &maps.m[ms + M_RB], bar, k0, j0 - H, plane);
-                tma_load_3d(dst + (TJ + H) * kRowBytes, &maps.m[ms + M_R3], bar, k0, 0, plane);
+                tma_load_3d(dst, &maps.m[ms + M_RR], bar, k0, j0 - H, plane);
+                tma_load_3d(dst + (hrows + H) * kRowBytes, &maps.m[ms + M_R3], bar, k0, 0, plane);
             } else {
                 tma_load_3d(dst, &maps.m[ms + M_RA], bar, k0, j0 - H, plane);
             }
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 }
                 return true;
             }
-            mbar_expect_tx(bar, C::kSlotBytes);
+            mbar_expect_tx(bar, slot_bytes);
 #pragma unroll
             for (int set = 0; set < C::kSets; set++) {
                 const uint32_t dst = s0 + r * C::kSlotBytes + set * C::kSetE * sizeof(TS);
@@ -210,25 +214,25 @@ __global__ void __launch_bounds__(kThreads, 2)
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
     };
-    const int kw = k0 + tx;
+    const int txc = WHOLE ? tx : min(tx, w - 1);  // lanes past the valid columns read the last one and store nothing
     double az[H];
 #pragma unroll
-    for (int l = 0; l < H; l++) az[l] = co.a[2][l] * ia[kw];
+    for (int l = 0; l < H; l++) az[l] = co.a[2][l] * ia[k0 + txc];
     // set-relative element offsets of this thread
     constexpr bool DL = C::kDivLoads;
     constexpr int oQ = DL ? 0 : H * kTK;                    // queue value (row ty of the tile)
     constexpr int oY = DL ? kTileE + H * kTK : H * kTK;     // j stencil centre
     constexpr int oZ = DL ? kTileE + kRowsE : H * kTK;      // k stencil centre row
     constexpr int oL = DL ? 2 * kTileE + kRowsE : kRowsE;   // left k halo
-    const int qoff = oQ + ty * kTK + tx, yoff = oY + ty * kTK + tx;
+    const int qoff = oQ + ty * kTK + txc, yoff = oY + ty * kTK + txc;
     // walls: this warp's row, and whether its j stencil reaches across a wall
     // (the component whose j derivative is taken: U*_1 for DIV, p for CORR)
     constexpr int CY = MODE == PROJ_DIV ? 1 : 0;
     const int jrow = j0 + ty;
     const bool nearw = WALLS && jrow < g.N1 && (jrow < H || jrow + H > g.N1 - 1);
     auto zoff = [&](int s) -> int {
-        const int x = tx + s;
-        return x < 0 ? oL + ty * 4 + 4 + x : (x >= kTK ? oL + kLRE + ty * 4 + (x - kTK) : oZ + ty * kTK + x);
+        const int x = txc + s;
+        return x < 0 ? oL + ty * 4 + 4 + x : (x >= w ? oL + kLRE + ty * 4 + (x - w) : oZ + ty * kTK + x);
     };
     auto val = [&](const TS *sl, int o) -> double {
         if constexpr (C::kSets == 2)
@@ -275,8 +279,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         };
         auto vz = [&](int, int s) -> double { return val(sl, zoff(s)); };
         const double dy = (WALLS && nearw) ? d1<double, H>(vyg, CY, co.a[1]) : d1<double, H>(vy, CY, co.a[1]);
-        const bool store = !WALLS || jrow < g.N1;
-        const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
+        const bool store = WHOLE || (tx < w && ty < hrows);
+        const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + ty) * g.N2 + k0 + tx;
         if constexpr (MODE == PROJ_DIV) {
             const double d = d1<double, H>(vx, 0, co.a[0]) + dy + d1<double, H>(vz, 2, az);
             release(empty(cur % kRing));  // the slot's values are in registers
@@ -361,7 +365,8 @@ template <typename T> bool encode4(CUtensorMap *m, const T *base, const Geo &g)
 template <typename T> bool encode_rows(ProjMaps &pm, int ms, const T *f, const Geo &g)
 {
     return encode3(&pm.m[ms + M_RA], f, g, kTK, TJ + 2 * kH) && encode3(&pm.m[ms + M_R3], f, g, kTK, kH) &&
-           encode3(&pm.m[ms + M_RB], f, g, kTK, TJ + kH);
+           encode3(&pm.m[ms + M_RB], f, g, kTK, TJ + kH) &&
+           encode3(&pm.m[ms + M_RR], f, g, kTK, (g.N1 - 1) % TJ + 1 + kH);
 }
 
 // i-chunk.  The 2H warm-up planes of a chunk load the queue's tile rows alone;
@@ -370,7 +375,7 @@ template <typename T> bool encode_rows(ProjMaps &pm, int ms, const T *f, const G
 // 384: 20 planes 129 us, 96 planes 140 us)
 int proj_ichunk(const Geo &g, double tail)
 {
-    const long long tiles = (long long)(g.N2 / kTK) * ((g.N1 + TJ - 1) / TJ);
+    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + TJ - 1) / TJ);
     return march_chunk(g.N0, tiles, 2, 2.5, g.wallY ? 0.45 : tail);
 }
 
@@ -379,15 +384,16 @@ cudaError_t launch_w(const Geo &g, const Coef<double> &co, const Walls<double> &
                      const ProjArgs &a, const ProjMaps &pm, int *err, cudaStream_t st)
 {
     using C = ProjCfg<MODE, SPLIT>;
-    auto kern = k_proj_tma<MODE, SPLIT, WALLS>;
-    static bool attr = false;
-    if (!attr) {
+    const bool whole = !WALLS && g.N2 % kTK == 0 && g.N1 % TJ == 0;
+    auto kern = whole ? k_proj_tma<MODE, SPLIT, WALLS, !WALLS> : k_proj_tma<MODE, SPLIT, WALLS, false>;
+    static bool attr[2] = {false, false};
+    if (!attr[whole]) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        attr = true;
+        attr[whole] = true;
     }
     const int ch = proj_ichunk(g, MODE == PROJ_DIV ? 0.15 : 0.3);
-    const dim3 grid(g.N2 / kTK, (g.N1 + TJ - 1) / TJ, (g.N0 + ch - 1) / ch);
+    const dim3 grid((g.N2 + kTK - 1) / kTK, (g.N1 + TJ - 1) / TJ, (g.N0 + ch - 1) / ch);
     kern<<<grid, dim3(kTK, TJ + 1), C::kSmem, st>>>(g, co, wl, ia, a, pm, ch, err);
     return cudaSuccess;
 }
@@ -402,12 +408,10 @@ cudaError_t launch(const Geo &g, const Coef<double> &co, const Walls<double> &wl
 
 }  // namespace
 
-// tile width divides N2; periodic y: the tile height divides N1; walls in y
-// (the field's ghost BCs on, wl_on): any N1 of at least two tiles
-bool proj_tma_fits(const Geo &g, bool wl_on)
+// (wl_on: the field's wall ghost BCs are on; f32: a field read as FP32 pairs)
+bool proj_tma_fits(const Geo &g, bool wl_on, bool f32)
 {
-    if (wl_on != (g.wallY != 0)) return false;
-    return g.N2 % kTK == 0 && g.N1 >= 2 * TJ && (g.wallY || g.N1 % TJ == 0);
+    return wl_on == (g.wallY != 0) && tma_mesh_fits(g, f32 ? 4 : 2, TJ);
 }
 
 cudaError_t launch_div_tma(const Geo &g, const Coef<double> &co, const Walls<double> &wl, const double *ia,

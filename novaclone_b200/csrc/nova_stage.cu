@@ -220,7 +220,9 @@ cudaError_t launch_stage64(int phys, int stage, bool stretch, const Geo &g, cons
                            const StageArgs64 &a, cudaStream_t st, const StageExec &ex, const StageDiag *dg,
                            bool *dg_done)
 {
-    if (phys == PHYS_NS && ex.impl != STAGE_MARCH && ex.err && stage_tma_fits(g, true))
+    // (forcing the TMA kernel on FP64 wall stages is refused)
+    if (phys == PHYS_NS && ex.impl != STAGE_MARCH && ex.err && stage_tma_fits(g, true) &&
+        !(wl.on && ex.impl == STAGE_TMA))
         return launch_stage_tma64(stage, stretch, g, wl, co, ia, corr2, dt, visc, a, ex.err, st, dg, dg_done);
     if (phys != PHYS_NS && !wl.on && ex.impl != STAGE_MARCH && ex.err && stage <= 4 && mhd_tma_fits(g, true))
         return launch_mhd_tma64(phys, stage, stretch, g, co, ia, corr2, dt, visc, a, ex.err, st);

@@ -11,8 +11,8 @@
 // ring, and the pointwise epilogue operands into a second ring; the consumer
 // warps keep the six components' i stencil in a register queue and read the j
 // and k stencils from the slot.  Periodic wrap: k halo boxes start at the
-// wrapped column (the tile width divides N2), a boundary tile's j rows arrive
-// as two boxes.  Every mbarrier wait is bounded (nova_tma.cuh).
+// wrapped column, a boundary tile's j rows arrive as two boxes; the last tiles
+// may be ragged (tma_mesh_fits).  Every mbarrier wait is bounded (nova_tma.cuh).
 //
 // FP64: TJ = 8 (a slot of the two fields is 24 KB, 209 KB with the epilogue
 // ring; one block per SM, 8 consumer warps of 232 registers); FP32:
@@ -72,6 +72,7 @@ template <typename T, int NE> constexpr size_t mhd_smem_bytes()
 struct MhdMaps {
     CUtensorMap tcbA[2], tcb3[2], tcbB[2];  // halo'd rows of each field: TJ+6, 3 or TJ+3 rows
     CUtensorMap tcbC[2];                    // each field's TJ tile rows alone (the queue-only planes)
+    CUtensorMap tcbR[2];                    // the last j tile's rows and the H before them
     CUtensorMap lr[2];                      // k-halo boxes (4 x 8 x 3) of each field
     CUtensorMap e[3];                       // epilogue operands
 };
@@ -92,7 +93,7 @@ __device__ __forceinline__ void mhd_epi_read(const T *se, int c, T &e0, T &e1, T
     }
 }
 
-template <typename T, int PHYS, int STAGE, bool STRETCH, class Args>
+template <typename T, int PHYS, int STAGE, bool STRETCH, class Args, bool WHOLE>
 __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
     k_mhd_tma(Geo g, Coef<T> co, StageCoef<T> sc, const T *__restrict__ ia, const T *__restrict__ corr2, T dt,
               T visc, Args args, const __grid_constant__ MhdMaps maps, int ichunk, int *err)
@@ -118,6 +119,8 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
     const int k0 = blockIdx.x * kTK, j0 = blockIdx.y * TJ;
     const int ib = blockIdx.z * ichunk, ie = min(ib + ichunk, g.N0);
     const int nout = ie - ib;
+    // valid columns and rows of the tile (WHOLE: the mesh has no ragged tile)
+    const int w = WHOLE ? kTK : min(kTK, g.N2 - k0), hrows = WHOLE ? TJ : min(TJ, g.N1 - j0);
 
     if (ty == TJ && lane == 0) {
         for (int r = 0; r < kRing; r++) {
@@ -136,8 +139,9 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
     if (ty >= TJ) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
         if (ty > TJ || lane != 0) return;
-        const bool jlo = j0 < H, jhi = j0 + TJ + H > g.N1;
-        const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + kTK == g.N2) ? 0 : k0 + kTK;
+        const bool jlo = j0 < H, jhi = j0 + TJ >= g.N1;
+        const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + w == g.N2) ? 0 : k0 + kTK;
+        const uint32_t slot_bytes = kSlotBytes - (jhi ? 2 * (TJ - hrows) * kRowBytes : 0);
         auto issue_s = [&](int n) -> bool {  // stencil load n: plane ib - H + n, both fields
             const int r = n % kRing;
             if (n >= kRing && !mbar_wait(empty(r), ((n / kRing) + 1) & 1, err)) return false;
@@ -152,7 +156,7 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
                                 plane);
                 return true;
             }
-            mbar_expect_tx(bar, kSlotBytes);
+            mbar_expect_tx(bar, slot_bytes);
 #pragma unroll
             for (int f = 0; f < 2; f++) {
                 const uint32_t dst = s0 + r * kSlotBytes + f * kFieldBytes;
@@ -160,8 +164,8 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
                     tma_load_4d(dst, &maps.tcb3[f], bar, k0, 0, g.N1 - H, plane);
                     tma_load_4d(dst + H * kRowBytes, &maps.tcbB[f], bar, k0, 0, 0, plane);
                 } else if (jhi) {
-                    tma_load_4d(dst, &maps.tcbB[f], bar, k0, 0, j0 - H, plane);
-                    tma_load_4d(dst + (TJ + H) * kRowBytes, &maps.tcb3[f], bar, k0, 0, 0, plane);
+                    tma_load_4d(dst, &maps.tcbR[f], bar, k0, 0, j0 - H, plane);
+                    tma_load_4d(dst + (hrows + H) * kRowBytes, &maps.tcb3[f], bar, k0, 0, 0, plane);
                 } else {
                     tma_load_4d(dst, &maps.tcbA[f], bar, k0, 0, j0 - H, plane);
                 }
@@ -204,9 +208,10 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
     };
-    const int kw = k0 + tx;
-    const T iak = ia[kw];
-    const T c2k = STRETCH ? corr2[kw] : T(0);
+    const bool on = WHOLE || (tx < w && ty < hrows);
+    const int txc = WHOLE ? tx : min(tx, w - 1);  // lanes past the valid columns read the last one and store nothing
+    const T iak = ia[k0 + txc];
+    const T c2k = STRETCH ? corr2[k0 + txc] : T(0);
 
     if constexpr (sizeof(T) == 8)
         asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
@@ -215,11 +220,11 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
 
     // slot offsets within a field: centre, and the k neighbour at s (inside the
     // row box or in the left/right halo boxes); component stride kTK in both
-    const int cen = (H + ty) * kRowE + tx;
+    const int cen = (H + ty) * kRowE + txc;
     const int lrrow = (ty / kLRB) * 3 * kLRB * 4 + (ty % kLRB) * 4;
     auto zoff = [&](int s) -> int {
-        const int x = tx + s;
-        return x < 0 ? kTcbE + lrrow + 4 + x : (x >= kTK ? kTcbE + kLRE + lrrow + (x - kTK) : cen + s);
+        const int x = txc + s;
+        return x < 0 ? kTcbE + lrrow + 4 + x : (x >= w ? kTcbE + kLRE + lrrow + (x - w) : cen + s);
     };
     // component c (0-2 the stage field, 3-5 the frozen one) within a slot
     auto fc = [](int c) -> int { return (c / 3) * kFieldE + (c % 3) * kTK; };
@@ -246,7 +251,7 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
     }
 
     int es = 0, eph = 0;  // epilogue ring slot and phase of step p
-    long long idx = (long long)ib * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
+    long long idx = (long long)ib * g.N12 + (long long)(j0 + ty) * g.N2 + k0 + tx;
     // step p = 7 m + R: queue head plane p + 2H, centre plane p + H
     auto step = [&](auto Rc, int m, int p) -> bool {
         constexpr int R = decltype(Rc)::value;
@@ -285,6 +290,7 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
         }
 #pragma unroll
         for (int c = 0; c < 3; c++) {
+            if (!on) break;
             const long long o = (long long)c * g.N3 + idx;
             if constexpr (sizeof(T) == 8)
                 rk_store64<STAGE>(args, o, y0[c], e0[c], e1[c], lo[c], dt * rhs[c]);
@@ -353,7 +359,7 @@ template <typename T> bool encode(CUtensorMap *m, const T *base, const Geo &g, u
 
 template <typename T> int mhd_ichunk(const Geo &g)
 {
-    const long long tiles = (long long)(g.N2 / kTK) * (g.N1 / MhdCfg<T>::TJ);
+    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + MhdCfg<T>::TJ - 1) / MhdCfg<T>::TJ);
     return march_chunk(g.N0, tiles, 1, 2.5);
 }
 
@@ -370,19 +376,20 @@ cudaError_t launch_mhd(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     for (int f = 0; f < 2; f++)
         ok = ok && encode(&maps.tcbA[f], fld[f], g, Cf::TJ + 2 * kH) && encode(&maps.tcb3[f], fld[f], g, kH) &&
              encode(&maps.tcbB[f], fld[f], g, Cf::TJ + kH) && encode(&maps.tcbC[f], fld[f], g, Cf::TJ) &&
-             encode(&maps.lr[f], fld[f], g, 0);
+             encode(&maps.lr[f], fld[f], g, 0) && encode(&maps.tcbR[f], fld[f], g, (g.N1 - 1) % Cf::TJ + 1 + kH);
     for (int f = 0; f < NE; f++) ok = ok && encode(&maps.e[f], ef[f], g, Cf::TJ);
     if (!ok) return cudaErrorInvalidValue;
     constexpr size_t smem = mhd_smem_bytes<T, NE>();
-    auto kern = k_mhd_tma<T, PHYS, STAGE, STRETCH, Args>;
-    static bool attr = false;
-    if (!attr) {
+    const bool whole = g.N2 % kTK == 0 && g.N1 % Cf::TJ == 0;
+    auto kern = whole ? k_mhd_tma<T, PHYS, STAGE, STRETCH, Args, true> : k_mhd_tma<T, PHYS, STAGE, STRETCH, Args, false>;
+    static bool attr[2] = {false, false};
+    if (!attr[whole]) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        attr = true;
+        attr[whole] = true;
     }
     const int ch = mhd_ichunk<T>(g);
-    const dim3 grid(g.N2 / kTK, g.N1 / Cf::TJ, (g.N0 + ch - 1) / ch);
+    const dim3 grid((g.N2 + kTK - 1) / kTK, (g.N1 + Cf::TJ - 1) / Cf::TJ, (g.N0 + ch - 1) / ch);
     kern<<<grid, dim3(kTK, Cf::kThreads / kTK), smem, st>>>(g, co, stage_coef(co, visc), ia, corr2, dt, visc, a, maps, ch, err);
     return cudaSuccess;
 }
@@ -416,8 +423,7 @@ cudaError_t launch_mhd_any(int phys, int stage, bool stretch, const Geo &g, cons
 
 bool mhd_tma_fits(const Geo &g, bool fp64)
 {
-    const int tj = fp64 ? MhdCfg<double>::TJ : MhdCfg<float>::TJ;
-    return !g.wallY && g.N2 % kTK == 0 && g.N1 % tj == 0 && g.N1 >= 2 * tj;
+    return !g.wallY && tma_mesh_fits(g, fp64 ? 2 : 4, fp64 ? MhdCfg<double>::TJ : MhdCfg<float>::TJ);
 }
 
 cudaError_t launch_mhd_tma64(int phys, int stage, bool stretch, const Geo &g, const Coef<double> &co, const double *ia,

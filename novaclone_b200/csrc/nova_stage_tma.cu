@@ -11,9 +11,12 @@
 // into a ring of kRing shared-memory slots, each completed by an mbarrier
 // transaction count, and the pointwise epilogue operands of the plane (RK base
 // and accumulator, box 32 x 3 x TJ) into a second ring.  Periodic wrap needs
-// no ghost storage: in k the halo boxes start at the wrapped column (the tile
-// width divides N2), in j a boundary tile's rows arrive as two boxes (3 and
-// TJ + 3 rows) that land back to back in the slot.
+// no ghost storage: in k the halo boxes start at the wrapped column, in j a
+// boundary tile's rows arrive as two boxes (3 rows, and TJ + 3 or, in the last
+// tile, its rows + 3) that land back to back in the slot.  The last tile of
+// either direction may be ragged (tma_mesh_fits): its k neighbours past the
+// last column come from the right halo box, its spare lanes store nothing.
+// 120 x 75 x 100 FP64, stages 0-3: 21, 23, 23, 25 us; the march 24, 27, 27, 32.
 //
 // The consumer warps keep the i stencil in a register queue (the centre of
 // each arriving plane), read the j and k stencils from the slot of the plane
@@ -87,12 +90,14 @@ template <typename T, int NE, bool DIAG = false> constexpr size_t tma_smem_bytes
 {
     using C = TmaCfg<T>;
     constexpr int ering = C::template kERing<NE>;
-    return ((size_t)C::kRing * C::kSlotE + (size_t)ering * NE * C::kEpiE) * sizeof(T) + 8 * (2 * C::kRing + 2 * ering) + (DIAG ? 8 * (kDiagParts + 6 * kTK) * C::kWarps : 0);
+    return ((size_t)C::kRing * C::kSlotE + (size_t)ering * NE * C::kEpiE) * sizeof(T) + 8 * (2 * C::kRing + 2 * ering) + 8 +  // the ghost rows' barrier
+           (DIAG ? 8 * (kDiagParts + 6 * kTK) * C::kWarps : 0);
 }
 
 struct StageMaps {
     CUtensorMap tcbA, tcb3, tcbB;  // halo'd rows of the stencil field: TJ+6, 3 or TJ+3 rows
     CUtensorMap tcbC;              // its TJ tile rows alone (the queue-only planes)
+    CUtensorMap tcbR;              // the last j tile's rows and the H before them
     CUtensorMap lr;                // k-halo boxes (4 x 8 x 3) of the stencil field
     CUtensorMap e[3];              // epilogue operands
 };
@@ -113,13 +118,15 @@ __device__ __forceinline__ void epi_read(const double *se, int c, double &e0, do
 // nodes (nova_diag.cuh: energy, |U|, U_x, the divergence the stage arithmetic
 // forms anyway, and the two curls from the stencil values it holds) into
 // dpart[block * kDiagParts] (the B terms zero).
-// WALLS (FP32, walls on the y nodes j = 0 and j = N1 - 1): one row box per
-// plane from j0 - H (the bulk copy fills rows outside 0..N1-1 with zeros, the
-// last tile may be ragged); in a warp with a row within H of a wall, a valid
-// row's j neighbour across the wall is the wall_ghost of its mirror row (the
-// march's formula); rows past N1 - 1 compute but store nothing.  (FP64 wall
-// stages stay on the march: at 96 registers a thread the ghost branch spills.)
-template <typename T, int STAGE, bool STRETCH, class Args, bool DIAG, bool WALLS = false>
+// WALLS (walls on the y nodes j = 0 and j = N1 - 1): one row box per plane from
+// j0 - H (the bulk copy fills rows outside 0..N1-1 with zeros); the ghost rows
+// are written into the slot before the plane is computed, so the arithmetic is
+// the periodic one.  (Forming the ghosts in the accessors instead duplicated
+// the loop body: FP32 164 us, FP64 258 us with spills, against 120 and
+// 166 us on the 256 x 257 x 128 shear mesh; FP64 on the march 180 us.)
+// WHOLE: the mesh has no ragged tile (FP64: the checks cost 2% at 64^3; DIAG
+// launches take such meshes only)
+template <typename T, int STAGE, bool STRETCH, class Args, bool DIAG, bool WALLS, bool WHOLE>
 __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
     k_stage_tma(Geo g, Coef<T> co, StageCoef<T> sc, const Walls<T> wl, const T *__restrict__ ia,
                 const T *__restrict__ corr2, T dt, T visc, Args args, const __grid_constant__ StageMaps maps,
@@ -127,7 +134,6 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
 {
     static_assert(!DIAG || (sizeof(T) == 8 && (STAGE == 0 || STAGE == 4)), "diagnostics of an FP64 state only");
     static_assert(!(DIAG && WALLS), "diagnostics on periodic meshes");
-    static_assert(!WALLS || sizeof(T) == 4, "FP64 wall stages run the register-queue march");
     using C = TmaCfg<T>;
     constexpr int NE = epi_fields<T, STAGE>();
     constexpr int H = kH, TJ = C::TJ, kRing = C::kRing, kERing = C::template kERing<NE>;
@@ -149,8 +155,12 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
     const int k0 = blockIdx.x * kTK, j0 = blockIdx.y * TJ;
     const int ib = blockIdx.z * ichunk, ie = min(ib + ichunk, g.N0);
     const int nout = ie - ib, nld = nout + 2 * H;
+    // valid columns and rows of the tile
+    const int w = WHOLE ? kTK : min(kTK, g.N2 - k0), hrows = WHOLE ? TJ : min(TJ, g.N1 - j0);
+    const uint32_t gbar = bar0 + 8u * (2 * kRing + 2 * kERing);    // WALLS: the ghost rows' barrier
 
     if (ty == C::kWarps && lane == 0) {  // the producer warp's lane initialises the barriers
+        if (WALLS) mbar_init(gbar, C::kWarps);
         for (int r = 0; r < kRing; r++) {
             mbar_init(full(r), 1);
             mbar_init(empty(r), C::kWarps);
@@ -167,8 +177,9 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
     if (ty >= C::kWarps) {
         if constexpr (sizeof(T) == 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
         if (ty > C::kWarps || lane != 0) return;
-        const bool jlo = j0 < H, jhi = j0 + TJ + H > g.N1;
-        const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + kTK == g.N2) ? 0 : k0 + kTK;
+        const bool jlo = j0 < H, jhi = j0 + TJ >= g.N1;
+        const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + w == g.N2) ? 0 : k0 + kTK;
+        const uint32_t slot_bytes = kSlotBytes - (!WALLS && jhi ? (TJ - hrows) * kRowBytes : 0);
         auto issue_s = [&](int n) -> bool {  // stencil load n: plane ib - H + n
             const int r = n % kRing;
             if (n >= kRing && !mbar_wait(empty(r), ((n / kRing) + 1) & 1, err)) return false;
@@ -180,15 +191,15 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
                 tma_load_4d(dst + H * kRowBytes, &maps.tcbC, bar, k0, 0, j0, plane);
                 return true;
             }
-            mbar_expect_tx(bar, kSlotBytes);
+            mbar_expect_tx(bar, slot_bytes);
             if (WALLS) {
                 tma_load_4d(dst, &maps.tcbA, bar, k0, 0, j0 - H, plane);
             } else if (jlo) {
                 tma_load_4d(dst, &maps.tcb3, bar, k0, 0, g.N1 - H, plane);
                 tma_load_4d(dst + H * kRowBytes, &maps.tcbB, bar, k0, 0, 0, plane);
             } else if (jhi) {
-                tma_load_4d(dst, &maps.tcbB, bar, k0, 0, j0 - H, plane);
-                tma_load_4d(dst + (TJ + H) * kRowBytes, &maps.tcb3, bar, k0, 0, 0, plane);
+                tma_load_4d(dst, &maps.tcbR, bar, k0, 0, j0 - H, plane);
+                tma_load_4d(dst + (hrows + H) * kRowBytes, &maps.tcb3, bar, k0, 0, 0, plane);
             } else {
                 tma_load_4d(dst, &maps.tcbA, bar, k0, 0, j0 - H, plane);
             }
@@ -231,12 +242,39 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
     };
-    // slot offset of the element at tile row r, tile column x (-4 <= x < kTK + 4):
+    // slot offset of the element at tile row r, tile column x (-4 <= x < w + 4):
     // the row box, or the left/right halo boxes ([box][c][8 rows][4]);
     // component stride kTK in both
     auto soff = [&](int r, int x) -> int {
         const int lrrow = (r / kLRB) * 3 * kLRB * 4 + (r % kLRB) * 4;
-        return x < 0 ? kTcbE + lrrow + 4 + x : (x >= kTK ? kTcbE + kLRE + lrrow + (x - kTK) : (H + r) * kRowE + x);
+        return x < 0 ? kTcbE + lrrow + 4 + x
+                     : (x >= w ? kTcbE + kLRE + lrrow + (x - w) : (H + r) * kRowE + x);
+    };
+    // Walls: the box's rows beyond a wall arrive zero filled; before a plane is
+    // computed, warps 0-2 write its ghost rows there (warp l - 1 the l-th row of
+    // either wall, wall_ghost of the mirror row), H steps ahead, and every step
+    // passes a barrier of the consumer warps (an mbarrier: bounded).  Only the
+    // tiles that reach a wall do either.
+    const bool glo = WALLS && j0 == 0, ghi = WALLS && j0 + TJ + H > g.N1;
+    auto ghost_rows = [&](int slot) {
+        if (!WALLS || ty >= H || !(glo || ghi)) return;
+        T *sl = reinterpret_cast<T *>(smraw) + slot * kSlotE;
+        const int l = ty + 1;
+        auto put = [&](int side, int to, int from) {
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                sl[to * kRowE + c * kTK + lane] = wall_ghost(wl, side, c, l, sl[from * kRowE + c * kTK + lane]);
+        };
+        if (glo) put(0, H - l, H + l);
+        const int rg = g.N1 - 1 + l - j0;  // tile row of the north ghost
+        if (ghi && rg < TJ + H) put(1, H + rg, H + rg - 2 * l);
+        // the slot is refilled by bulk copies (async proxy) later
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    };
+    auto ghost_sync = [&](int p) -> bool {
+        if (!WALLS || !(glo || ghi)) return true;
+        release(gbar);
+        return __all_sync(0xffffffffu, mbar_wait(gbar, p & 1, err));
     };
 
     // i-stencil queue of the centre values of planes cur-3 .. cur+3.
@@ -250,17 +288,18 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
     // queue shifted by moves, 231, 247, 247, 315 us unrolled (byte floors 123,
     // 184, 184, 307); with the diagnostics in stage 0: 525 -> 439 us.
     // DIAG: the running diagnostics in shared memory (the registers hold the queue)
-    double *dred = reinterpret_cast<double *>(smraw + (bar0 - s0) + 8 * (2 * kRing + 2 * kERing));
+    double *dred = reinterpret_cast<double *>(smraw + (bar0 - s0) + 8 * (2 * kRing + 2 * kERing + 1));
     DiagAccSm dacc{dred + kDiagParts * C::kWarps + ty * kTK + tx, C::kWarps * kTK};
     if constexpr (DIAG) dacc.init();
     if constexpr (sizeof(T) == 8) {
         // 16 x 32 x 112 + 4 x 32 x 24 = 60416 registers of the 20 x 32 x 96 = 61440 at launch
         asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-        const int kw = k0 + tx;
-        const T iak = ia[kw];
-        const T c2k = STRETCH ? corr2[kw] : T(0);
-        const int cen = (H + ty) * kRowE + tx;
-        auto zoff = [&](int s) -> int { return soff(ty, tx + s); };
+        const bool on = WHOLE || (tx < w && ty < hrows);
+        const int txc = WHOLE ? tx : min(tx, w - 1);  // lanes past the valid columns read the last one and store nothing
+        const T iak = ia[k0 + txc];
+        const T c2k = STRETCH ? corr2[k0 + txc] : T(0);
+        const int cen = (H + ty) * kRowE + txc;
+        auto zoff = [&](int s) -> int { return soff(ty, txc + s); };
         T q[2 * H + 1][3];
         bool ok = true;
         for (int n = 0; n < 2 * H; n++) {  // queue: planes ib-3 .. ib+2
@@ -272,10 +311,13 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
             const T *sl = ring + (n % kRing) * kSlotE;
 #pragma unroll
             for (int c = 0; c < 3; c++) q[n][c] = sl[cen + c * kTK];
-            if (n < H || n >= H + nout) release(empty(n % kRing));  // queue-only plane
+            if (n < H || n >= H + nout)
+                release(empty(n % kRing));  // queue-only plane
+            else
+                ghost_rows(n % kRing);
         }
         int es = 0, eph = 0;  // epilogue ring slot and phase of step p
-        long long idx = (long long)ib * g.N12 + (long long)(j0 + ty) * g.N2 + kw;
+        long long idx = (long long)ib * g.N12 + (long long)(j0 + ty) * g.N2 + k0 + tx;
         // step p = 7 m + R: queue head plane p + 2H, centre plane p + H
         auto step = [&](auto Rc, int m, int p) -> bool {
             constexpr int R = decltype(Rc)::value;
@@ -287,8 +329,12 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
                 const T *sh = ring + sHd * kSlotE;
 #pragma unroll
                 for (int c = 0; c < 3; c++) q[kQ][c] = sh[cen + c * kTK];
-                if (hd >= H + nout) release(empty(sHd));
+                if (hd >= H + nout)
+                    release(empty(sHd));
+                else
+                    ghost_rows(sHd);
             }
+            if (!ghost_sync(p)) return false;
             const T *sl = ring + sCur * kSlotE;
             constexpr int kC = (R + H) % (2 * H + 1);
             auto vx = [&](int c, int s) -> T { return q[(R + H + s + 2 * H + 1) % (2 * H + 1)][c]; };
@@ -300,7 +346,7 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
             if constexpr (DIAG) {
                 double q1, hs;
                 curl_terms<H>(vx, vy, vz, 0, co.a[0], co.a[1], co.a[2], iak, q1, hs);
-                dacc.add(u0, divu, q1, hs);
+                if (on) dacc.add(u0, divu, q1, hs);
             }
             release(empty(sCur));  // the slot's values are in registers
 
@@ -316,9 +362,10 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
                     eph ^= 1;
                 }
             }
+            if (on)
 #pragma unroll
-            for (int c = 0; c < 3; c++)
-                rk_store64<STAGE>(args, (long long)c * g.N3 + idx, u0[c], e0[c], e1[c], e2[c], dt * rhs[c]);
+                for (int c = 0; c < 3; c++)
+                    rk_store64<STAGE>(args, (long long)c * g.N3 + idx, u0[c], e0[c], e1[c], e2[c], dt * rhs[c]);
             idx += g.N12;
             return true;
         };
@@ -341,13 +388,10 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
         // arithmetic (ns_rhs2); pairs load as 8-byte shared-memory words.
         static_assert(kRing == 2 * H + 1, "queue rotation and ring slots share one period");
         static_assert(2 * C::kWarps == TJ, "two tile rows per consumer warp");
-        const int r = 2 * ty + (lane >> 4), kk = 2 * (lane & 15);
+        // (lanes past the valid columns work on the last pair and store nothing)
+        const int r = 2 * ty + (lane >> 4), kk = min(2 * (lane & 15), w - 2);
         const int cen = (H + r) * kRowE + kk;
-        const int jrow = j0 + r;
-        // the rows next to a wall take the j neighbours across it from ghosts
-        // (the choice is made per warp: its two rows together)
-        const bool nearw =
-            WALLS && __any_sync(0xffffffffu, jrow < g.N1 && (jrow < H || jrow + H > g.N1 - 1));
+        const bool on = 2 * (lane & 15) < w && r < hrows;
         // the z neighbours' pairs starting at kk - 4, kk - 2, kk + 2, kk + 4
         const int zm4 = soff(r, kk - 4), zm2 = soff(r, kk - 2), zp2 = soff(r, kk + 2), zp4 = soff(r, kk + 4);
         const float2 iak = *reinterpret_cast<const float2 *>(ia + k0 + kk);
@@ -364,7 +408,10 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
             const T *sl = ring + (n % kRing) * kSlotE;
 #pragma unroll
             for (int c = 0; c < 3; c++) q[n][c] = ld2(sl, cen + c * kTK);
-            if (n < H || n >= H + nout) release(empty(n % kRing));  // queue-only plane
+            if (n < H || n >= H + nout)
+                release(empty(n % kRing));  // queue-only plane
+            else
+                ghost_rows(n % kRing);
         }
 
         int es = 0, eph = 0;  // epilogue ring slot and phase of step p
@@ -380,22 +427,16 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
                 const T *sh = ring + sHd * kSlotE;
 #pragma unroll
                 for (int c = 0; c < 3; c++) q[kQ][c] = ld2(sh, cen + c * kTK);
-                if (hd >= H + nout) release(empty(sHd));
+                if (hd >= H + nout)
+                    release(empty(sHd));
+                else
+                    ghost_rows(sHd);
             }
+            if (!ghost_sync(p)) return false;
             const T *sl = ring + sCur * kSlotE;
             constexpr int kC = (R + H) % (2 * H + 1);
             auto vx = [&](int c, int s) -> float2 { return q[(R + H + s + 2 * H + 1) % (2 * H + 1)][c]; };
             auto vy = [&](int c, int s) -> float2 { return ld2(sl, cen + s * kRowE + c * kTK); };
-            auto vyg = [&](int c, int s) -> float2 {
-                const int jj = jrow + s;
-                if (jrow < g.N1 && (jj < 0 || jj > g.N1 - 1)) {
-                    const int side = jj < 0 ? 0 : 1, l = jj < 0 ? -jj : jj - (g.N1 - 1);
-                    const int jm = jj < 0 ? l : g.N1 - 1 - l;  // the mirror row, inside the slot
-                    const float2 f = ld2(sl, cen + (jm - jrow) * kRowE + c * kTK);
-                    return make_float2(wall_ghost(wl, side, c, l, f.x), wall_ghost(wl, side, c, l, f.y));
-                }
-                return ld2(sl, cen + s * kRowE + c * kTK);
-            };
             // odd offsets straddle two loaded pairs (the centre pair is the queue's)
             auto vz = [&](int c, int s) -> float2 {
                 const int o = c * kTK;
@@ -411,10 +452,7 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
             };
             const float2 u0[3] = {q[kC][0], q[kC][1], q[kC][2]};
             float2 rhs[3];
-            if (WALLS && nearw)
-                ns_rhs2<H, STRETCH>(vx, vyg, vz, u0, co, sc, iak, c2k, visc, rhs);
-            else
-                ns_rhs2<H, STRETCH>(vx, vy, vz, u0, co, sc, iak, c2k, visc, rhs);
+            ns_rhs2<H, STRETCH>(vx, vy, vz, u0, co, sc, iak, c2k, visc, rhs);
             release(empty(sCur));  // the slot's values are in registers
 
             const float2 zz = f2(0.0f);
@@ -446,7 +484,7 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
                 }
             }
             const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + r) * g.N2 + k0 + kk;
-            if (!WALLS || jrow < g.N1) {
+            if (on) {
 #pragma unroll
                 for (int c = 0; c < 3; c++)
                     rk_store32x2<STAGE>(args, (long long)c * g.N3 + idx, u0[c], e0[c], e1[c], lo[c],
@@ -537,7 +575,7 @@ template <typename T> bool encode(CUtensorMap *m, const T *base, const Geo &g, u
 template <typename T> int tma_ichunk(const Geo &g)
 {
     using C = TmaCfg<T>;
-    const long long tiles = (long long)(g.N2 / kTK) * ((g.N1 + C::TJ - 1) / C::TJ);
+    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + C::TJ - 1) / C::TJ);
     return march_chunk(g.N0, tiles, C::kBlocksPerSM, 2.5, g.wallY ? 0.45 : 0.15);
 }
 
@@ -551,19 +589,23 @@ cudaError_t launch_tma(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     memset(&maps, 0, sizeof maps);
     using Cf = TmaCfg<T>;
     bool ok = encode(&maps.tcbA, Y, g, Cf::TJ + 2 * kH) && encode(&maps.tcb3, Y, g, kH) &&
-              encode(&maps.tcbB, Y, g, Cf::TJ + kH) && encode(&maps.tcbC, Y, g, Cf::TJ) && encode(&maps.lr, Y, g, 0);
+              encode(&maps.tcbB, Y, g, Cf::TJ + kH) && encode(&maps.tcbC, Y, g, Cf::TJ) && encode(&maps.lr, Y, g, 0) &&
+              encode(&maps.tcbR, Y, g, (g.N1 - 1) % Cf::TJ + 1 + kH);
     for (int f = 0; f < NE; f++) ok = ok && encode(&maps.e[f], ef[f], g, Cf::TJ);
     if (!ok) return cudaErrorInvalidValue;
     constexpr size_t smem = tma_smem_bytes<T, NE, DIAG>();
-    auto kern = k_stage_tma<T, STAGE, STRETCH, Args, DIAG, WALLS>;
-    static bool attr = false;
-    if (!attr) {
+    constexpr bool kW = sizeof(T) == 8 && !WALLS;  // has a whole-tile instantiation
+    const bool whole = kW && g.N2 % kTK == 0 && g.N1 % Cf::TJ == 0;
+    auto kern = whole ? k_stage_tma<T, STAGE, STRETCH, Args, DIAG, WALLS, kW>
+                      : k_stage_tma<T, STAGE, STRETCH, Args, DIAG, WALLS, DIAG>;
+    static bool attr[2] = {false, false};
+    if (!attr[whole]) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        attr = true;
+        attr[whole] = true;
     }
     const int ch = tma_ichunk<T>(g);
-    const dim3 grid(g.N2 / kTK, (g.N1 + Cf::TJ - 1) / Cf::TJ, (g.N0 + ch - 1) / ch);
+    const dim3 grid((g.N2 + kTK - 1) / kTK, (g.N1 + Cf::TJ - 1) / Cf::TJ, (g.N0 + ch - 1) / ch);
     kern<<<grid, dim3(kTK, Cf::kThreads / kTK), smem, st>>>(g, co, stage_coef(co, visc), wl, ia, corr2, dt, visc, a, maps,
                                                      ch, err, dpart);
     return cudaSuccess;
@@ -588,14 +630,9 @@ cudaError_t launch_tma_stage(int stage, bool stretch, const Geo &g, const Coef<T
                              T dt, T visc, const Args &a, const T *const *ef, int *err, cudaStream_t st,
                              const Walls<T> &wl)
 {
-    if constexpr (sizeof(T) == 4) {
-        if (wl.on)
-            return stretch
-                       ? launch_tma_stage_w<T, true, Args, true>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl)
+    if (wl.on)
+        return stretch ? launch_tma_stage_w<T, true, Args, true>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl)
                        : launch_tma_stage_w<T, false, Args, true>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl);
-    } else {
-        if (wl.on) return cudaErrorNotSupported;
-    }
     return stretch ? launch_tma_stage_w<T, true, Args, false>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl)
                    : launch_tma_stage_w<T, false, Args, false>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl);
 }
@@ -609,14 +646,7 @@ bool tma_encode_field(CUtensorMap *m, const double *base, const Geo &g, unsigned
 
 bool stage_tma_fits(const Geo &g, bool fp64)
 {
-    // tile width divides N2 (k halo boxes start at a wrapped column); periodic
-    // y: the tile height (16 rows for FP64, 8 for FP32) divides N1 with at
-    // most one wrap per tile in j; walls in y (FP32 only: the FP64 wall
-    // stages run faster on the march): any N1 of at least two tiles (the
-    // last tile may be ragged)
-    const int tj = fp64 ? TmaCfg<double>::TJ : TmaCfg<float>::TJ;
-    if (g.wallY && fp64) return false;
-    return g.N2 % kTK == 0 && g.N1 >= 2 * tj && (g.wallY || g.N1 % tj == 0);
+    return tma_mesh_fits(g, fp64 ? 2 : 4, fp64 ? TmaCfg<double>::TJ : TmaCfg<float>::TJ);
 }
 
 cudaError_t launch_stage_tma64(int stage, bool stretch, const Geo &g, const Walls<double> &wl, const Coef<double> &co,
@@ -629,10 +659,11 @@ cudaError_t launch_stage_tma64(int stage, bool stretch, const Geo &g, const Wall
         ef[1] = a.Y1;
         ef[2] = a.Y2;
     }
-    if (dg && !stretch && !wl.on && (stage == 0 || stage == 4)) {
-        using Cf = TmaCfg<double>;
+    using Cf = TmaCfg<double>;
+    if (dg && !stretch && !wl.on && (stage == 0 || stage == 4) && g.N2 % kTK == 0 && g.N1 % Cf::TJ == 0) {
         const int ch = tma_ichunk<double>(g);
-        const long long nb = (long long)(g.N2 / kTK) * (g.N1 / Cf::TJ) * ((g.N0 + ch - 1) / ch);
+        const long long nb =
+            (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + Cf::TJ - 1) / Cf::TJ) * ((g.N0 + ch - 1) / ch);
         if (nb <= dg->cap) {
             const cudaError_t e =
                 stage == 0 ? launch_tma<double, 0, false, StageArgs64, true>(g, co, ia, corr2, dt, visc, a, a.Y, ef,
