@@ -121,14 +121,22 @@ struct nova_ctx {
     double *d_ia64 = nullptr, *d_corr64 = nullptr;
     float *d_ia32 = nullptr, *d_corr32 = nullptr;
     double *d_kx2 = nullptr, *d_ky2 = nullptr, *d_kz2 = nullptr;
-    cufftHandle plan_f = 0, plan_b = 0;
-    bool plans = false;
-    // N0 a length of nova_spec.cuh: the i direction runs fused with the scale
-    // (k_pois_i) between transforms of the (j, k) planes: by the library's own
-    // line kernels where N1 and N2/2 are such lengths too (own_jk), else by
-    // plan_f/plan_b, batched 2-D cuFFT plans.  NOVA_FFT=cufft keeps the plans.
-    bool pois_i = false;
-    bool own_jk = false;
+    // The spectral solve of FP64 runs ([0]) and of FP32-split runs ([1]).
+    // FP64: with N0 a length of nova_spec.cuh the i direction runs fused with
+    // the scale (k_pois_i) between transforms of the (j, k) planes, by the
+    // library's own line kernels where N1 and N2/2 are such lengths too
+    // (own_jk), else by batched 2-D cuFFT plans; other N0: 3-D cuFFT plans and
+    // k_scale.  Split: the plans only (batched 2-D around k_pois_i for N0 = 64
+    // and 256 on periodic meshes, else 3-D), so that a split run's results do
+    // not depend on which transform the FP64 side uses: U is rounded to the
+    // (hi, lo) pair after the correction, and a solve that rounds differently
+    // in the last place flips hi by an FP32 ulp at some nodes, which the FP32
+    // right-hand side amplifies (p moved by up to 1.2e-7 of its rms after 8
+    // steps on 160 x 90 x 140).  NOVA_FFT=cufft: the plans for FP64 as well.
+    struct Fft {
+        cufftHandle f = 0, b = 0;
+        bool plans = false, pois_i = false, own_jk = false, ready = false;
+    } fft[2];
     bool fft_plans = false;
     double *d_twN = nullptr;               // W_N0^m, m = 0..N0-1 (re, im)
     double *d_twR = nullptr, *d_twC = nullptr;  // W_N2^m and W_N1^m
@@ -137,7 +145,6 @@ struct nova_ctx {
     bool fft2 = false;
     bool fft_cluster = false;
     bool pois_direct = false;  // NOVA_POIS_I=direct: k_pois_i also where k_pois_tma fits
-    bool fft_ready = false;
     double *d_tw256 = nullptr;
     cufftHandle dct_f = 0, dct_b = 0;  // wall Poisson on the even extension in y
     bool dct_plans = false;
@@ -406,38 +413,39 @@ nova_status twiddle_table(nova_ctx *ctx, double **d, int N)
     return NOVA_OK;
 }
 
-nova_status ensure_fft(nova_ctx *ctx)
+nova_status ensure_fft(nova_ctx *ctx, bool split)
 {
-    if (ctx->fft_ready) return NOVA_OK;
+    nova_ctx::Fft &F = ctx->fft[split];
+    if (F.ready) return NOVA_OK;
     const Geo &g = ctx->g;
     nova_status s;
-    if (pois_i_fits(g) && ctx->fft_cluster && fft2_fits(g)) {
+    if (!g.wallY && pois_i_fits(g) && ctx->fft_cluster && fft2_fits(g)) {
         // the (j, k) planes by the cluster kernels, the i direction by k_pois_i
         std::vector<double> tw = twiddles(g.N0), t256 = twiddles(256);
         if ((s = dalloc(ctx, &ctx->d_twN, tw.size())) != NOVA_OK) return s;
         CK(cudaMemcpy(ctx->d_twN, tw.data(), sizeof(double) * tw.size(), cudaMemcpyHostToDevice));
         if ((s = dalloc(ctx, &ctx->d_tw256, t256.size())) != NOVA_OK) return s;
         CK(cudaMemcpy(ctx->d_tw256, t256.data(), sizeof(double) * t256.size(), cudaMemcpyHostToDevice));
-        ctx->pois_i = true;
+        F.pois_i = true;
         ctx->fft2 = true;
         const size_t nspec = (size_t)g.N0 * g.N1 * (g.N2 / 2 + 1);
         if ((s = dalloc(ctx, (double **)&ctx->d_spec, 2 * nspec)) != NOVA_OK) return s;
         if ((s = dalloc(ctx, &ctx->d_rhs, (size_t)g.N3)) != NOVA_OK) return s;
-        ctx->fft_ready = true;
+        F.ready = true;
         return NOVA_OK;
     }
     // the transform runs over the N[1] unique y nodes of poisson::rhs (poisson.cpp:167-181),
     // which with walls are the first N[1] of the N[1]+1 stored rows
     const int ny = ctx->md.N[1];
-    const bool pi = pois_i_fits(g);
+    const bool pi = split ? !g.wallY && (g.N0 == 64 || g.N0 == 256) : pois_i_fits(g);
     if (pi && (s = twiddle_table(ctx, &ctx->d_twN, g.N0)) != NOVA_OK) return s;
     const size_t nspec = (size_t)g.N0 * ny * (g.N2 / 2 + 1);
-    if (pi && !ctx->fft_plans && spec_cols_fit(ny) && spec_rows_fit(g.N2)) {
+    if (pi && !split && !ctx->fft_plans && spec_cols_fit(ny) && spec_rows_fit(g.N2)) {
         if ((s = twiddle_table(ctx, &ctx->d_twR, g.N2)) != NOVA_OK) return s;
         if ((s = twiddle_table(ctx, &ctx->d_twC, ny)) != NOVA_OK) return s;
         if ((s = dalloc(ctx, (double **)&ctx->d_spec, 2 * nspec)) != NOVA_OK) return s;
         if ((s = dalloc(ctx, &ctx->d_rhs, (size_t)g.N3)) != NOVA_OK) return s;
-        ctx->pois_i = ctx->own_jk = ctx->fft_ready = true;
+        F.pois_i = F.own_jk = F.ready = true;
         return NOVA_OK;
     }
     // 3-D transform, or for k_pois_i the (j, k) planes batched over i; both
@@ -448,19 +456,19 @@ nova_status ensure_fft(nova_ctx *ctx)
     int cembed3[3] = {g.N0, ny, g.N2 / 2 + 1}, cembed2[2] = {ny, g.N2 / 2 + 1};
     int *n = pi ? n2d : n3d, *rembed = pi ? rembed2 : rembed3, *cembed = pi ? cembed2 : cembed3;
     const int rdist = (pi ? 1 : g.N0) * g.N1 * g.N2, cdist = (pi ? 1 : g.N0) * ny * (g.N2 / 2 + 1);
-    if ((s = fft_check(ctx, cufftPlanMany(&ctx->plan_f, rank, n, rembed, 1, rdist, cembed, 1, cdist, CUFFT_D2Z, batch),
+    if ((s = fft_check(ctx, cufftPlanMany(&F.f, rank, n, rembed, 1, rdist, cembed, 1, cdist, CUFFT_D2Z, batch),
                        "cufftPlanMany D2Z")) != NOVA_OK)
         return s;
-    if ((s = fft_check(ctx, cufftPlanMany(&ctx->plan_b, rank, n, cembed, 1, cdist, rembed, 1, rdist, CUFFT_Z2D, batch),
+    if ((s = fft_check(ctx, cufftPlanMany(&F.b, rank, n, cembed, 1, cdist, rembed, 1, rdist, CUFFT_Z2D, batch),
                        "cufftPlanMany Z2D")) != NOVA_OK) {
-        cufftDestroy(ctx->plan_f);
+        cufftDestroy(F.f);
         return s;
     }
-    ctx->plans = true;
-    ctx->pois_i = pi;
+    F.plans = true;
+    F.pois_i = pi;
     if ((s = dalloc(ctx, (double **)&ctx->d_spec, 2 * nspec)) != NOVA_OK) return s;
     if ((s = dalloc(ctx, &ctx->d_rhs, (size_t)g.N3)) != NOVA_OK) return s;
-    ctx->fft_ready = true;
+    F.ready = true;
     return NOVA_OK;
 }
 
@@ -484,10 +492,11 @@ nova_status stage_fail(nova_ctx *ctx, cudaError_t e)
 }
 
 // rhs (device, N3 doubles) -> p: spectral inverse of div(grad(.)) (poisson::solve)
-nova_status poisson_device(nova_ctx *ctx, const double *rhs, double *p)
+nova_status poisson_device(nova_ctx *ctx, const double *rhs, double *p, bool split)
 {
     nova_status s;
-    if ((s = ensure_fft(ctx)) != NOVA_OK) return s;
+    if ((s = ensure_fft(ctx, split)) != NOVA_OK) return s;
+    const nova_ctx::Fft &F = ctx->fft[split];
     if ((s = ensure_red(ctx)) != NOVA_OK) return s;  // the error word of k_pois_tma
     ProfScope ps(ctx, NOVA_K_FFT);
     const long long nuniq = (long long)ctx->g.N0 * ctx->md.N[1] * ctx->g.N2;
@@ -500,7 +509,7 @@ nova_status poisson_device(nova_ctx *ctx, const double *rhs, double *p)
         CKL("cluster FFT / k_pois_i");
         return NOVA_OK;
     }
-    if (ctx->own_jk) {
+    if (F.own_jk) {
         const int ny = ctx->md.N[1], nzh = ctx->g.N2 / 2 + 1;
         launch_rows_fwd(ctx->g.N0, ny, ctx->g.N12, ctx->g.N2, rhs, ctx->d_spec, ctx->d_twR, ctx->stream);
         launch_cols_j(ctx->g.N0, ny, nzh, false, ctx->d_spec, ctx->d_twC, ctx->stream);
@@ -512,12 +521,12 @@ nova_status poisson_device(nova_ctx *ctx, const double *rhs, double *p)
         CKL("line transforms / k_pois_i");
         return NOVA_OK;
     }
-    cufftSetStream(ctx->plan_f, ctx->stream);
-    cufftSetStream(ctx->plan_b, ctx->stream);
-    if ((s = fft_check(ctx, cufftExecD2Z(ctx->plan_f, (cufftDoubleReal *)rhs, (cufftDoubleComplex *)ctx->d_spec),
+    cufftSetStream(F.f, ctx->stream);
+    cufftSetStream(F.b, ctx->stream);
+    if ((s = fft_check(ctx, cufftExecD2Z(F.f, (cufftDoubleReal *)rhs, (cufftDoubleComplex *)ctx->d_spec),
                        "cufftExecD2Z")) != NOVA_OK)
         return s;
-    if (ctx->pois_i) {
+    if (F.pois_i) {
         launch_pois_i(ctx->g, ctx->md.N[1], ctx->d_spec, ctx->d_twN, ctx->d_kx2, ctx->d_ky2, ctx->d_kz2,
                       1.0 / (double)nuniq, ctx->pois_direct ? nullptr : ctx->d_flag + 1, ctx->stream);
         ctx->launches += 1;
@@ -528,7 +537,7 @@ nova_status poisson_device(nova_ctx *ctx, const double *rhs, double *p)
         ctx->launches += 1;
         CKL("k_scale");
     }
-    if ((s = fft_check(ctx, cufftExecZ2D(ctx->plan_b, (cufftDoubleComplex *)ctx->d_spec, (cufftDoubleReal *)p),
+    if ((s = fft_check(ctx, cufftExecZ2D(F.b, (cufftDoubleComplex *)ctx->d_spec, (cufftDoubleReal *)p),
                        "cufftExecZ2D")) != NOVA_OK)
         return s;
     return NOVA_OK;
@@ -545,12 +554,12 @@ std::vector<double> ky2_walls(const nova_ctx *ctx)
 
 // the wall Poisson with DCT-I along y on the N[1] + 1 stored rows (N[1] = 256):
 // batched 2-D D2Z over (i, k), k_pois_dct (DCT-I, scale, DCT-I), 2-D Z2D
-nova_status poisson_device_dct1(nova_ctx *ctx, const double *rhs, double *p)
+nova_status poisson_device_dct1(nova_ctx *ctx, const double *rhs, double *p, bool split)
 {
     const Geo &g = ctx->g;
     const int ny = ctx->md.N[1], nzh = g.N2 / 2 + 1;
     nova_status s;
-    const bool own = !ctx->fft_plans && spec_rows_fit(g.N2) && spec_cols_fit(g.N0);
+    const bool own = !split && !ctx->fft_plans && spec_rows_fit(g.N2) && spec_cols_fit(g.N0);
     if (own && !ctx->dct2_own) {
         if ((s = twiddle_table(ctx, &ctx->d_twR, g.N2)) != NOVA_OK) return s;
         if ((s = twiddle_table(ctx, &ctx->d_twN, g.N0)) != NOVA_OK) return s;
@@ -612,12 +621,12 @@ nova_status poisson_device_dct1(nova_ctx *ctx, const double *rhs, double *p)
 // the wall Poisson of NOVA_POISSON_DCT: even extension in y, periodic solve on
 // the doubled domain (modified wavenumbers of period 2 L_y), restriction to
 // the stored rows
-nova_status poisson_device_dct(nova_ctx *ctx, const double *rhs, double *p)
+nova_status poisson_device_dct(nova_ctx *ctx, const double *rhs, double *p, bool split)
 {
     const Geo &g = ctx->g;
     const int ny = ctx->md.N[1];
     nova_status s;
-    if (!ctx->dct_extend && pois_dct_fits(g, ny)) return poisson_device_dct1(ctx, rhs, p);
+    if (!ctx->dct_extend && pois_dct_fits(g, ny)) return poisson_device_dct1(ctx, rhs, p, split);
     if (!ctx->dct_plans) {
         if ((s = fft_check(ctx, cufftPlan3d(&ctx->dct_f, g.N0, 2 * ny, g.N2, CUFFT_D2Z), "cufftPlan3d D2Z (walls)")) !=
             NOVA_OK)
@@ -776,10 +785,11 @@ extern "C" nova_status nova_destroy(nova_ctx *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     prof_collect(ctx);
     for (auto e : ctx->ev_pool) cudaEventDestroy(e);
-    if (ctx->plans) {
-        cufftDestroy(ctx->plan_f);
-        cufftDestroy(ctx->plan_b);
-    }
+    for (const nova_ctx::Fft &F : ctx->fft)
+        if (F.plans) {
+            cufftDestroy(F.f);
+            cufftDestroy(F.b);
+        }
     if (ctx->dct_plans) {
         cufftDestroy(ctx->dct_f);
         cufftDestroy(ctx->dct_b);
@@ -1114,12 +1124,12 @@ extern "C" nova_status nova_poisson_solve(nova_ctx *ctx, const nova_field *rhs, 
     if (!on_mesh(ctx, rhs) || !on_mesh(ctx, p)) return fail(ctx, NOVA_E_INVALID, "nova_poisson_solve: field of another mesh");
     if (rhs->nc != 1 || p->nc != 1 || rhs->prec != NOVA_F64 || p->prec != NOVA_F64)
         return fail(ctx, NOVA_E_INVALID, "nova_poisson_solve: needs FP64 scalar fields");
-    nova_status s = ensure_fft(ctx);
+    nova_status s = ensure_fft(ctx, false);
     if (s == NOVA_OK) s = ensure_red(ctx);
     if (s != NOVA_OK) return s;
     CK(cudaMemsetAsync(ctx->d_flag + 1, 0, sizeof(int), ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_rhs, rhs->d64, sizeof(double) * ctx->g.N3, cudaMemcpyDeviceToDevice, ctx->stream));
-    if ((s = poisson_device(ctx, ctx->d_rhs, p->d64)) != NOVA_OK) return s;
+    if ((s = poisson_device(ctx, ctx->d_rhs, p->d64, false)) != NOVA_OK) return s;
     int perr = 0;
     CK(cudaMemcpyAsync(&perr, ctx->d_flag + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1197,7 +1207,7 @@ nova_status ensure_work(nova_ctx *ctx, int prec)
     }
     // the FP32-split path's U* (FP64, the projection's input)
     if (s == NOVA_OK && prec != NOVA_F64) s = dalloc(ctx, &ctx->w64[0], n);
-    if (s == NOVA_OK) s = ensure_fft(ctx);
+    if (s == NOVA_OK) s = ensure_fft(ctx, prec != NOVA_F64);
     if (s == NOVA_OK) s = ensure_red(ctx);
     return s;
 }
@@ -1291,7 +1301,8 @@ nova_status evolve(nova_ctx *ctx, const nova_run_desc *rd, int phys, nova_field 
             }
             CKL("divergence kernel");
             nova_status s =
-                dct ? poisson_device_dct(ctx, ctx->d_rhs, p->d64) : poisson_device(ctx, ctx->d_rhs, p->d64);
+                dct ? poisson_device_dct(ctx, ctx->d_rhs, p->d64, Y->prec != NOVA_F64)
+                            : poisson_device(ctx, ctx->d_rhs, p->d64, Y->prec != NOVA_F64);
             if (s != NOVA_OK) return s;
             if (walls && !dct) {
                 launch_wall_fix64(g, pfix, p->d64, st);
@@ -1363,7 +1374,8 @@ nova_status evolve(nova_ctx *ctx, const nova_run_desc *rd, int phys, nova_field 
             ctx->launches += 1;
         }
         CKL("k_div_tiled");
-        nova_status s = dct ? poisson_device_dct(ctx, ctx->d_rhs, p->d64) : poisson_device(ctx, ctx->d_rhs, p->d64);
+        nova_status s = dct ? poisson_device_dct(ctx, ctx->d_rhs, p->d64, Y->prec != NOVA_F64)
+                            : poisson_device(ctx, ctx->d_rhs, p->d64, Y->prec != NOVA_F64);
         if (s != NOVA_OK) return s;
         if (walls && !dct) {
             launch_wall_fix64(g, pfix, p->d64, st);
@@ -1442,7 +1454,8 @@ nova_status evolve(nova_ctx *ctx, const nova_run_desc *rd, int phys, nova_field 
             ctx->launches += 1;
         }
         CKL("k_div_tiled");
-        nova_status s = dct ? poisson_device_dct(ctx, ctx->d_rhs, p->d64) : poisson_device(ctx, ctx->d_rhs, p->d64);
+        nova_status s = dct ? poisson_device_dct(ctx, ctx->d_rhs, p->d64, Y->prec != NOVA_F64)
+                            : poisson_device(ctx, ctx->d_rhs, p->d64, Y->prec != NOVA_F64);
         if (s != NOVA_OK) return s;
         if (walls && !dct) {
             launch_wall_fix64(g, pfix, p->d64, st);
@@ -1590,7 +1603,7 @@ nova_status rk_loop64(nova_ctx *ctx, const nova_run_desc *rd, int phys, double v
     if (e != cudaSuccess) return stage_fail(ctx, e);
     ctx->launches += 1;
     CKL("k_div_tiled");
-    nova_status s = poisson_device(ctx, ctx->d_rhs, ctx->w64[1]);
+    nova_status s = poisson_device(ctx, ctx->d_rhs, ctx->w64[1], false);
     if (s != NOVA_OK) return s;
     e = launch_correct(ctx->h, g, Walls<double>{}, ctx->co64, ctx->d_ia64, ctx->w64[1], div, out, out, nullptr,
                        nullptr, nullptr, nullptr, st, StageExec{ctx->stage_impl, ctx->d_flag + 1});
@@ -1640,7 +1653,7 @@ nova_status rk_loop32(nova_ctx *ctx, const nova_run_desc *rd, int phys, double v
     if (e != cudaSuccess) return stage_fail(ctx, e);
     ctx->launches += 1;
     CKL("k_div_tiled");
-    nova_status s = poisson_device(ctx, ctx->d_rhs, pbuf);
+    nova_status s = poisson_device(ctx, ctx->d_rhs, pbuf, true);
     if (s != NOVA_OK) return s;
     e = launch_correct(ctx->h, g, Walls<double>{}, ctx->co64, ctx->d_ia64, pbuf, div, Us64, nullptr, nullptr, nullptr,
                        ohi, olo, st, StageExec{ctx->stage_impl, ctx->d_flag + 1});
@@ -1660,7 +1673,8 @@ nova_status fwd_step64(nova_ctx *ctx, const nova_run_desc *rd, const double *Uin
 }
 
 // out = P in = in - G L^-1 D in (the projection is symmetric: its own adjoint)
-nova_status project64(nova_ctx *ctx, const double *in, double *out, double *pbuf)
+// (split: in an FP32-split adjoint)
+nova_status project64(nova_ctx *ctx, const double *in, double *out, double *pbuf, bool split)
 {
     const Geo &g = ctx->g;
     cudaError_t e = launch_div_proj(ctx->h, g, Walls<double>{}, ctx->co64, ctx->d_ia64, in, nullptr, nullptr, 1.0,
@@ -1668,7 +1682,7 @@ nova_status project64(nova_ctx *ctx, const double *in, double *out, double *pbuf
     if (e != cudaSuccess) return stage_fail(ctx, e);
     ctx->launches += 1;
     CKL("k_div_tiled");
-    nova_status s = poisson_device(ctx, ctx->d_rhs, pbuf);
+    nova_status s = poisson_device(ctx, ctx->d_rhs, pbuf, split);
     if (s != NOVA_OK) return s;
     e = launch_correct(ctx->h, g, Walls<double>{}, ctx->co64, ctx->d_ia64, pbuf, 1.0, in, out, nullptr, nullptr,
                        nullptr, nullptr, ctx->stream, StageExec{ctx->stage_impl, ctx->d_flag + 1});
@@ -1817,7 +1831,7 @@ extern "C" nova_status nova_adjoint_grad(nova_ctx *ctx, const nova_adj_desc *ad,
         for (int t = m - 1; t >= 0; t--) {
             {
                 ProfScope ps(ctx, NOVA_K_DIV);
-                if ((s = project64(ctx, lam, mu, gB)) != NOVA_OK) return s;
+                if ((s = project64(ctx, lam, mu, gB, false)) != NOVA_OK) return s;
             }
             const double dt = rd->dt, nu = rd->nu;
             auto adj = [&](int stage, const AdjArgs &a) {
@@ -1975,7 +1989,7 @@ nova_status adjoint_mhd(nova_ctx *ctx, const nova_adj_desc *ad, const nova_state
     };
     auto proj = [&](const double *in) {
         ProfScope ps(ctx, NOVA_K_DIV);
-        return project64(ctx, in, mu, gB);
+        return project64(ctx, in, mu, gB, false);
     };
     enum { UB = 0, BU = 1, BB = 2 };
     for (int c = nck - 1; c >= 0; c--) {
@@ -2144,7 +2158,7 @@ nova_status adjoint_split(nova_ctx *ctx, const nova_adj_desc *ad, const nova_sta
         for (int t = m - 1; t >= 0; t--) {
             {
                 ProfScope ps(ctx, NOVA_K_DIV);
-                if ((s = project64(ctx, lam, mu, pbuf)) != NOVA_OK) return s;
+                if ((s = project64(ctx, lam, mu, pbuf, true)) != NOVA_OK) return s;
             }
             adj(4, AdjArgs32{Ys(t, 4), nullptr, mu, nullptr, gA, Lam, nullptr});
             adj(3, AdjArgs32{Ys(t, 3), gA, mu, Lam, gB, Lam, nullptr});
@@ -2302,7 +2316,7 @@ nova_status adjoint_mhd_split(nova_ctx *ctx, const nova_adj_desc *ad, const nova
     };
     auto proj = [&](const double *in) {
         ProfScope ps(ctx, NOVA_K_DIV);
-        return project64(ctx, in, mu, pbuf);
+        return project64(ctx, in, mu, pbuf, true);
     };
     enum { UB = 0, BU = 1, BB = 2 };
     for (int c = nck - 1; c >= 0; c--) {
