@@ -100,9 +100,10 @@ __global__ void k_fdm_setref(double *ap, double *b, long long n, double val)
 
 // partial sums of (b - A x)^2 over the (N0+1)(N1+1)(N2+1) nodes the reference
 // loops over: its duplicate periodic node N of each direction is node 0 here,
-// so node 0 of a direction counts twice.  A block takes whole (i, j) rows, two
-// at a time so that both rows' loads are in flight together, its threads
-// along k.
+// so node 0 of a direction counts twice.  A block takes whole (i, j) rows, as
+// many side by side as its threads cover (tpr threads per row: 128^3 took 54 us
+// with one row of 128 nodes per 256 threads, 34 us with two), two such
+// groups at a time so that both groups' loads are in flight together.
 __device__ __forceinline__ double fdm_res_node(const Geo &g, const double *__restrict__ coef,
                                                const double *__restrict__ x, int row, int k)
 {
@@ -122,14 +123,14 @@ __device__ __forceinline__ double fdm_res_node(const Geo &g, const double *__res
 }
 
 __global__ void __launch_bounds__(256, 4) k_fdm_res(Geo g, const double *__restrict__ coef,
-                                                    const double *__restrict__ x, double *part)
+                                                    const double *__restrict__ x, double *part, int tpr)
 {
     __shared__ double sh[32];
-    const int rows = g.N0 * g.N1;
+    const int rows = g.N0 * g.N1, rpb = blockDim.x / tpr, step = gridDim.x * rpb;
     double acc = 0.0;
-    for (int row = blockIdx.x; row < rows; row += 2 * gridDim.x) {
-        const int row2 = row + gridDim.x;
-        for (int k = threadIdx.x; k < g.N2; k += blockDim.x) {
+    for (int row = blockIdx.x * rpb + threadIdx.x / tpr; row < rows; row += 2 * step) {
+        const int row2 = row + step;
+        for (int k = threadIdx.x % tpr; k < g.N2; k += tpr) {
             const double a = fdm_res_node(g, coef, x, row, k);
             const double b = row2 < rows ? fdm_res_node(g, coef, x, row2, k) : 0.0;
             acc = __dadd_rn(acc, __dadd_rn(a, b));
@@ -359,8 +360,12 @@ __global__ void __launch_bounds__(FDM_LINE_THREADS, 4) k_fdm_factor(Geo g, const
 // Every thread loads its tile elements of the next chunk into registers
 // before the block waits for warp 0, so those loads are in flight during the
 // recurrences and the barriers.
-template <int AXIS>
-__global__ void __launch_bounds__(FDM_LINE_THREADS, 3) k_fdm_line(Geo g, const double *__restrict__ coef,
+// MINB: resident blocks per SM.  Three (80 registers) hold every prefetched
+// operand; four (64 registers, a few spilled) pay where they turn two waves into
+// one: 128^3, 512 blocks, 50 -> 42 us; at 256^3 (2048 blocks) 298 -> 312 us, at
+// 75 x 64 x 90 14 -> 18 us.
+template <int AXIS, int MINB>
+__global__ void __launch_bounds__(FDM_LINE_THREADS, MINB) k_fdm_line(Geo g, const double *__restrict__ coef,
                                                                 const double *__restrict__ fac,
                                                                 const double *__restrict__ ls,
                                                                 const double *__restrict__ xin, double *xout)
@@ -576,7 +581,9 @@ void launch_fdm_setref(const Geo &g, double *coef, long long n, double val, cuda
 void launch_fdm_residual(const Geo &g, const double *coef, const double *x, double *part, int nb, double *out,
                          cudaStream_t st)
 {
-    k_fdm_res<<<nb, 256, 0, st>>>(g, coef, x, part);
+    int tpr = 32;
+    while (tpr < 256 && tpr < g.N2) tpr *= 2;
+    k_fdm_res<<<nb, 256, 0, st>>>(g, coef, x, part, tpr);
     const double count = (double)(g.N0 + 1) * (double)(g.N1 + 1) * (double)(g.N2 + 1);
     k_fdm_res_final<<<1, 256, 0, st>>>(part, nb, count, out);
 }
@@ -600,12 +607,14 @@ void launch_fdm_line(int axis, const Geo &g, const double *coef, const double *f
     // one block per FDM_LT consecutive values of the fastest fixed coordinate
     const int fast = axis == 2 ? g.N1 : g.N2, slow = axis == 0 ? g.N1 : g.N0;
     const unsigned nb = (unsigned)slow * (unsigned)((fast + FDM_LT - 1) / FDM_LT);
+    const bool four = nb > 3 * 148 && nb <= 4 * 148;
+    auto go = [&](auto kern) { kern<<<nb, FDM_LINE_THREADS, 0, st>>>(g, coef, fac, ls, xin, xout); };
     if (axis == 0)
-        k_fdm_line<0><<<nb, FDM_LINE_THREADS, 0, st>>>(g, coef, fac, ls, xin, xout);
+        four ? go(k_fdm_line<0, 4>) : go(k_fdm_line<0, 3>);
     else if (axis == 1)
-        k_fdm_line<1><<<nb, FDM_LINE_THREADS, 0, st>>>(g, coef, fac, ls, xin, xout);
+        four ? go(k_fdm_line<1, 4>) : go(k_fdm_line<1, 3>);
     else
-        k_fdm_line<2><<<nb, FDM_LINE_THREADS, 0, st>>>(g, coef, fac, ls, xin, xout);
+        four ? go(k_fdm_line<2, 4>) : go(k_fdm_line<2, 3>);
 }
 
 }  // namespace nova
