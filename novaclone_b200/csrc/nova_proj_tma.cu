@@ -241,6 +241,14 @@ __global__ void __launch_bounds__(kThreads, 2)
             return (double)sl[o];
     };
 
+    // i queue of planes cur-3 .. cur+3: plane ib - H + x lives in q[x % 7], and the
+    // loop is unrolled by 7 (= 2H + 1 = kRing), so the rotation is register renaming
+    // and every ring slot index a compile-time constant of the unrolled step.
+    // Queue moves and slot arithmetic bound the rolled loop: divergence at 256^3 108
+    // -> 94 us (82 of bytes), 128^3 17.8 -> 15.5, shear walls 69 -> 60, 120 x 75 x
+    // 100 12.2 -> 10.9; correction at 120 x 75 x 100 14.3 -> 12.6, at 256^3 150 (147
+    // of bytes) before and after.
+    static_assert(kRing == 2 * H + 1, "queue rotation and ring slots share one period");
     double q[2 * H + 1];
     bool ok = true;
     for (int n = 0; n < 2 * H; n++) {
@@ -249,24 +257,22 @@ __global__ void __launch_bounds__(kThreads, 2)
             ok = false;
             break;
         }
-        q[n + 1] = val(ring + (n % kRing) * C::kSlotE, qoff);
+        q[n] = val(ring + (n % kRing) * C::kSlotE, qoff);
         if (n < H || n >= H + nout) release(empty(n % kRing));
     }
-    for (int p = 0; p < nout && ok; p++) {
-        const int hd = p + 2 * H;
-        ok = mbar_wait(full(hd % kRing), (hd / kRing) & 1, err);
-        if (!__all_sync(0xffffffffu, ok)) {
-            ok = false;
-            break;
-        }
-#pragma unroll
-        for (int s = 0; s < 2 * H; s++) q[s] = q[s + 1];
-        q[2 * H] = val(ring + (hd % kRing) * C::kSlotE, qoff);
-        if (hd >= H + nout) release(empty(hd % kRing));
+    const bool store = WHOLE || (tx < w && ty < hrows);
+    long long idx = (long long)ib * g.N12 + (long long)(j0 + ty) * g.N2 + k0 + tx;
+    int es = 0, eph = 0;  // epilogue ring slot and phase of step p
+    // step p = 7 m + R: queue head plane p + 2H, centre plane p + H
+    auto step = [&](auto Rc, int m, int p) -> bool {
+        constexpr int R = decltype(Rc)::value;
+        constexpr int sHd = (R + 2 * H) % kRing, sCur = (R + H) % kRing;
+        if (!__all_sync(0xffffffffu, mbar_wait(full(sHd), (m + (R + 2 * H) / kRing) & 1, err))) return false;
+        q[sHd] = val(ring + sHd * C::kSlotE, qoff);
+        if (p + 2 * H >= H + nout) release(empty(sHd));
 
-        const int cur = p + H;
-        const TS *sl = ring + (cur % kRing) * C::kSlotE;
-        auto vx = [&](int, int s) -> double { return q[H + s]; };
+        const TS *sl = ring + sCur * C::kSlotE;
+        auto vx = [&](int, int s) -> double { return q[(R + H + s) % kRing]; };
         auto vy = [&](int, int s) -> double { return val(sl, yoff + s * kTK); };
         auto vyg = [&](int, int s) -> double {
             const int jj = jrow + s;
@@ -279,27 +285,25 @@ __global__ void __launch_bounds__(kThreads, 2)
         };
         auto vz = [&](int, int s) -> double { return val(sl, zoff(s)); };
         const double dy = (WALLS && nearw) ? d1<double, H>(vyg, CY, co.a[1]) : d1<double, H>(vy, CY, co.a[1]);
-        const bool store = WHOLE || (tx < w && ty < hrows);
-        const long long idx = (long long)(ib + p) * g.N12 + (long long)(j0 + ty) * g.N2 + k0 + tx;
         if constexpr (MODE == PROJ_DIV) {
             const double d = d1<double, H>(vx, 0, co.a[0]) + dy + d1<double, H>(vz, 2, az);
-            release(empty(cur % kRing));  // the slot's values are in registers
+            release(empty(sCur));  // the slot's values are in registers
             if (store) a.rhs[idx] = d / a.divisor;
         } else {
             const double gr[3] = {d1<double, H>(vx, 0, co.a[0]), dy, d1<double, H>(vz, 0, az)};
-            release(empty(cur % kRing));  // the slot's values are in registers
-            ok = mbar_wait(efull(p % kERing), (p / kERing) & 1, err);
-            if (!__all_sync(0xffffffffu, ok)) {
-                ok = false;
-                break;
-            }
-            const TE *se = ering + (p % kERing) * NE * C::kEpiE + ty * 3 * kTK + tx;
+            release(empty(sCur));  // the slot's values are in registers
+            if (!__all_sync(0xffffffffu, mbar_wait(efull(es), eph, err))) return false;
+            const TE *se = ering + es * NE * C::kEpiE + ty * 3 * kTK + tx;
             double us[3];
 #pragma unroll
             for (int c = 0; c < 3; c++)
                 us[c] = (SPLIT && MODE == PROJ_CORR) ? (double)se[c * kTK] + (double)se[C::kEpiE + c * kTK]
                                                      : (double)se[c * kTK];
-            release(eempty(p % kERing));
+            release(eempty(es));
+            if (++es == kERing) {
+                es = 0;
+                eph ^= 1;
+            }
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 if (!store) break;
@@ -314,6 +318,21 @@ __global__ void __launch_bounds__(kThreads, 2)
                 }
             }
         }
+        idx += g.N12;
+        return true;
+    };
+    using I0 = std::integral_constant<int, 0>;
+    using I1 = std::integral_constant<int, 1>;
+    using I2 = std::integral_constant<int, 2>;
+    using I3 = std::integral_constant<int, 3>;
+    using I4 = std::integral_constant<int, 4>;
+    using I5 = std::integral_constant<int, 5>;
+    using I6 = std::integral_constant<int, 6>;
+    for (int m = 0, p = 0; ok && p < nout; m++, p += kRing) {
+        ok = step(I0{}, m, p) && (p + 1 >= nout || (step(I1{}, m, p + 1) && (p + 2 >= nout ||
+             (step(I2{}, m, p + 2) && (p + 3 >= nout || (step(I3{}, m, p + 3) && (p + 4 >= nout ||
+             (step(I4{}, m, p + 4) && (p + 5 >= nout || (step(I5{}, m, p + 5) && (p + 6 >= nout ||
+             step(I6{}, m, p + 6))))))))))));
     }
 }
 
@@ -384,8 +403,11 @@ cudaError_t launch_w(const Geo &g, const Coef<double> &co, const Walls<double> &
                      const ProjArgs &a, const ProjMaps &pm, int *err, cudaStream_t st)
 {
     using C = ProjCfg<MODE, SPLIT>;
-    const bool whole = !WALLS && g.N2 % kTK == 0 && g.N1 % TJ == 0;
-    auto kern = whole ? k_proj_tma<MODE, SPLIT, WALLS, !WALLS> : k_proj_tma<MODE, SPLIT, WALLS, false>;
+    // the whole-tile form for the corrections alone (split 192 x 192 x 384: 131 us
+    // against 133); in the divergence it spills (256^3: 107 us against 94)
+    constexpr bool kWhole = MODE != PROJ_DIV && !WALLS;
+    const bool whole = kWhole && g.N2 % kTK == 0 && g.N1 % TJ == 0;
+    auto kern = whole ? k_proj_tma<MODE, SPLIT, WALLS, kWhole> : k_proj_tma<MODE, SPLIT, WALLS, false>;
     static bool attr[2] = {false, false};
     if (!attr[whole]) {
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
