@@ -21,13 +21,12 @@
 
 #include <type_traits>
 
-// unroll factor of the plane loop (2H+1 would turn the queue rotation into
-// register renaming, but the extra live ranges cost more than the moves)
+// default unroll factor of the plane loop (2H + 1 turns the queue rotation into
+// register renaming; where the extra live ranges fit the registers a kernel asks
+// for it, in the others they cost more than the moves)
 #ifndef NOVA_MARCH_UNROLL
 #define NOVA_MARCH_UNROLL 1
 #endif
-#define NOVA_PRAGMA(x) _Pragma(#x)
-#define NOVA_UNROLL(n) NOVA_PRAGMA(unroll n)
 
 namespace nova {
 
@@ -63,7 +62,7 @@ template <typename T, class Ld> struct MarchLd<T, Ld, std::void_t<typename Ld::R
 // body(idx, q, vx, vy, vz) runs for valid threads once per plane, with idx
 // the thread's node, q the register queue and vx/vy/vz(c, s) the neighbour
 // accessors along i, j, k.
-template <typename T, int H, int NC, bool WALLS, class Ld, class Pre, class Body>
+template <typename T, int H, int NC, bool WALLS, int UNROLL = NOVA_MARCH_UNROLL, class Ld, class Pre, class Body>
 __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, TileSmem<T, H, NC> &sm, const Ld &ld,
                                            int ib, int ie, Pre &&pre, Body &&body)
 {
@@ -159,7 +158,7 @@ __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, Til
         if (valid) pre(plane + colOff, true);
     }
 
-    NOVA_UNROLL(NOVA_MARCH_UNROLL)
+#pragma unroll UNROLL
     for (int i = ib; i < ie; i++) {
         const int b = (i - ib) & 1;
 #pragma unroll
@@ -202,11 +201,11 @@ __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, Til
     }
 }
 
-template <typename T, int H, int NC, bool WALLS, class Ld, class Body>
+template <typename T, int H, int NC, bool WALLS, int UNROLL = NOVA_MARCH_UNROLL, class Ld, class Body>
 __device__ __forceinline__ void tile_march(const Geo &g, const Walls<T> &wl, TileSmem<T, H, NC> &sm, const Ld &ld,
                                            int ib, int ie, Body &&body)
 {
-    tile_march<T, H, NC, WALLS>(g, wl, sm, ld, ib, ie, NoPre{}, body);
+    tile_march<T, H, NC, WALLS, UNROLL>(g, wl, sm, ld, ib, ie, NoPre{}, body);
 }
 
 // of a tile march (k tiles x j tiles x i chunks)

@@ -14,6 +14,9 @@
 // U 551, 638, 631, 562 -> 495, 533, 532, 615 us, rho 246, 271, 272, 259 -> 228, 242,
 // 242, 282 us, T 298, 322, 321, 300 -> 296, 305, 303, 373 us; the last stage reads
 // Y1 and Y2 where it read one sum, the others no longer read and write it.
+// The U and rho loops unroll by the queue period: U -> 477, 518, 515, 622, rho ->
+// 224, 237, 237, 281 (96 x 75 x 90: U 28.1, 30.0, 30.1, 33.9 -> 27.4, 29.0, 29.3,
+// 31.9); the T loop spills.
 //   U:   RHS = -div(rho U, U) - grad p + laplacian(mu, U) [- (rho T) g]
 //   rho: RHS = -div(rho U)
 //   T:   RHS = -div(rho U, T) + laplacian(ka, T)
@@ -115,7 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wc_u(Geo g, Coef<double> co, co
         Tc = Tn;
         if (BUOY && load) Tn = a.T[nidx];
     };
-    tile_march<double, kH, 5, false>(g, wl, sm, ld, ib, ie, pre, [&](long long idx, auto &q, const auto &vx,
+    tile_march<double, kH, 5, false, 2 * kH + 1>(g, wl, sm, ld, ib, ie, pre, [&](long long idx, auto &q, const auto &vx,
                                                                     const auto &vy, const auto &vz) {
         double y1[3] = {0, 0, 0}, y2[3] = {0, 0, 0};
         if constexpr (STAGE == 3) {
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_wc_rho(Geo g, Coef<double> co, 
             }
         }
     };
-    tile_march<double, kH, 4, false>(g, wl, sm, ld, ib, ie, pre, [&](long long idx, auto &q, const auto &vx,
+    tile_march<double, kH, 4, false, 2 * kH + 1>(g, wl, sm, ld, ib, ie, pre, [&](long long idx, auto &q, const auto &vx,
                                                                     const auto &vy, const auto &vz) {
         double divV = 0.0;
         auto dir = [&](const auto &v, int d, const double *aa) {
