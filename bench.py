@@ -42,9 +42,9 @@ NU = 1.0 / 1600.0
 MHD_NU = 1.0 / 1000.0
 CFL = 0.3
 # algorithmic HBM bytes per grid point for one classical RK4 step of the NS
-# stage kernels (3 components): FP64 stages 72 + 120 + 120 + 72; FP32-split
+# stage kernels (3 components): FP64 stages 48 + 72 + 72 + 120; FP32-split
 # stages 36 + 60 + 60 + 72 (see the stage-kernel epilogue in nova_stage.cu)
-STAGE_BYTES = {"f64": 384.0, "f32split": 228.0}
+STAGE_BYTES = {"f64": 312.0, "f32split": 228.0}
 STAGE_LAUNCHES_PER_STEP = 4
 # fdMatrix::solve, FP64 bytes per node per iteration that the algorithm must
 # move: the residual reads the 8 matrix fields and x (72); each of the three
@@ -547,11 +547,12 @@ def hbm_roof(alg_bytes, sec, what):
 SHEAR_STAGE_BYTES = {"f64": 72.0, "f32split": 60.0}
 SHEAR_STEP_BYTES = {k: 4 * (v + 32 + 48 + 56) for k, v in SHEAR_STAGE_BYTES.items()}
 #   MHD jet, the app's scheme (literal U loop: one stage reading U, B and
-#   writing U*; projection; classical B loop with U frozen: 96, 144, 144, 96
+#   writing U*; projection; classical B loop with U frozen: 72, 96, 96, 144
 #   FP64 / 48, 72, 72, 84 split; cleaning projection)
-JET_STEP_BYTES = {"f64": 72 + 120 + 96 + 144 + 144 + 96 + 120, "f32split": 60 + 120 + 48 + 72 + 72 + 84 + 120}
-#   weakly compressible: 5 evolved components at 136 B each (4 RK stages)
-WC_STEP_BYTES = 5 * 136.0
+JET_STEP_BYTES = {"f64": 72 + 120 + 72 + 96 + 96 + 144 + 120, "f32split": 60 + 120 + 48 + 72 + 72 + 84 + 120}
+#   weakly compressible: 5 evolved components at 104 B each (RK stages
+#   16, 24, 24, 40)
+WC_STEP_BYTES = 5 * 104.0
 
 
 def shear_leg(args, nova, torch, dist, world):
