@@ -27,7 +27,7 @@ using namespace nova;
 // per operator call (ex::grad, ex::div, ...); with a cudaMalloc and a cudaFree
 // each (about 0.35 + 0.3 ms) the operator calls of a 128^3 step took 5.5 ms
 // around 1.3 ms of kernels, now 1.4 ms.  A buffer is put here only after the
-// work that uses it has been waited for.  At most kKeep bytes stay (the oldest
+// work that uses it has been waited for (nova_field_destroy, nova_fdm_destroy).  At most kKeep bytes stay (the oldest
 // go first); all go when an allocation fails or the context is destroyed,
 // after which buffers still held by fields or matrices are freed directly.
 class BufCache {
@@ -89,8 +89,11 @@ struct nova_field {
     double *d64;
     float *hi, *lo;
     nova_bc bc;  // setBC of the reference field: index face + 6*comp
-    const nova_ctx *owner;           // the context whose stream carries the field's work
+    const nova_ctx *owner;           // the context that made it
     std::shared_ptr<BufCache> home;  // where its buffers go back to
+    // an entry point of another context has taken the field (on_mesh): its work
+    // may be on any stream, and stays there after a call that returned early
+    mutable int shared = 0;
 };
 
 namespace {
@@ -664,10 +667,13 @@ nova_status poisson_device_dct(nova_ctx *ctx, const double *rhs, double *p, bool
 
 // a field of this context's mesh: its buffers hold the context's N3 nodes per
 // component (a field made by a context of another mesh would be read or
-// written past its end)
+// written past its end).  Every entry point that hands a field's buffers to the
+// device passes here, so a field that another context uses is marked.
 bool on_mesh(const nova_ctx *ctx, const nova_field *f)
 {
-    return f && f->n3 == ctx->g.N3;
+    if (!f || f->n3 != ctx->g.N3) return false;
+    if (f->owner != ctx) __atomic_store_n(&f->shared, 1, __ATOMIC_RELAXED);
+    return true;
 }
 
 bool valid_field(const nova_ctx *ctx, const nova_field *f, int nc)
@@ -888,9 +894,10 @@ extern "C" nova_status nova_field_create(nova_ctx *ctx, int ncomp, int precision
 extern "C" nova_status nova_field_destroy(nova_ctx *ctx, nova_field *f)
 {
     if (!f) return NOVA_E_INVALID;
-    // the owner's stream carries every use that has not been waited for (a copy
-    // through another context waits for itself)
-    if (ctx && ctx == f->owner)
+    // a field that only its owner used has all its work on the owner's stream;
+    // any other may have it on any stream, and the next field that gets the
+    // buffer is ordered behind the owner's alone
+    if (ctx && ctx == f->owner && !__atomic_load_n(&f->shared, __ATOMIC_RELAXED))
         cudaStreamSynchronize(ctx->stream);
     else
         cudaDeviceSynchronize();
@@ -990,7 +997,7 @@ static nova_status soa_in(nova_ctx *ctx, nova_field *f, const double *src, cudaM
         ctx->launches += 1;
         CKL("k_split");
     }
-    if (f->owner != ctx) CK(cudaStreamSynchronize(ctx->stream));  // nova_field_destroy waits for the owner's stream
+    if (f->owner != ctx) CK(cudaStreamSynchronize(ctx->stream));  // the owner's next use is on another stream
     return NOVA_OK;
 }
 
@@ -2604,6 +2611,8 @@ extern "C" nova_status nova_fdm_solve(nova_ctx *ctx, nova_fdm *a, double tol, in
     if (cur != a->x->d64) {
         CK(cudaMemcpyAsync(a->x->d64, cur, sizeof(double) * g.N3, cudaMemcpyDeviceToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
+    } else if (a->x->owner != ctx) {
+        CK(cudaStreamSynchronize(ctx->stream));  // the last sweeps wrote x: the owner's next use is on another stream
     }
     if (its) *its = n;
     if (res) *res = r;
