@@ -1,5 +1,6 @@
 // C ABI of libnova_b200 (include/nova_gpu.h): contexts, fields, the ex::
 // drop-in operators, the cuFFT projection and the fused time advance.
+#include "nova_bufcache.h"
 #include "nova_gpu.h"
 #include "nova_internal.cuh"
 #include "nova_mesh.cuh"
@@ -14,73 +15,12 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
-#include <mutex>
 #include <new>
 #include <string>
 #include <utility>
 #include <vector>
 
 using namespace nova;
-
-// Device buffers of dropped fields and matrices that a context keeps for its
-// next ones, by size.  The reference's explicit programs make and drop a field
-// per operator call (ex::grad, ex::div, ...); with a cudaMalloc and a cudaFree
-// each (about 0.35 + 0.3 ms) the operator calls of a 128^3 step took 5.5 ms
-// around 1.3 ms of kernels, now 1.4 ms.  A buffer is put here only after the
-// work that uses it has been waited for (nova_field_destroy, nova_fdm_destroy).  At most kKeep bytes stay (the oldest
-// go first); all go when an allocation fails or the context is destroyed,
-// after which buffers still held by fields or matrices are freed directly.
-class BufCache {
-public:
-    static constexpr size_t kKeep = size_t(1) << 30;
-    void *take(size_t bytes)
-    {
-        std::lock_guard<std::mutex> l(mu_);
-        for (size_t q = idle_.size(); q-- > 0;)
-            if (idle_[q].second == bytes) {
-                void *p = idle_[q].first;
-                held_ -= bytes;
-                idle_.erase(idle_.begin() + q);
-                return p;
-            }
-        return nullptr;
-    }
-    void put(void *p, size_t bytes)
-    {
-        if (!p) return;
-        std::lock_guard<std::mutex> l(mu_);
-        if (!open_ || bytes > kKeep) {
-            cudaFree(p);
-            return;
-        }
-        while (held_ + bytes > kKeep) drop();
-        idle_.emplace_back(p, bytes);
-        held_ += bytes;
-    }
-    void trim()
-    {
-        std::lock_guard<std::mutex> l(mu_);
-        while (!idle_.empty()) drop();
-    }
-    void close()
-    {
-        trim();
-        std::lock_guard<std::mutex> l(mu_);
-        open_ = false;
-    }
-
-private:
-    void drop()
-    {
-        cudaFree(idle_.front().first);
-        held_ -= idle_.front().second;
-        idle_.erase(idle_.begin());
-    }
-    std::mutex mu_;
-    std::vector<std::pair<void *, size_t>> idle_;
-    size_t held_ = 0;
-    bool open_ = true;
-};
 
 struct nova_field {
     int nc;
