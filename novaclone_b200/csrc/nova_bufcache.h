@@ -7,6 +7,7 @@
 
 #include <memory>
 #include <mutex>
+#include <new>
 #include <utility>
 #include <vector>
 
@@ -47,7 +48,12 @@ public:
             return;
         }
         while (held_ + bytes > kKeep) drop();
-        idle_.emplace_back(p, bytes);
+        try {
+            idle_.emplace_back(p, bytes);
+        } catch (const std::bad_alloc &) {  // the callers are C entry points
+            cudaFree(p);
+            return;
+        }
         held_ += bytes;
     }
     void trim()

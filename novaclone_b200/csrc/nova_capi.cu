@@ -644,8 +644,12 @@ extern "C" nova_status nova_create(const nova_mesh_desc *md, nova_ctx **out)
         if (md->N[a] < 1 || !(md->L[a] > 0.0) || (md->walls[a] != 0 && md->walls[a] != 1)) return NOVA_E_INVALID;
     if (md->walls[0] || md->walls[2]) return NOVA_E_UNSUPPORTED;  // walls in y only
     if (md->walls[1] && md->N[1] < md->m) return NOVA_E_INVALID;   // the mirrored halo needs m/2 nodes per wall
-    nova_ctx *ctx = new (std::nothrow) nova_ctx();
-    if (!ctx) return NOVA_E_OOM;
+    nova_ctx *ctx = nullptr;
+    try {
+        ctx = new nova_ctx();  // its members allocate too
+    } catch (const std::bad_alloc &) {
+        return NOVA_E_OOM;
+    }
     ctx->md = *md;
     ctx->h = md->m / 2;
     if (const char *impl = std::getenv("NOVA_STAGE_IMPL")) {

@@ -4,7 +4,9 @@
 
 #include <atomic>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <new>
 #include <thread>
 
 static std::atomic<long> freed{0};
@@ -16,6 +18,18 @@ extern "C" cudaError_t cudaFree(void *)
 }
 
 using nova::BufCache;
+
+// host allocation failures on demand
+static bool no_memory = false;
+
+void *operator new(size_t n)
+{
+    void *p = no_memory ? nullptr : std::malloc(n ? n : 1);
+    if (!p) throw std::bad_alloc();
+    return p;
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 static void *buf(long n) { return reinterpret_cast<void *>(n + 1); }
 
@@ -70,8 +84,25 @@ static bool bound_and_reuse()
     return ok && freed == 4 && cache->take(64) == nullptr;
 }
 
+// a buffer that the list cannot take for want of host memory is freed, and nothing is thrown
+static bool host_memory()
+{
+    freed = 0;
+    auto cache = std::make_shared<BufCache>();
+    no_memory = true;
+    bool thrown = false;
+    try {
+        cache->put(buf(0), 64);
+    } catch (...) {
+        thrown = true;
+    }
+    no_memory = false;
+    return !thrown && freed == 1 && cache->take(64) == nullptr;
+}
+
 int main(int, char **argv)
 {
+    if (!std::strcmp(argv[1], "host_memory")) return host_memory() ? 0 : 1;
     if (!std::strcmp(argv[1], "close_race")) return close_race() ? 0 : 1;
     if (!std::strcmp(argv[1], "bound_and_reuse")) return bound_and_reuse() ? 0 : 1;
     return 2;
