@@ -5,6 +5,7 @@
 
 #include <cuda_runtime_api.h>
 
+#include <algorithm>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -18,15 +19,36 @@ namespace nova {
 // each (about 0.35 + 0.3 ms) the operator calls of a 128^3 step took 5.5 ms
 // around 1.3 ms of kernels, now 1.4 ms.  A buffer is put here only after the
 // work that uses it has been waited for (nova_field_destroy, nova_fdm_destroy).
-// At most kKeep bytes stay (the oldest go first); all go when an allocation
-// fails or the context is destroyed, after which buffers still held by fields
-// or matrices are freed directly.
+// At most kKeep bytes stay (the oldest go first).  All go when the context is
+// destroyed, after which buffers still held by fields or matrices are freed
+// directly, and when an allocation or an FFT plan of any context in the process
+// fails, which is then tried again (retry).
 class BufCache {
 public:
     static constexpr size_t kKeep = size_t(1) << 30;
-    BufCache() = default;
+    BufCache()
+    {
+        Live &r = live();
+        std::lock_guard<std::mutex> l(r.mu);
+        r.all.push_back(this);
+    }
     BufCache(const BufCache &) = delete;
-    ~BufCache() { trim(); }
+    ~BufCache()
+    {
+        {
+            Live &r = live();
+            std::lock_guard<std::mutex> l(r.mu);
+            r.all.erase(std::find(r.all.begin(), r.all.end(), this));
+        }
+        trim();
+    }
+    // make() -> 0 or an error code; after an error the idle buffers of every
+    // context go back to the device, and if there were any it is called once more
+    template <class Make> static auto retry(Make &&make) -> decltype(make())
+    {
+        auto e = make();
+        return static_cast<int>(e) != 0 && trim_all() ? make() : e;
+    }
     void *take(size_t bytes)
     {
         std::lock_guard<std::mutex> l(mu_);
@@ -56,10 +78,12 @@ public:
         }
         held_ += bytes;
     }
-    void trim()
+    bool trim()  // whether there was anything to free
     {
         std::lock_guard<std::mutex> l(mu_);
+        const bool any = !idle_.empty();
         while (!idle_.empty()) drop();
+        return any;
     }
     // from here on put() frees (set under the lock that empties the list: a
     // buffer put between the two would stay allocated for good)
@@ -71,6 +95,23 @@ public:
     }
 
 private:
+    struct Live {  // the caches of the process; never destroyed: contexts may outlive static objects
+        std::mutex mu;
+        std::vector<BufCache *> all;
+    };
+    static Live &live()
+    {
+        static Live *r = new Live;
+        return *r;
+    }
+    static bool trim_all()
+    {
+        Live &r = live();
+        std::lock_guard<std::mutex> l(r.mu);
+        bool any = false;
+        for (BufCache *c : r.all) any = c->trim() || any;
+        return any;
+    }
     void drop()
     {
         cudaFree(idle_.front().first);

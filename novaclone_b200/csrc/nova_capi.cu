@@ -214,17 +214,27 @@ nova_status fft_check(nova_ctx *ctx, cufftResult r, const char *what)
     return fail(ctx, NOVA_E_CUDA, std::string(what) + ": cuFFT error " + std::to_string((int)r));
 }
 
+// make() -> a cuFFT plan, whose work areas are cuFFT's own allocations
+template <class Make> nova_status fft_plan(nova_ctx *ctx, const char *what, Make make)
+{
+    const cufftResult r = BufCache::retry([&] {
+        const cufftResult q = make();
+        if (q != CUFFT_SUCCESS) cudaGetLastError();  // reported by its value
+        return q;
+    });
+    return fft_check(ctx, r, what);
+}
+
 template <typename T>
 nova_status dalloc(nova_ctx *ctx, T **p, size_t n)
 {
     if (*p) return NOVA_OK;
     const size_t bytes = sizeof(T) * (n ? n : 1);
-    cudaError_t e = cudaMalloc((void **)p, bytes);
-    if (e == cudaErrorMemoryAllocation) {  // the idle buffers first
-        cudaGetLastError();
-        ctx->bufs->trim();
-        e = cudaMalloc((void **)p, bytes);
-    }
+    const cudaError_t e = BufCache::retry([&] {
+        const cudaError_t r = cudaMalloc((void **)p, bytes);
+        if (r == cudaErrorMemoryAllocation) cudaGetLastError();  // reported by its value
+        return r;
+    });
     if (e != cudaSuccess) *p = nullptr;
     return cuda_check(ctx, e, "cudaMalloc");
 }
@@ -399,11 +409,15 @@ nova_status ensure_fft(nova_ctx *ctx, bool split)
     int cembed3[3] = {g.N0, ny, g.N2 / 2 + 1}, cembed2[2] = {ny, g.N2 / 2 + 1};
     int *n = pi ? n2d : n3d, *rembed = pi ? rembed2 : rembed3, *cembed = pi ? cembed2 : cembed3;
     const int rdist = (pi ? 1 : g.N0) * g.N1 * g.N2, cdist = (pi ? 1 : g.N0) * ny * (g.N2 / 2 + 1);
-    if ((s = fft_check(ctx, cufftPlanMany(&F.f, rank, n, rembed, 1, rdist, cembed, 1, cdist, CUFFT_D2Z, batch),
-                       "cufftPlanMany D2Z")) != NOVA_OK)
+    s = fft_plan(ctx, "cufftPlanMany D2Z", [&] {
+        return cufftPlanMany(&F.f, rank, n, rembed, 1, rdist, cembed, 1, cdist, CUFFT_D2Z, batch);
+    });
+    if (s != NOVA_OK)
         return s;
-    if ((s = fft_check(ctx, cufftPlanMany(&F.b, rank, n, cembed, 1, cdist, rembed, 1, rdist, CUFFT_Z2D, batch),
-                       "cufftPlanMany Z2D")) != NOVA_OK) {
+    s = fft_plan(ctx, "cufftPlanMany Z2D", [&] {
+        return cufftPlanMany(&F.b, rank, n, cembed, 1, cdist, rembed, 1, rdist, CUFFT_Z2D, batch);
+    });
+    if (s != NOVA_OK) {
         cufftDestroy(F.f);
         return s;
     }
@@ -511,11 +525,15 @@ nova_status poisson_device_dct1(nova_ctx *ctx, const double *rhs, double *p, boo
     if (!own && !ctx->dct2_plans) {
         // element (i, j, k) of a batch-j plane at j N2 + i N1 N2 + k; spectrum at (i N1 + j) nzh + kz
         int n[2] = {g.N0, g.N2}, rin[2] = {g.N0, (int)g.N12}, cin[2] = {g.N0, g.N1 * nzh};
-        if ((s = fft_check(ctx, cufftPlanMany(&ctx->dct2_f, 2, n, rin, 1, g.N2, cin, 1, nzh, CUFFT_D2Z, g.N1),
-                           "cufftPlanMany D2Z (walls, DCT)")) != NOVA_OK)
+        s = fft_plan(ctx, "cufftPlanMany D2Z (walls, DCT)", [&] {
+            return cufftPlanMany(&ctx->dct2_f, 2, n, rin, 1, g.N2, cin, 1, nzh, CUFFT_D2Z, g.N1);
+        });
+        if (s != NOVA_OK)
             return s;
-        if ((s = fft_check(ctx, cufftPlanMany(&ctx->dct2_b, 2, n, cin, 1, nzh, rin, 1, g.N2, CUFFT_Z2D, g.N1),
-                           "cufftPlanMany Z2D (walls, DCT)")) != NOVA_OK) {
+        s = fft_plan(ctx, "cufftPlanMany Z2D (walls, DCT)", [&] {
+            return cufftPlanMany(&ctx->dct2_b, 2, n, cin, 1, nzh, rin, 1, g.N2, CUFFT_Z2D, g.N1);
+        });
+        if (s != NOVA_OK) {
             cufftDestroy(ctx->dct2_f);
             return s;
         }
@@ -571,11 +589,15 @@ nova_status poisson_device_dct(nova_ctx *ctx, const double *rhs, double *p, bool
     nova_status s;
     if (!ctx->dct_extend && pois_dct_fits(g, ny)) return poisson_device_dct1(ctx, rhs, p, split);
     if (!ctx->dct_plans) {
-        if ((s = fft_check(ctx, cufftPlan3d(&ctx->dct_f, g.N0, 2 * ny, g.N2, CUFFT_D2Z), "cufftPlan3d D2Z (walls)")) !=
-            NOVA_OK)
+        s = fft_plan(ctx, "cufftPlan3d D2Z (walls)", [&] {
+            return cufftPlan3d(&ctx->dct_f, g.N0, 2 * ny, g.N2, CUFFT_D2Z);
+        });
+        if (s != NOVA_OK)
             return s;
-        if ((s = fft_check(ctx, cufftPlan3d(&ctx->dct_b, g.N0, 2 * ny, g.N2, CUFFT_Z2D), "cufftPlan3d Z2D (walls)")) !=
-            NOVA_OK) {
+        s = fft_plan(ctx, "cufftPlan3d Z2D (walls)", [&] {
+            return cufftPlan3d(&ctx->dct_b, g.N0, 2 * ny, g.N2, CUFFT_Z2D);
+        });
+        if (s != NOVA_OK) {
             cufftDestroy(ctx->dct_f);
             return s;
         }

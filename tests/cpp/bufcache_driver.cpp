@@ -22,14 +22,14 @@ using nova::BufCache;
 // host allocation failures on demand
 static bool no_memory = false;
 
-void *operator new(size_t n)
+__attribute__((noinline)) void *operator new(size_t n)
 {
     void *p = no_memory ? nullptr : std::malloc(n ? n : 1);
     if (!p) throw std::bad_alloc();
     return p;
 }
-void operator delete(void *p) noexcept { std::free(p); }
-void operator delete(void *p, size_t) noexcept { std::free(p); }
+__attribute__((noinline)) void operator delete(void *p) noexcept { std::free(p); }
+__attribute__((noinline)) void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 static void *buf(long n) { return reinterpret_cast<void *>(n + 1); }
 
@@ -100,8 +100,30 @@ static bool host_memory()
     return !thrown && freed == 1 && cache->take(64) == nullptr;
 }
 
+// a failed allocation gives back the idle buffers of every context and is tried once more
+static bool out_of_memory()
+{
+    freed = 0;
+    auto a = std::make_shared<BufCache>(), b = std::make_shared<BufCache>(), gone = std::make_shared<BufCache>();
+    int calls = 0;
+    auto fails = [&] { return ++calls, 7; };
+    bool ok = BufCache::retry(fails) == 7 && calls == 1;  // nothing to give back: no second try
+    a->put(buf(0), 64);
+    b->put(buf(1), 64);
+    gone->put(buf(2), 64);
+    gone.reset();
+    calls = 0;
+    ok = ok && freed == 1 && BufCache::retry([&] { return ++calls, freed == 3 ? 0 : 2; }) == 0 && calls == 2;
+    a->put(buf(3), 64);
+    calls = 0;
+    ok = ok && BufCache::retry([&] { return ++calls, 0; }) == 0 && calls == 1 && freed == 3;
+    ok = ok && BufCache::retry(fails) == 7 && calls == 3 && freed == 4;
+    return ok && a->take(64) == nullptr && b->take(64) == nullptr;
+}
+
 int main(int, char **argv)
 {
+    if (!std::strcmp(argv[1], "out_of_memory")) return out_of_memory() ? 0 : 1;
     if (!std::strcmp(argv[1], "host_memory")) return host_memory() ? 0 : 1;
     if (!std::strcmp(argv[1], "close_race")) return close_race() ? 0 : 1;
     if (!std::strcmp(argv[1], "bound_and_reuse")) return bound_and_reuse() ? 0 : 1;

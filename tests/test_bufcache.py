@@ -21,7 +21,8 @@ def driver(tmp_path_factory):
 
 # close_race: buffers dropped on other threads while the context is destroyed
 # host_memory: no room on the host to note a buffer (an exception must not leave a C entry point)
-@pytest.mark.parametrize("scenario", ["bound_and_reuse", "close_race", "host_memory"])
+# out_of_memory: a failed device allocation or FFT plan gets the idle buffers of every context
+@pytest.mark.parametrize("scenario", ["bound_and_reuse", "close_race", "host_memory", "out_of_memory"])
 def test_every_buffer_is_freed_once(driver, scenario):
     r = subprocess.run([driver, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout
