@@ -43,7 +43,8 @@ constexpr int kWarps = TJ;
 // 8 x 32 x 232 + 4 x 32 x 24 = 62464 of 12 x 32 x 168 = 64512 at launch (at 168 the
 // unrolled loop spilled 100 B; 256^3, s = 4..1: 579, 705, 716, 655 -> 493, 557, 571,
 // 565 us; MHD pieces at 128^3 100-105 -> 83-90 us)
-constexpr int kThreads = kTK * (TJ + 4);
+using Split = RegSplit<kTK * TJ, 232, 4 * kTK, 24>;
+constexpr int kThreads = Split::kThreads;
 constexpr int kRing = 7;
 constexpr int kERing = 3;
 constexpr int kLRB = 8;                      // rows of the k-halo box
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     // ---- producer warp: lane 0 issues every load of the block ----
     if (ty >= TJ) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        Split::producer();
         if (ty > TJ || lane != 0) return;
         const bool jlo = j0 < H, jhi = j0 + TJ >= g.N1;
         const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + w == g.N2) ? 0 : k0 + kTK;
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 
     // ---- consumer warps ----
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    Split::consumer();
     auto release = [&](uint32_t bar) {
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
@@ -315,6 +316,7 @@ cudaError_t launch_adj_s(const Geo &g, const Coef<double> &co, const double *ia,
     constexpr size_t smem = adj_smem_bytes<NE>();
     static bool attr = false;
     if (!attr) {
+        if (const cudaError_t e = reg_split_ok(Split{}, k_adj_tma<KIND, S>); e != cudaSuccess) return e;
         cudaFuncSetAttribute(k_adj_tma<KIND, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }

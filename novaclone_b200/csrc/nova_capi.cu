@@ -445,6 +445,8 @@ nova_status stage_fail(nova_ctx *ctx, cudaError_t e)
         return fail(ctx, NOVA_E_UNSUPPORTED,
                     "NOVA_STAGE_IMPL=tma: the TMA stage kernel needs N2 >= 32 with whole 16-byte rows and no one or two columns beyond a 32-column tile, and N1 at least twice the tile height (16 rows FP64, 8 FP32) with, for periodic y, no one or two rows beyond a tile; walls in y only in FP32");
     if (e == cudaErrorInvalidValue) return fail(ctx, NOVA_E_CUDA, "stage kernel: cuTensorMapEncodeTiled failed");
+    if (e == cudaErrorInvalidConfiguration)
+        return fail(ctx, NOVA_E_CUDA, "stage kernel: compiled with too few registers for its register split");
     return cuda_check(ctx, e, "stage kernel");
 }
 

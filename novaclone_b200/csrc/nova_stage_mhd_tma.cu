@@ -40,7 +40,8 @@ template <typename T> struct MhdCfg {
     // the producer has a warpgroup of its own, which hands its registers to the
     // consumers: FP64 8 x 32 x 232 + 4 x 32 x 24 = 62464 of 12 x 32 x 168 = 64512
     // at launch, FP32 16 x 32 x 112 + 4 x 32 x 24 = 60416 of 20 x 32 x 96 = 61440
-    static constexpr int kThreads = kTK * (TJ + 4);
+    using Split = RegSplit<kTK * TJ, sizeof(T) == 8 ? 232 : 112, 4 * kTK, 24>;
+    static constexpr int kThreads = Split::kThreads;
     static constexpr int kRing = 7;
     template <int NE> static constexpr int kERing = (sizeof(T) == 8 && NE == 3) ? 2 : 3;
     static constexpr int kTcbE = (TJ + 2 * kH) * kRowE;  // one field's halo'd rows
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
 
     // ---- producer warp: lane 0 issues every load of the block ----
     if (ty >= TJ) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        C::Split::producer();
         if (ty > TJ || lane != 0) return;
         const bool jlo = j0 < H, jhi = j0 + TJ >= g.N1;
         const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + w == g.N2) ? 0 : k0 + kTK;
@@ -213,10 +214,7 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
     const T iak = ia[k0 + txc];
     const T c2k = STRETCH ? corr2[k0 + txc] : T(0);
 
-    if constexpr (sizeof(T) == 8)
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
-    else
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+    C::Split::consumer();
 
     // slot offsets within a field: centre, and the k neighbour at s (inside the
     // row box or in the left/right halo boxes); component stride kTK in both
@@ -384,6 +382,7 @@ cudaError_t launch_mhd(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     auto kern = whole ? k_mhd_tma<T, PHYS, STAGE, STRETCH, Args, true> : k_mhd_tma<T, PHYS, STAGE, STRETCH, Args, false>;
     static bool attr[2] = {false, false};
     if (!attr[whole]) {
+        if (const cudaError_t e = reg_split_ok(typename Cf::Split{}, kern); e != cudaSuccess) return e;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         attr[whole] = true;

@@ -56,10 +56,11 @@ constexpr int kLRB = 8;         // rows of one k-halo box
 // one producer warp, whose elected lane issues the loads in the order the
 // consumers need them and blocks on the ring's `empty` barriers alone, so it
 // never delays the arithmetic.
+using Split64 = RegSplit<kTK * 16, 112, 4 * kTK, 24>;  // FP64: 16 consumer warps
 template <typename T> struct TmaCfg {
     static constexpr int TJ = sizeof(T) == 8 ? 16 : 8;
     static constexpr int kWarps = sizeof(T) == 8 ? TJ : TJ / 2;  // consumer warps
-    static constexpr int kThreads = kTK * (kWarps + (sizeof(T) == 8 ? 4 : 1));  // plus the producer warp (FP64: its warpgroup)
+    static constexpr int kThreads = sizeof(T) == 8 ? Split64::kThreads : kTK * (kWarps + 1);  // plus the producer warp (FP64: its warpgroup)
     static constexpr int kBlocksPerSM = sizeof(T) == 8 ? 1 : 3;
     static constexpr int kRing = 7;   // stencil slots: the queue head runs kRing - 2H - 1 planes behind the loads
     // epilogue slots (two for the FP64 last stage, whose three fields leave no room for a third)
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
 
     // ---- producer warp: lane 0 issues every load of the block ----
     if (ty >= C::kWarps) {
-        if constexpr (sizeof(T) == 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+        if constexpr (sizeof(T) == 8) Split64::producer();
         if (ty > C::kWarps || lane != 0) return;
         const bool jlo = j0 < H, jhi = j0 + TJ >= g.N1;
         const int kl = (k0 == 0 ? g.N2 : k0) - 4, kr = (k0 + w == g.N2) ? 0 : k0 + kTK;
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
     if constexpr (DIAG) dacc.init();
     if constexpr (sizeof(T) == 8) {
         // 16 x 32 x 112 + 4 x 32 x 24 = 60416 registers of the 20 x 32 x 96 = 61440 at launch
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+        Split64::consumer();
         const bool on = WHOLE || (tx < w && ty < hrows);
         const int txc = WHOLE ? tx : min(tx, w - 1);  // lanes past the valid columns read the last one and store nothing
         const T iak = ia[k0 + txc];
@@ -600,6 +601,8 @@ cudaError_t launch_tma(const Geo &g, const Coef<T> &co, const T *ia, const T *co
                       : k_stage_tma<T, STAGE, STRETCH, Args, DIAG, WALLS, DIAG>;
     static bool attr[2] = {false, false};
     if (!attr[whole]) {
+        if constexpr (sizeof(T) == 8)
+            if (const cudaError_t e = reg_split_ok(Split64{}, kern); e != cudaSuccess) return e;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         attr[whole] = true;

@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "nova_regsplit.h"
+
 namespace nova {
 
 constexpr unsigned long long kWaitLimitNs = 1000000000ull;  // 1 s
@@ -101,6 +103,26 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tma_encode_tiled()
         return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
     }();
     return fn;
+}
+
+// Registers of a warp-specialised kernel: CONSUMERS threads rise to INC, PRODUCERS
+// (whole warpgroups) fall to DEC.
+template <int CONSUMERS, int INC, int PRODUCERS, int DEC> struct RegSplit {
+    static_assert(CONSUMERS % 128 == 0 && PRODUCERS % 128 == 0, "setmaxnreg is executed by whole warpgroups");
+    static constexpr int kThreads = CONSUMERS + PRODUCERS;
+    __device__ static void consumer() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(INC)); }
+    __device__ static void producer() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(DEC)); }
+};
+
+// whether the registers the compiler gave `kern` cover the split (before its
+// first launch: the consumers' wait for them has no bound)
+template <int CONSUMERS, int INC, int PRODUCERS, int DEC, class Kern>
+cudaError_t reg_split_ok(RegSplit<CONSUMERS, INC, PRODUCERS, DEC>, Kern kern)
+{
+    cudaFuncAttributes at;
+    const cudaError_t e = cudaFuncGetAttributes(&at, kern);
+    if (e != cudaSuccess) return e;
+    return reg_split_fits(at.numRegs, CONSUMERS, INC, PRODUCERS, DEC) ? cudaSuccess : cudaErrorInvalidConfiguration;
 }
 
 // 3-D tiled load (a single component of a field: dims k, j, i)
