@@ -2636,7 +2636,8 @@ extern "C" nova_status nova_advance_wc(nova_ctx *ctx, const nova_wc_desc *wd, no
     const Geo &g = ctx->g;
     const bool str = ctx->md.hyperbolic_z != 0;
     double *w0 = ctx->w64[0], *w1 = ctx->w64[1], *w2 = ctx->w64[2];
-    // one RK loop of the quantity q (stored in qf): stage states in w0, w1, w2, the last stage writes qf
+    // one RK loop of the quantity q (stored in qf): stage states in w0, w1, w2 (T loop: w0, w1, w0, and
+    // the accumulator in w2), the last stage writes qf
     auto loop = [&](int which, double *qf, double visc) {
         WcArgs a{};
         a.U = st->U->d64;
@@ -2646,12 +2647,14 @@ extern "C" nova_status nova_advance_wc(nova_ctx *ctx, const nova_wc_desc *wd, no
         a.Q0 = qf;
         a.Y1 = w0;
         a.Y2 = w1;
+        a.acc = w2;
         a.dt = wd->dt;
         a.visc = visc;
         a.eos_k = wd->eos_k;
         for (int c = 0; c < 3; c++) a.g[c] = wd->g[c];
-        const double *ys[4] = {qf, w0, w1, w2};
-        double *yn[4] = {w0, w1, w2, qf};
+        double *y3 = which == WC_LOOP_T ? w0 : w2;
+        const double *ys[4] = {qf, w0, w1, y3};
+        double *yn[4] = {w0, w1, y3, qf};
         for (int stage = 0; stage < 4; stage++) {
             ProfScope ps(ctx, NOVA_K_STAGE);
             a.Y = ys[stage];

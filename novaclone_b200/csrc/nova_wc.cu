@@ -4,18 +4,25 @@
 // march of nova_tile.cuh (FP64, periodic meshes).
 //
 // Every loop is the reference's classical RK4 on a conserved quantity q*rho
-// with rho frozen during the U and T loops (app/shearLayerWC/UEqn.H:11-41,
-// TEqn.H:91-117; rho itself: rhoEqn.H:53-78).  Its sums divide through by rho,
-// and the stage states carry the increments, so no accumulator is kept:
+// with rho frozen during the U and T loops (RK4W = 1/6, 1/3, 1/3, 1/6):
+//   d   = dt * RHS(stage state)
+//   acc = acc + RK4W[s] d                       (acc starts at rho*q0)
+//   s<3: q = (rho*q0)/rho + c_s (d/rho),  c_s = (int(s/2)+1)/2 = 1/2, 1/2, 1
+//   s=3: q = acc/rho
+// (app/shearLayerWC/UEqn.H:11-41, TEqn.H:91-117; for rho itself, rhoEqn.H:53-78,
+// q = rhoOld + c_s d and acc/1).  The T loop does that.  In the U and rho loops
+// the sums divide through by rho and the stage states carry the increments, so
+// that no accumulator is kept:
 //   d = dt * RHS(stage state) / rho   (rho loop: dt * RHS)
 //   Y1 = q0 + d/2, Y2 = q0 + d/2, Y3 = q0 + d,
 //   q  = q0 + [(Y1 - q0) + 2 (Y2 - q0) + (Y3 - q0)]/3 + d/6
 // 256^3, stages 0-3, with an accumulator and term-by-term advection -> now:
-// U 551, 638, 631, 562 -> 495, 533, 532, 615 us, rho 246, 271, 272, 259 -> 228, 242,
-// 242, 282 us, T 298, 322, 321, 300 -> 296, 305, 303, 373 us; the last stage reads
-// Y1 and Y2 where it read one sum, the others no longer read and write it.
-// The U and rho loops unroll by the queue period: U -> 477, 518, 515, 622, rho ->
-// 224, 237, 237, 281 (96 x 75 x 90: U 28.1, 30.0, 30.1, 33.9 -> 27.4, 29.0, 29.3,
+// U 551, 639, 633, 562 -> 485, 525, 525, 629 us, rho 246, 271, 271, 260 -> 228, 241,
+// 241, 285 us: the last stage reads Y1 and Y2 where it read one sum, the others
+// no longer read and write it.  The T loop loses that way: 298, 322, 321, 300 ->
+// 295, 304, 303, 378 us (loaded ahead, its Y1 and Y2 spill, 582 us).
+// The U and rho loops unroll by the queue period: U 495, 533, 532, 615, rho 228, 242,
+// 242, 282 us rolled (96 x 75 x 90: U 28.1, 30.0, 30.1, 33.9 -> 27.4, 29.0, 29.3,
 // 31.9); the T loop spills.
 //   U:   RHS = -div(rho U, U) - grad p + laplacian(mu, U) [- (rho T) g]
 //   rho: RHS = -div(rho U)
@@ -33,6 +40,9 @@ namespace nova {
 namespace {
 
 constexpr int kH = 3;
+
+__device__ __forceinline__ double rk4w(int s) { return s == 0 || s == 3 ? 1.0 / 6.0 : 1.0 / 3.0; }
+__device__ __forceinline__ double stage_c(int s) { return (double)(int(s / 2) + 1) / 2.0; }
 
 struct ZMetric {
     double iak, az[kH], bz[kH], bsum, c2k;
@@ -206,16 +216,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_wc_t(Geo g, Coef<double> co, co
     auto ld = [&](int c, long long o) -> double {
         return c == 0 ? a.Y[o] : (c == 1 ? a.rho[o] : a.U[(long long)(c - 2) * g.N3 + o]);
     };
-    // the next plane's base loads ahead; Y1 and Y2 (last stage) at the start of the
-    // plane (ahead they spill: 582 us at 256^3)
-    double q0n = 0.0, q0c = 0.0;
+    double q0n = 0.0, accn = 0.0, q0c = 0.0, accc = 0.0;  // next plane's base and accumulator, loading ahead
     auto pre = [&](long long nidx, bool load) {
         q0c = q0n;
-        if (STAGE > 0 && load) q0n = a.Q0[nidx];
+        accc = accn;
+        if (STAGE > 0 && load) {
+            q0n = a.Q0[nidx];
+            accn = a.acc[nidx];
+        }
     };
     tile_march<double, kH, 5, false>(g, wl, sm, ld, ib, ie, pre, [&](long long idx, auto &q, const auto &vx,
                                                                     const auto &vy, const auto &vz) {
-        const double y1 = STAGE == 3 ? a.Y1[idx] : 0.0, y2 = STAGE == 3 ? a.Y2[idx] : 0.0;
         const double t0 = q[kH][0], r0 = q[kH][1];
         const double V0[3] = {r0 * q[kH][2], r0 * q[kH][3], r0 * q[kH][4]};
         // (term by term: one component does not pay for the shared weights' registers)
@@ -231,7 +242,16 @@ __global__ void __launch_bounds__(kThreads, 2) k_wc_t(Geo g, Coef<double> co, co
         dir(vy, 1, co.a[1], co.b[1], false);
         dir(vz, 2, zm.az, zm.bz, true);
         const double e = -(0.5 * fma(t0, divV, adv)) + a.visc * (fma(-zm.bsum, t0, lap) - zm.c2k * duz);
-        a.Ynext[idx] = wc_rk<STAGE>(t0, q0c, y1, y2, (a.dt / r0) * e);
+        const double d = a.dt * e;
+        const double q0 = STAGE == 0 ? t0 : q0c;
+        const double acc = (STAGE == 0 ? r0 * q0 : accc) + rk4w(STAGE) * d;
+        const double ir = 1.0 / r0;  // the divisions by rho below as products (within an ulp)
+        if (STAGE < 3) {
+            a.acc[idx] = acc;
+            a.Ynext[idx] = (r0 * q0) * ir + stage_c(STAGE) * (d * ir);
+        } else {
+            a.Ynext[idx] = acc * ir;
+        }
     });
 }
 

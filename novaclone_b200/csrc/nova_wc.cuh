@@ -14,7 +14,8 @@ struct WcArgs {
     const double *rho;  // rho, frozen during the U and T loops
     const double *T;    // T of the buoyancy term (U loop, shear case)
     const double *Q0;   // the loop's value at the start of the step (stages 1-3)
-    const double *Y1, *Y2;  // the states after stages 0 and 1 (stage 3)
+    const double *Y1, *Y2;  // U and rho loops: the states after stages 0 and 1 (stage 3)
+    double *acc;            // T loop: the RK accumulator of rho T
     double *Ynext;      // next stage state, or the updated field after stage 3
     double *p;          // read (halo'd) by the U loop, written from the EOS by the last rho stage
     double dt, visc, eos_k;
