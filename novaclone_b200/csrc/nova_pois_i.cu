@@ -48,21 +48,32 @@ __global__ void __launch_bounds__(column_threads<R1, R2>(), column_blocks<R1, R2
     double2 *S = tw + N;                               // transpose buffer [R1][R2][kSpecCols]
     const int tid = threadIdx.x;
     const int col = tid % kSpecCols, t = tid / kSpecCols;
-    const long long c = blockIdx.x * (long long)kSpecCols + col;  // column j nzh + kz
+    // column j nzh + kz in 32 bits (2^31 columns of 16 or more nodes exceed any
+    // memory): the two 64-bit divisions cost 2 us at 256 x 256 x 250
+    const unsigned c = blockIdx.x * kSpecCols + col;
     const bool valid = c < ncol;
     double2 *p = spec + (valid ? c : 0);  // element i at p[i ncol]
+    // one address and two strides (as products per element the addresses spilled: 98
+    // -> 89 us at 256 x 250 x 256, 240 x 250 x 260 91 -> 80, 75 x 77 x 79 8.1 -> 8.3)
+    p += t * ncol;
+    const long long step = R2 * ncol, ustep = T * ncol;
     double2 v[U][R1], w[R2];
 #pragma unroll
     for (int u = 0; u < U; u++)
 #pragma unroll
-        for (int n1 = 0; n1 < R1; n1++) v[u][n1] = valid ? p[(R2 * n1 + t + T * u) * ncol] : make_double2(0.0, 0.0);
-    const double kyz = ky2[valid ? c / nzh : 0], kzz = kz2[valid ? c % nzh : 0];
+        for (int n1 = 0; n1 < R1; n1++) v[u][n1] = valid ? p[n1 * step + u * ustep] : make_double2(0.0, 0.0);
     for (int m = tid; m < N; m += column_threads<R1, R2>()) tw[m] = twN[m];
     __syncthreads();
     column_fft<R1, R2, false>(v, w, S, tw, t, col);
+    // S is rewritten below: for R1 = R2 every thread holds its values by now, and the
+    // barrier here keeps the scale's operands out of the registers of the forward
+    // step (256 x 250 x 256 88.6 -> 83.9 us, 64 x 64 x 62 5.1 -> 4.9); else it waits for
+    // threads without a second step (240 x 250 x 260 79.8 us, here 104)
+    if (R1 == R2) __syncthreads();
     // scale: -1 / k'^2 / (N0 N1 N2), 0 where k'^2 < 1e-16 (k'^2 summed in
     // k_scale's order; one reciprocal per element instead of two divisions)
     if (T == R1 || t < R1) {
+        const double kyz = ky2[valid ? c / (unsigned)nzh : 0u], kzz = kz2[valid ? c % (unsigned)nzh : 0u];
 #pragma unroll
         for (int k2 = 0; k2 < R2; k2++) {
             const double k2v = (kx2[t + R1 * k2] + kyz) + kzz;
@@ -72,7 +83,7 @@ __global__ void __launch_bounds__(column_threads<R1, R2>(), column_blocks<R1, R2
         // inverse, step 1 (thread = k1 = t): DFT over k2, twiddle W_N^-(n2 t)
         dft<R2, N, true>(w, tw);
     }
-    __syncthreads();  // S is rewritten
+    if (R1 != R2) __syncthreads();
     if (T == R1 || t < R1)
 #pragma unroll
         for (int n2 = 0; n2 < R2; n2++)
@@ -87,7 +98,7 @@ __global__ void __launch_bounds__(column_threads<R1, R2>(), column_blocks<R1, R2
         dft<R1, N, true>(v[u], tw);
         if (valid)
 #pragma unroll
-            for (int n1 = 0; n1 < R1; n1++) p[(n2 + R2 * n1) * ncol] = v[u][n1];
+            for (int n1 = 0; n1 < R1; n1++) p[n1 * step + u * ustep] = v[u][n1];
     }
 }
 
