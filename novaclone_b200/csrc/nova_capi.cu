@@ -432,7 +432,7 @@ nova_status ensure_fft(nova_ctx *ctx, bool split)
 nova_status ensure_red(nova_ctx *ctx)
 {
     nova_status s;
-    if ((s = dalloc(ctx, &ctx->d_part, (size_t)diag_blocks(ctx->g) * kDiagParts)) != NOVA_OK) return s;
+    if (!ctx->d_part && (s = dalloc(ctx, &ctx->d_part, (size_t)diag_blocks(ctx->g) * kDiagParts)) != NOVA_OK) return s;
     if ((s = dalloc(ctx, &ctx->d_scalar, 1)) != NOVA_OK) return s;
     // [0] non-finite diagnostics, [1] a stage pipeline wait timed out
     if ((s = dalloc(ctx, &ctx->d_flag, 2)) != NOVA_OK) return s;

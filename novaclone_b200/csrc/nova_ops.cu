@@ -530,9 +530,12 @@ static int diag_chunk(const Geo &g, int nf)
     return march_chunk(g.N0, tiles, 2, 3.0, g.wallY ? 0.45 : 0.15);
 }
 
+// full occupancy of blocks of 256 threads: the least number of partials kept
+constexpr int kMinBlocks = 148 * 8;
+
 int diag_blocks(const Geo &g)
 {
-    long long most = 1184;
+    long long most = kMinBlocks;
     for (int nf = 1; nf <= 2; nf++) {
         const dim3 gr = tile_grid(g, diag_chunk(g, nf));
         const long long nb = (long long)nf * gr.x * gr.y * gr.z;
@@ -608,9 +611,8 @@ void launch_diag_final(const double *part, int nb, const DiagFinal &fin, double 
 
 void launch_maxabs(const Geo &g, const double *s, double *part, double *out, cudaStream_t st)
 {
-    const int nb = diag_blocks(g);
-    k_maxabs_part<<<nb, 256, 0, st>>>(g.N3, Ld64{s, g.N3}, part);
-    k_max_final<<<1, 256, 0, st>>>(part, nb, out);
+    k_maxabs_part<<<kMinBlocks, 256, 0, st>>>(g.N3, Ld64{s, g.N3}, part);
+    k_max_final<<<1, 256, 0, st>>>(part, kMinBlocks, out);
 }
 
 // The allocation-free reduction's scratch: kMaxabsStaticParts partials, then
