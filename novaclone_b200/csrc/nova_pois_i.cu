@@ -34,6 +34,12 @@
 
 namespace nova {
 
+// N0 of group G: false where N0 is none of its lengths
+template <int G>
+bool pois_group(const Geo &g, int ny, void *spec, const double *twN, const double *kx2, const double *ky2,
+                const double *kz2, double invN3, cudaStream_t st);
+
+#ifdef NOVA_FFT_GROUP
 namespace {
 
 template <int R1, int R2>
@@ -113,6 +119,26 @@ void launch_r(const Geo &g, int ny, void *spec, const double *twN, const double 
     k_pois_i<R1, R2><<<(unsigned)((ncol + kSpecCols - 1) / kSpecCols), column_threads<R1, R2>(), smem, st>>>(
         nzh, ncol, (double2 *)spec, (const double2 *)twN, kx2, ky2, kz2, invN3);
 }
+
+}  // namespace
+
+template <int G>
+bool pois_group(const Geo &g, int ny, void *spec, const double *twN, const double *kx2, const double *ky2,
+                const double *kz2, double invN3, cudaStream_t st)
+{
+    switch (g.N0) {
+#define NOVA_X(l, r1, r2) \
+    case l: launch_r<r1, r2>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st); return true;
+        NOVA_FFT_GROUP(NOVA_X)
+#undef NOVA_X
+    default: return false;
+    }
+}
+
+template bool pois_group<NOVA_PART>(const Geo &, int, void *, const double *, const double *, const double *,
+                                    const double *, double, cudaStream_t);
+#else
+namespace {
 
 // ---- N0 = 256 on a TMA-fed, double-buffered tile ----
 constexpr int kTR = 16, kTN = kTR * kTR;  // 256 = 16 x 16
@@ -280,13 +306,13 @@ void launch_pois_i(const Geo &g, int ny, void *spec, const double *twN, const do
     if (g.N0 == 256 && err && pois_tma_fits(g, ny) &&
         launch_pois_tma(g, ny, spec, twN, kx2, ky2, kz2, invN3, err, st))
         return;
-    switch (g.N0) {
-#define NOVA_X(l, r1, r2) \
-    case l: launch_r<r1, r2>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st); break;
-        NOVA_FFT_LENGTHS(NOVA_X)
-#undef NOVA_X
-    default: break;
-    }
+    (void)(pois_group<0>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st) ||
+           pois_group<1>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st) ||
+           pois_group<2>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st) ||
+           pois_group<3>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st) ||
+           pois_group<4>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st) ||
+           pois_group<5>(g, ny, spec, twN, kx2, ky2, kz2, invN3, st));
 }
+#endif
 
 }  // namespace nova

@@ -17,6 +17,7 @@
 // past N1 - 1 store nothing.
 // Every mbarrier wait is bounded (nova_tma.cuh).
 #include "nova_internal.cuh"
+#include "nova_parts.h"
 #include "nova_tma.cuh"
 
 #include <cudaTypedefs.h>
@@ -39,6 +40,8 @@ constexpr int kRowsE = (TJ + 2 * kH) * kTK;  // a component's rows with the j ha
 constexpr int kTileE = TJ * kTK;             // a component's tile rows
 constexpr int kLRE = TJ * 4;                 // one side's k halo of a component
 
+}  // namespace
+
 // PROJ_CORR_MIX: the correction of an FP32-split state whose U* arrives in FP64
 enum ProjMode { PROJ_DIV = 0, PROJ_CORR = 1, PROJ_CORR_MIX = 2 };
 
@@ -59,6 +62,23 @@ struct ProjMaps {
     CUtensorMap m[16];
 };
 
+struct ProjArgs {
+    double divisor, s;
+    double *rhs;                // DIV output
+    double *U64;                // CORR output (FP64)
+    float *hi, *lo;             // CORR output (split)
+};
+
+// the kernels of one mode, precision and mesh kind: a part of this source
+template <int MODE, bool SPLIT, bool WALLS> struct ProjPart {
+    static cudaError_t launch(const Geo &g, const Coef<double> &co, const Walls<double> &wl, const double *ia,
+                              const ProjArgs &a, const ProjMaps &pm, int *err, cudaStream_t st);
+};
+constexpr int kProjParts = 10;  // (DIV, DIV split, CORR, CORR split, CORR_MIX) x walls
+
+#if NOVA_PART < 10
+namespace {
+
 template <int MODE, bool SPLIT> struct ProjCfg {
     static constexpr bool kDivLoads = MODE == PROJ_DIV;
     using TS = typename std::conditional<kDivLoads && SPLIT, float, double>::type;  // stencil element
@@ -73,13 +93,6 @@ template <int MODE, bool SPLIT> struct ProjCfg {
     static constexpr uint32_t kEpiBytes = kEpiE * sizeof(TE);
     static constexpr size_t kSmem =
         (size_t)kRing * kSlotBytes + (size_t)kERing * kNE * kEpiBytes + 8 * 2 * (kRing + kERing) + 16 * kWarps;
-};
-
-struct ProjArgs {
-    double divisor, s;
-    double *rhs;                // DIV output
-    double *U64;                // CORR output (FP64)
-    float *hi, *lo;             // CORR output (split)
 };
 
 template <int MODE, bool SPLIT, bool WALLS, bool WHOLE>
@@ -337,6 +350,45 @@ __global__ void __launch_bounds__(kThreads, 2)
 }
 
 // ------------------------------------------------------------------ host --
+// i-chunk.  The 2H warm-up planes of a chunk load the queue's tile rows alone;
+// the correction streams twice the bytes of the divergence per plane and its
+// last blocks are later (256^3: 24 planes 147 us, 64 planes 152 us; 192 x 192 x
+// 384: 20 planes 129 us, 96 planes 140 us)
+int proj_ichunk(const Geo &g, double tail)
+{
+    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + TJ - 1) / TJ);
+    return march_chunk(g.N0, tiles, 2, 2.5, g.wallY ? 0.45 : tail);
+}
+
+}  // namespace
+
+template <int MODE, bool SPLIT, bool WALLS>
+cudaError_t ProjPart<MODE, SPLIT, WALLS>::launch(const Geo &g, const Coef<double> &co, const Walls<double> &wl,
+                                                 const double *ia, const ProjArgs &a, const ProjMaps &pm, int *err,
+                                                 cudaStream_t st)
+{
+    using C = ProjCfg<MODE, SPLIT>;
+    // the whole-tile form for the corrections alone (split 192 x 192 x 384: 131 us
+    // against 133); in the divergence it spills (256^3: 107 us against 94)
+    constexpr bool kWhole = MODE != PROJ_DIV && !WALLS;
+    const bool whole = kWhole && g.N2 % kTK == 0 && g.N1 % TJ == 0;
+    auto kern = whole ? k_proj_tma<MODE, SPLIT, WALLS, kWhole> : k_proj_tma<MODE, SPLIT, WALLS, false>;
+    static bool attr[2] = {false, false};
+    if (!attr[whole]) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
+        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        attr[whole] = true;
+    }
+    const int ch = proj_ichunk(g, MODE == PROJ_DIV ? 0.15 : 0.3);
+    const dim3 grid((g.N2 + kTK - 1) / kTK, (g.N1 + TJ - 1) / TJ, (g.N0 + ch - 1) / ch);
+    kern<<<grid, dim3(kTK, TJ + 1), C::kSmem, st>>>(g, co, wl, ia, a, pm, ch, err);
+    return cudaSuccess;
+}
+
+template struct ProjPart<NOVA_PART / 4, (NOVA_PART / 2 % 2 != 0 || NOVA_PART / 4 == PROJ_CORR_MIX), NOVA_PART % 2 != 0>;
+#else
+namespace {
+
 using EncodeFn = PFN_cuTensorMapEncodeTiled_v12000;
 
 EncodeFn encode_fn()
@@ -388,44 +440,12 @@ template <typename T> bool encode_rows(ProjMaps &pm, int ms, const T *f, const G
            encode3(&pm.m[ms + M_RR], f, g, kTK, (g.N1 - 1) % TJ + 1 + kH);
 }
 
-// i-chunk.  The 2H warm-up planes of a chunk load the queue's tile rows alone;
-// the correction streams twice the bytes of the divergence per plane and its
-// last blocks are later (256^3: 24 planes 147 us, 64 planes 152 us; 192 x 192 x
-// 384: 20 planes 129 us, 96 planes 140 us)
-int proj_ichunk(const Geo &g, double tail)
-{
-    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + TJ - 1) / TJ);
-    return march_chunk(g.N0, tiles, 2, 2.5, g.wallY ? 0.45 : tail);
-}
-
-template <int MODE, bool SPLIT, bool WALLS>
-cudaError_t launch_w(const Geo &g, const Coef<double> &co, const Walls<double> &wl, const double *ia,
-                     const ProjArgs &a, const ProjMaps &pm, int *err, cudaStream_t st)
-{
-    using C = ProjCfg<MODE, SPLIT>;
-    // the whole-tile form for the corrections alone (split 192 x 192 x 384: 131 us
-    // against 133); in the divergence it spills (256^3: 107 us against 94)
-    constexpr bool kWhole = MODE != PROJ_DIV && !WALLS;
-    const bool whole = kWhole && g.N2 % kTK == 0 && g.N1 % TJ == 0;
-    auto kern = whole ? k_proj_tma<MODE, SPLIT, WALLS, kWhole> : k_proj_tma<MODE, SPLIT, WALLS, false>;
-    static bool attr[2] = {false, false};
-    if (!attr[whole]) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        attr[whole] = true;
-    }
-    const int ch = proj_ichunk(g, MODE == PROJ_DIV ? 0.15 : 0.3);
-    const dim3 grid((g.N2 + kTK - 1) / kTK, (g.N1 + TJ - 1) / TJ, (g.N0 + ch - 1) / ch);
-    kern<<<grid, dim3(kTK, TJ + 1), C::kSmem, st>>>(g, co, wl, ia, a, pm, ch, err);
-    return cudaSuccess;
-}
-
 template <int MODE, bool SPLIT>
 cudaError_t launch(const Geo &g, const Coef<double> &co, const Walls<double> &wl, const double *ia,
                    const ProjArgs &a, const ProjMaps &pm, int *err, cudaStream_t st)
 {
-    return wl.on ? launch_w<MODE, SPLIT, true>(g, co, wl, ia, a, pm, err, st)
-                 : launch_w<MODE, SPLIT, false>(g, co, wl, ia, a, pm, err, st);
+    return wl.on ? ProjPart<MODE, SPLIT, true>::launch(g, co, wl, ia, a, pm, err, st)
+                 : ProjPart<MODE, SPLIT, false>::launch(g, co, wl, ia, a, pm, err, st);
 }
 
 }  // namespace
@@ -486,5 +506,6 @@ cudaError_t launch_correct_tma(const Geo &g, const Coef<double> &co, const Walls
     if (!ok) return cudaErrorInvalidValue;
     return launch<PROJ_CORR, true>(g, co, pw, ia, a, pm, err, st);
 }
+#endif
 
 }  // namespace nova

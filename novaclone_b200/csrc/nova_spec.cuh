@@ -9,16 +9,37 @@
 
 #include "nova_fft.cuh"
 #include "nova_internal.cuh"
+#include "nova_parts.h"
 
 namespace nova {
 
-// (L, R1, R2), R1 <= R2
-#define NOVA_FFT_LENGTHS(X)                                                                             \
-    X(16, 4, 4) X(20, 4, 5) X(24, 4, 6) X(25, 5, 5) X(30, 5, 6) X(32, 4, 8) X(36, 6, 6) X(40, 4, 10)    \
-    X(45, 5, 9) X(48, 6, 8) X(50, 5, 10) X(54, 6, 9) X(60, 6, 10) X(64, 8, 8) X(72, 6, 12) X(75, 5, 15) \
-    X(80, 8, 10) X(90, 9, 10) X(96, 8, 12) X(100, 10, 10) X(108, 9, 12) X(120, 10, 12) X(128, 8, 16)    \
-    X(144, 12, 12) X(150, 10, 15) X(160, 10, 16) X(180, 12, 15) X(192, 12, 16) X(240, 15, 16)           \
-    X(256, 16, 16)
+// (L, R1, R2), R1 <= R2: the composites of the register DFTs that a mesh extent is
+// likely to be; 81, 135 and 225 are left to cuFFT.  Along k L is N2 / 2, so that rows
+// of 32 to 512 reals are covered; along i and j the extent itself, 16 to 256.
+// In six groups: a part of nova_spec_row.cu, nova_spec_col.cu and nova_pois_i.cu each.
+#define NOVA_FFT_G0(X) X(16, 4, 4) X(20, 4, 5) X(24, 4, 6) X(25, 5, 5) X(30, 5, 6)
+#define NOVA_FFT_G1(X) X(32, 4, 8) X(36, 6, 6) X(40, 4, 10) X(45, 5, 9) X(48, 6, 8)
+#define NOVA_FFT_G2(X) X(50, 5, 10) X(54, 6, 9) X(60, 6, 10) X(64, 8, 8) X(72, 6, 12)
+#define NOVA_FFT_G3(X) X(75, 5, 15) X(80, 8, 10) X(90, 9, 10) X(96, 8, 12) X(100, 10, 10)
+#define NOVA_FFT_G4(X) X(108, 9, 12) X(120, 10, 12) X(128, 8, 16) X(144, 12, 12) X(150, 10, 15)
+#define NOVA_FFT_G5(X) X(160, 10, 16) X(180, 12, 15) X(192, 12, 16) X(240, 15, 16) X(256, 16, 16)
+#define NOVA_FFT_LENGTHS(X) \
+    NOVA_FFT_G0(X) NOVA_FFT_G1(X) NOVA_FFT_G2(X) NOVA_FFT_G3(X) NOVA_FFT_G4(X) NOVA_FFT_G5(X)
+
+// the group of this part (the dispatch, part 6, has none)
+#if NOVA_PART == 0
+#define NOVA_FFT_GROUP NOVA_FFT_G0
+#elif NOVA_PART == 1
+#define NOVA_FFT_GROUP NOVA_FFT_G1
+#elif NOVA_PART == 2
+#define NOVA_FFT_GROUP NOVA_FFT_G2
+#elif NOVA_PART == 3
+#define NOVA_FFT_GROUP NOVA_FFT_G3
+#elif NOVA_PART == 4
+#define NOVA_FFT_GROUP NOVA_FFT_G4
+#elif NOVA_PART == 5
+#define NOVA_FFT_GROUP NOVA_FFT_G5
+#endif
 
 inline bool fft_length(int L)
 {

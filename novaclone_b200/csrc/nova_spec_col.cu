@@ -8,6 +8,10 @@
 
 namespace nova {
 
+// the lengths of group G: false where L is none of them
+template <int G> bool cols_group(int L, const Columns &C, bool inv, double2 *spec, const double2 *tw, cudaStream_t st);
+
+#ifdef NOVA_FFT_GROUP
 namespace {
 
 template <int R1, int R2, bool INV>
@@ -47,15 +51,30 @@ template <int R1, int R2> void col(const Columns &C, bool inv, double2 *spec, co
     }
 }
 
-void cols_any(int L, const Columns &C, bool inv, void *spec, const double *tw, cudaStream_t st)
+}  // namespace
+
+template <int G> bool cols_group(int L, const Columns &C, bool inv, double2 *spec, const double2 *tw, cudaStream_t st)
 {
     switch (L) {
-#define NOVA_X(l, r1, r2)                                                                            \
-    case l: col<r1, r2>(C, inv, (double2 *)spec, reinterpret_cast<const double2 *>(tw), st); break;
-        NOVA_FFT_LENGTHS(NOVA_X)
+#define NOVA_X(l, r1, r2) \
+    case l: col<r1, r2>(C, inv, spec, tw, st); return true;
+        NOVA_FFT_GROUP(NOVA_X)
 #undef NOVA_X
-    default: break;
+    default: return false;
     }
+}
+
+template bool cols_group<NOVA_PART>(int, const Columns &, bool, double2 *, const double2 *, cudaStream_t);
+#else
+namespace {
+
+void cols_any(int L, const Columns &C, bool inv, void *spec, const double *tw, cudaStream_t st)
+{
+    double2 *s = (double2 *)spec;
+    const double2 *w = reinterpret_cast<const double2 *>(tw);
+    (void)(cols_group<0>(L, C, inv, s, w, st) || cols_group<1>(L, C, inv, s, w, st) ||
+           cols_group<2>(L, C, inv, s, w, st) || cols_group<3>(L, C, inv, s, w, st) ||
+           cols_group<4>(L, C, inv, s, w, st) || cols_group<5>(L, C, inv, s, w, st));
 }
 
 }  // namespace
@@ -71,5 +90,6 @@ void launch_cols_i(int n0, long long per_plane, bool inv, void *spec, const doub
 {
     cols_any(n0, Columns{per_plane, 0, per_plane, (int)per_plane}, inv, spec, twL, st);
 }
+#endif
 
 }  // namespace nova

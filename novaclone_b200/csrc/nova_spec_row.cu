@@ -17,13 +17,19 @@
 
 namespace nova {
 
-namespace {
-
 // rows r = 0..rows-1: real row (r / ny) plane + (r % ny) N2, spectrum row r (m + 1)
 struct Rows {
     long long rows, plane;
     int ny;
 };
+
+// the half lengths m = N2 / 2 of group G: false where m is none of them
+template <int G>
+bool rows_group(int m, const Rows &R, bool inv, const double *x, double2 *spec, double *p, const double2 *tw,
+                cudaStream_t st);
+
+#ifdef NOVA_FFT_GROUP
+namespace {
 
 template <int R1, int R2> struct RowCfg {
     static constexpr int m = R1 * R2, T = Line<R1, R2>::T, U = Line<R1, R2>::U;
@@ -158,18 +164,35 @@ void row(const Rows &R, bool inv, const double *x, double2 *spec, double *p, con
     }
 }
 
+}  // namespace
+
+template <int G>
+bool rows_group(int m, const Rows &R, bool inv, const double *x, double2 *spec, double *p, const double2 *tw,
+                cudaStream_t st)
+{
+    switch (m) {
+#define NOVA_X(l, r1, r2) \
+    case l: row<r1, r2>(R, inv, x, spec, p, tw, st); return true;
+        NOVA_FFT_GROUP(NOVA_X)
+#undef NOVA_X
+    default: return false;
+    }
+}
+
+template bool rows_group<NOVA_PART>(int, const Rows &, bool, const double *, double2 *, double *, const double2 *,
+                                    cudaStream_t);
+#else
+namespace {
+
 void rows_any(const Rows &R, int n2, bool inv, const double *x, void *spec, double *p, const double *tw,
               cudaStream_t st)
 {
-    switch (n2 / 2) {
-#define NOVA_X(l, r1, r2)                                                                        \
-    case l:                                                                                      \
-        row<r1, r2>(R, inv, x, (double2 *)spec, p, reinterpret_cast<const double2 *>(tw), st);   \
-        break;
-        NOVA_FFT_LENGTHS(NOVA_X)
-#undef NOVA_X
-    default: break;
-    }
+    const int m = n2 / 2;
+    double2 *s = (double2 *)spec;
+    const double2 *w = reinterpret_cast<const double2 *>(tw);
+    (void)(rows_group<0>(m, R, inv, x, s, p, w, st) || rows_group<1>(m, R, inv, x, s, p, w, st) ||
+           rows_group<2>(m, R, inv, x, s, p, w, st) || rows_group<3>(m, R, inv, x, s, p, w, st) ||
+           rows_group<4>(m, R, inv, x, s, p, w, st) || rows_group<5>(m, R, inv, x, s, p, w, st));
 }
 
 }  // namespace
@@ -187,5 +210,6 @@ void launch_rows_inv(int planes, int ny, long long plane, int n2, const void *sp
 {
     rows_any(Rows{(long long)planes * ny, plane, ny}, n2, true, nullptr, const_cast<void *>(spec), x, twN, st);
 }
+#endif
 
 }  // namespace nova

@@ -18,6 +18,7 @@
 // ring; one block per SM, 8 consumer warps of 232 registers); FP32:
 // TJ = 16 (20 KB slots, 195 KB; one block of 17 warps).
 #include "nova_internal.cuh"
+#include "nova_parts.h"
 #include "nova_stage_math.cuh"
 #include "nova_tma.cuh"
 
@@ -51,6 +52,19 @@ template <typename T> struct MhdCfg {
     static constexpr int kEpiE = TJ * kRowE;
     static_assert(TJ % kLRB == 0 && kLRB * 4 == kTK, "k-halo boxes share the component stride of the row boxes");
 };
+
+}  // namespace
+
+// the kernels of one precision and mesh kind: a part of this source.  WHOLE: the
+// mesh has no ragged tile
+template <typename T, bool STRETCH, bool WHOLE> struct MhdPart {
+    using Args = std::conditional_t<sizeof(T) == 8, StageArgs64, StageArgs32>;
+    static cudaError_t launch(int phys, int stage, const Geo &g, const Coef<T> &co, const T *ia, const T *corr2, T dt,
+                              T visc, const Args &a, const T *const *ef, int *err, cudaStream_t st);
+};
+
+#if NOVA_PART < 8
+namespace {
 
 // epilogue operands per stage, in load order (as nova_stage_tma.cu):
 //   FP64:  s=1,2: U0   s=3: U0, Y1, Y2
@@ -361,7 +375,7 @@ template <typename T> int mhd_ichunk(const Geo &g)
     return march_chunk(g.N0, tiles, 1, 2.5);
 }
 
-template <typename T, int PHYS, int STAGE, bool STRETCH, class Args>
+template <typename T, int PHYS, int STAGE, bool STRETCH, class Args, bool WHOLE>
 cudaError_t launch_mhd(const Geo &g, const Coef<T> &co, const T *ia, const T *corr2, T dt, T visc, const Args &a,
                        const T *Y, const T *X, const T *const *ef, int *err, cudaStream_t st)
 {
@@ -378,14 +392,13 @@ cudaError_t launch_mhd(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     for (int f = 0; f < NE; f++) ok = ok && encode(&maps.e[f], ef[f], g, Cf::TJ);
     if (!ok) return cudaErrorInvalidValue;
     constexpr size_t smem = mhd_smem_bytes<T, NE>();
-    const bool whole = g.N2 % kTK == 0 && g.N1 % Cf::TJ == 0;
-    auto kern = whole ? k_mhd_tma<T, PHYS, STAGE, STRETCH, Args, true> : k_mhd_tma<T, PHYS, STAGE, STRETCH, Args, false>;
-    static bool attr[2] = {false, false};
-    if (!attr[whole]) {
+    auto kern = k_mhd_tma<T, PHYS, STAGE, STRETCH, Args, WHOLE>;
+    static bool attr = false;
+    if (!attr) {
         if (const cudaError_t e = reg_split_ok(typename Cf::Split{}, kern); e != cudaSuccess) return e;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        attr[whole] = true;
+        attr = true;
     }
     const int ch = mhd_ichunk<T>(g);
     const dim3 grid((g.N2 + kTK - 1) / kTK, (g.N1 + Cf::TJ - 1) / Cf::TJ, (g.N0 + ch - 1) / ch);
@@ -393,29 +406,43 @@ cudaError_t launch_mhd(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     return cudaSuccess;
 }
 
-template <typename T, int PHYS, bool STRETCH, class Args>
+template <typename T, int PHYS, bool STRETCH, bool WHOLE, class Args>
 cudaError_t launch_mhd_stage(int stage, const Geo &g, const Coef<T> &co, const T *ia, const T *corr2, T dt, T visc,
-                             const Args &a, const T *X, const T *const *ef, int *err, cudaStream_t st)
+                             const Args &a, const T *const *ef, int *err, cudaStream_t st)
 {
     switch (stage) {
-    case 0: return launch_mhd<T, PHYS, 0, STRETCH>(g, co, ia, corr2, dt, visc, a, a.Y, X, ef, err, st);
-    case 1: return launch_mhd<T, PHYS, 1, STRETCH>(g, co, ia, corr2, dt, visc, a, a.Y, X, ef, err, st);
-    case 2: return launch_mhd<T, PHYS, 2, STRETCH>(g, co, ia, corr2, dt, visc, a, a.Y, X, ef, err, st);
-    case 3: return launch_mhd<T, PHYS, 3, STRETCH>(g, co, ia, corr2, dt, visc, a, a.Y, X, ef, err, st);
-    default: return launch_mhd<T, PHYS, 4, STRETCH>(g, co, ia, corr2, dt, visc, a, a.Y, X, ef, err, st);
+    case 0: return launch_mhd<T, PHYS, 0, STRETCH, Args, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, a.X, ef, err, st);
+    case 1: return launch_mhd<T, PHYS, 1, STRETCH, Args, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, a.X, ef, err, st);
+    case 2: return launch_mhd<T, PHYS, 2, STRETCH, Args, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, a.X, ef, err, st);
+    case 3: return launch_mhd<T, PHYS, 3, STRETCH, Args, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, a.X, ef, err, st);
+    default: return launch_mhd<T, PHYS, 4, STRETCH, Args, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, a.X, ef, err, st);
     }
 }
 
+}  // namespace
+
+template <typename T, bool STRETCH, bool WHOLE>
+cudaError_t MhdPart<T, STRETCH, WHOLE>::launch(int phys, int stage, const Geo &g, const Coef<T> &co, const T *ia,
+                                               const T *corr2, T dt, T visc, const Args &a, const T *const *ef,
+                                               int *err, cudaStream_t st)
+{
+    return phys == PHYS_MHD_U
+               ? launch_mhd_stage<T, PHYS_MHD_U, STRETCH, WHOLE>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st)
+               : launch_mhd_stage<T, PHYS_MHD_B, STRETCH, WHOLE>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st);
+}
+
+template struct MhdPart<std::conditional_t<NOVA_PART / 4 == 0, double, float>, NOVA_PART / 2 % 2 != 0, NOVA_PART % 2 != 0>;
+#else
+namespace {
+
 template <typename T, class Args>
 cudaError_t launch_mhd_any(int phys, int stage, bool stretch, const Geo &g, const Coef<T> &co, const T *ia,
-                           const T *corr2, T dt, T visc, const Args &a, const T *X, const T *const *ef, int *err,
-                           cudaStream_t st)
+                           const T *corr2, T dt, T visc, const Args &a, const T *const *ef, int *err, cudaStream_t st)
 {
-    if (phys == PHYS_MHD_U)
-        return stretch ? launch_mhd_stage<T, PHYS_MHD_U, true>(stage, g, co, ia, corr2, dt, visc, a, X, ef, err, st)
-                       : launch_mhd_stage<T, PHYS_MHD_U, false>(stage, g, co, ia, corr2, dt, visc, a, X, ef, err, st);
-    return stretch ? launch_mhd_stage<T, PHYS_MHD_B, true>(stage, g, co, ia, corr2, dt, visc, a, X, ef, err, st)
-                   : launch_mhd_stage<T, PHYS_MHD_B, false>(stage, g, co, ia, corr2, dt, visc, a, X, ef, err, st);
+    const bool whole = g.N2 % kTK == 0 && g.N1 % MhdCfg<T>::TJ == 0;
+    const auto f = stretch ? (whole ? MhdPart<T, true, true>::launch : MhdPart<T, true, false>::launch)
+                           : (whole ? MhdPart<T, false, true>::launch : MhdPart<T, false, false>::launch);
+    return f(phys, stage, g, co, ia, corr2, dt, visc, a, ef, err, st);
 }
 
 }  // namespace
@@ -435,7 +462,7 @@ cudaError_t launch_mhd_tma64(int phys, int stage, bool stretch, const Geo &g, co
         ef[1] = a.Y1;
         ef[2] = a.Y2;
     }
-    return launch_mhd_any<double>(phys, stage, stretch, g, co, ia, corr2, dt, visc, a, a.X, ef, err, st);
+    return launch_mhd_any<double>(phys, stage, stretch, g, co, ia, corr2, dt, visc, a, ef, err, st);
 }
 
 cudaError_t launch_mhd_tma32(int phys, int stage, bool stretch, const Geo &g, const Coef<float> &co, const float *ia,
@@ -453,7 +480,8 @@ cudaError_t launch_mhd_tma32(int phys, int stage, bool stretch, const Geo &g, co
     } else if (stage == 4) {
         ef[0] = a.U0lo;
     }
-    return launch_mhd_any<float>(phys, stage, stretch, g, co, ia, corr2, dt, visc, a, a.X, ef, err, st);
+    return launch_mhd_any<float>(phys, stage, stretch, g, co, ia, corr2, dt, visc, a, ef, err, st);
 }
+#endif
 
 }  // namespace nova

@@ -31,6 +31,7 @@
 #include "nova_diag.cuh"
 #include "nova_internal.cuh"
 #include "nova_ops.cuh"
+#include "nova_parts.h"
 #include "nova_stage_math.cuh"
 #include "nova_tile.cuh"
 #include "nova_tma.cuh"
@@ -72,6 +73,73 @@ template <typename T> struct TmaCfg {
     static_assert(kRing >= 2 * kH + 1, "the queue and the plane computed fit in the ring");
     static_assert(TJ % kLRB == 0 && kLRB * 4 == kTK, "k-halo boxes share the component stride of the row boxes");
 };
+
+using EncodeFn = PFN_cuTensorMapEncodeTiled_v12000;
+
+EncodeFn encode_fn()
+{
+    static EncodeFn fn = []() -> EncodeFn {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            return nullptr;
+        return reinterpret_cast<EncodeFn>(p);
+    }();
+    return fn;
+}
+
+template <typename T> constexpr CUtensorMapDataType tmap_type()
+{
+    return sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+}
+
+// a 3-component field [c][i][j][k]; rows != 0: dims (k, c, j, i), box kTK x 3 x rows x 1;
+// rows == 0: dims (k, j, c, i), box 4 x kLRB x 3 x 1 (the k halos)
+template <typename T> bool encode(CUtensorMap *m, const T *base, const Geo &g, unsigned rows)
+{
+    EncodeFn fn = encode_fn();
+    if (!fn || !base) return false;
+    const cuuint64_t es = sizeof(T);
+    cuuint64_t dims[4], strides[3];
+    cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
+    if (rows) {
+        const cuuint64_t d[4] = {(cuuint64_t)g.N2, 3, (cuuint64_t)g.N1, (cuuint64_t)g.N0};
+        const cuuint64_t s[3] = {(cuuint64_t)g.N3 * es, (cuuint64_t)g.N2 * es, (cuuint64_t)g.N12 * es};
+        const cuuint32_t b[4] = {(cuuint32_t)kTK, 3, rows, 1};
+        memcpy(dims, d, sizeof d), memcpy(strides, s, sizeof s), memcpy(box, b, sizeof b);
+    } else {
+        const cuuint64_t d[4] = {(cuuint64_t)g.N2, (cuuint64_t)g.N1, 3, (cuuint64_t)g.N0};
+        const cuuint64_t s[3] = {(cuuint64_t)g.N2 * es, (cuuint64_t)g.N3 * es, (cuuint64_t)g.N12 * es};
+        const cuuint32_t b[4] = {4, (cuuint32_t)kLRB, 3, 1};
+        memcpy(dims, d, sizeof d), memcpy(strides, s, sizeof s), memcpy(box, b, sizeof b);
+    }
+    return fn(m, tmap_type<T>(), 4, const_cast<T *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <typename T> int tma_ichunk(const Geo &g)
+{
+    using C = TmaCfg<T>;
+    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + C::TJ - 1) / C::TJ);
+    return march_chunk(g.N0, tiles, C::kBlocksPerSM, 2.5, g.wallY ? 0.45 : 0.15);
+}
+
+}  // namespace
+
+// the kernels of one precision and mesh kind: a part of this source.  dpart: with
+// the diagnostics of the state the stage reads (FP64, uniform periodic whole-tile
+// meshes, stages 0 and 4)
+template <typename T, bool STRETCH, bool WALLS, bool WHOLE> struct StagePart {
+    using Args = std::conditional_t<sizeof(T) == 8, StageArgs64, StageArgs32>;
+    static cudaError_t launch(int stage, const Geo &g, const Coef<T> &co, const T *ia, const T *corr2, T dt, T visc,
+                              const Args &a, const T *const *ef, int *err, cudaStream_t st, const Walls<T> &wl,
+                              double *dpart);
+};
+
+#if NOVA_PART < 10
+namespace {
 
 // epilogue operands per stage, in load order
 //   FP64:  s=1,2,5: U0   s=3: U0, Y1, Y2
@@ -528,62 +596,9 @@ __global__ void __launch_bounds__(TmaCfg<T>::kThreads, TmaCfg<T>::kBlocksPerSM)
 }
 
 // ------------------------------------------------------------------ host --
-using EncodeFn = PFN_cuTensorMapEncodeTiled_v12000;
-
-EncodeFn encode_fn()
-{
-    static EncodeFn fn = []() -> EncodeFn {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            return nullptr;
-        return reinterpret_cast<EncodeFn>(p);
-    }();
-    return fn;
-}
-
-template <typename T> constexpr CUtensorMapDataType tmap_type()
-{
-    return sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-}
-
-// a 3-component field [c][i][j][k]; rows != 0: dims (k, c, j, i), box kTK x 3 x rows x 1;
-// rows == 0: dims (k, j, c, i), box 4 x kLRB x 3 x 1 (the k halos)
-template <typename T> bool encode(CUtensorMap *m, const T *base, const Geo &g, unsigned rows)
-{
-    EncodeFn fn = encode_fn();
-    if (!fn || !base) return false;
-    const cuuint64_t es = sizeof(T);
-    cuuint64_t dims[4], strides[3];
-    cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
-    if (rows) {
-        const cuuint64_t d[4] = {(cuuint64_t)g.N2, 3, (cuuint64_t)g.N1, (cuuint64_t)g.N0};
-        const cuuint64_t s[3] = {(cuuint64_t)g.N3 * es, (cuuint64_t)g.N2 * es, (cuuint64_t)g.N12 * es};
-        const cuuint32_t b[4] = {(cuuint32_t)kTK, 3, rows, 1};
-        memcpy(dims, d, sizeof d), memcpy(strides, s, sizeof s), memcpy(box, b, sizeof b);
-    } else {
-        const cuuint64_t d[4] = {(cuuint64_t)g.N2, (cuuint64_t)g.N1, 3, (cuuint64_t)g.N0};
-        const cuuint64_t s[3] = {(cuuint64_t)g.N2 * es, (cuuint64_t)g.N3 * es, (cuuint64_t)g.N12 * es};
-        const cuuint32_t b[4] = {4, (cuuint32_t)kLRB, 3, 1};
-        memcpy(dims, d, sizeof d), memcpy(strides, s, sizeof s), memcpy(box, b, sizeof b);
-    }
-    return fn(m, tmap_type<T>(), 4, const_cast<T *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-template <typename T> int tma_ichunk(const Geo &g)
-{
-    using C = TmaCfg<T>;
-    const long long tiles = (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + C::TJ - 1) / C::TJ);
-    return march_chunk(g.N0, tiles, C::kBlocksPerSM, 2.5, g.wallY ? 0.45 : 0.15);
-}
-
-template <typename T, int STAGE, bool STRETCH, class Args, bool DIAG = false, bool WALLS = false>
+template <typename T, int STAGE, bool STRETCH, class Args, bool DIAG, bool WALLS, bool WHOLE>
 cudaError_t launch_tma(const Geo &g, const Coef<T> &co, const T *ia, const T *corr2, T dt, T visc, const Args &a,
-                       const T *Y, const T *const *ef, int *err, cudaStream_t st, double *dpart = nullptr,
-                       const Walls<T> &wl = Walls<T>{})
+                       const T *Y, const T *const *ef, int *err, cudaStream_t st, double *dpart, const Walls<T> &wl)
 {
     constexpr int NE = epi_fields<T, STAGE>();
     StageMaps maps;
@@ -595,17 +610,14 @@ cudaError_t launch_tma(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     for (int f = 0; f < NE; f++) ok = ok && encode(&maps.e[f], ef[f], g, Cf::TJ);
     if (!ok) return cudaErrorInvalidValue;
     constexpr size_t smem = tma_smem_bytes<T, NE, DIAG>();
-    constexpr bool kW = sizeof(T) == 8 && !WALLS;  // has a whole-tile instantiation
-    const bool whole = kW && g.N2 % kTK == 0 && g.N1 % Cf::TJ == 0;
-    auto kern = whole ? k_stage_tma<T, STAGE, STRETCH, Args, DIAG, WALLS, kW>
-                      : k_stage_tma<T, STAGE, STRETCH, Args, DIAG, WALLS, DIAG>;
-    static bool attr[2] = {false, false};
-    if (!attr[whole]) {
+    auto kern = k_stage_tma<T, STAGE, STRETCH, Args, DIAG, WALLS, WHOLE>;
+    static bool attr = false;
+    if (!attr) {
         if constexpr (sizeof(T) == 8)
             if (const cudaError_t e = reg_split_ok(Split64{}, kern); e != cudaSuccess) return e;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        attr[whole] = true;
+        attr = true;
     }
     const int ch = tma_ichunk<T>(g);
     const dim3 grid((g.N2 + kTK - 1) / kTK, (g.N1 + Cf::TJ - 1) / Cf::TJ, (g.N0 + ch - 1) / ch);
@@ -614,30 +626,52 @@ cudaError_t launch_tma(const Geo &g, const Coef<T> &co, const T *ia, const T *co
     return cudaSuccess;
 }
 
-template <typename T, bool STRETCH, class Args, bool WALLS>
-cudaError_t launch_tma_stage_w(int stage, const Geo &g, const Coef<T> &co, const T *ia, const T *corr2, T dt, T visc,
-                               const Args &a, const T *const *ef, int *err, cudaStream_t st, const Walls<T> &wl)
+}  // namespace
+
+template <typename T, bool STRETCH, bool WALLS, bool WHOLE>
+cudaError_t StagePart<T, STRETCH, WALLS, WHOLE>::launch(int stage, const Geo &g, const Coef<T> &co, const T *ia,
+                                                        const T *corr2, T dt, T visc, const Args &a,
+                                                        const T *const *ef, int *err, cudaStream_t st,
+                                                        const Walls<T> &wl, double *dpart)
 {
+    if constexpr (sizeof(T) == 8 && !STRETCH && !WALLS && WHOLE)
+        if (dpart)
+            return stage == 0
+                       ? launch_tma<T, 0, false, Args, true, false, true>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, dpart, wl)
+                       : launch_tma<T, 4, false, Args, true, false, true>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, dpart, wl);
     switch (stage) {
-    case 0: return launch_tma<T, 0, STRETCH, Args, false, WALLS>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
-    case 1: return launch_tma<T, 1, STRETCH, Args, false, WALLS>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
-    case 2: return launch_tma<T, 2, STRETCH, Args, false, WALLS>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
-    case 3: return launch_tma<T, 3, STRETCH, Args, false, WALLS>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
-    case 5: return launch_tma<T, 5, STRETCH, Args, false, WALLS>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
-    default: return launch_tma<T, 4, STRETCH, Args, false, WALLS>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
+    case 0: return launch_tma<T, 0, STRETCH, Args, false, WALLS, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
+    case 1: return launch_tma<T, 1, STRETCH, Args, false, WALLS, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
+    case 2: return launch_tma<T, 2, STRETCH, Args, false, WALLS, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
+    case 3: return launch_tma<T, 3, STRETCH, Args, false, WALLS, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
+    case 5: return launch_tma<T, 5, STRETCH, Args, false, WALLS, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
+    default: return launch_tma<T, 4, STRETCH, Args, false, WALLS, WHOLE>(g, co, ia, corr2, dt, visc, a, a.Y, ef, err, st, nullptr, wl);
     }
 }
+
+// parts 0-5 FP64: periodic (uniform, stretched) x (ragged, whole), walls (uniform, stretched);
+// 6-9 FP32: (periodic, walls) x (uniform, stretched)
+#if NOVA_PART < 4
+template struct StagePart<double, NOVA_PART / 2 != 0, false, NOVA_PART % 2 != 0>;
+#elif NOVA_PART < 6
+template struct StagePart<double, NOVA_PART % 2 != 0, true, false>;
+#else
+template struct StagePart<float, NOVA_PART % 2 != 0, (NOVA_PART >= 8), false>;
+#endif
+#else
+namespace {
 
 template <typename T, class Args>
 cudaError_t launch_tma_stage(int stage, bool stretch, const Geo &g, const Coef<T> &co, const T *ia, const T *corr2,
                              T dt, T visc, const Args &a, const T *const *ef, int *err, cudaStream_t st,
-                             const Walls<T> &wl)
+                             const Walls<T> &wl, double *dpart)
 {
-    if (wl.on)
-        return stretch ? launch_tma_stage_w<T, true, Args, true>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl)
-                       : launch_tma_stage_w<T, false, Args, true>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl);
-    return stretch ? launch_tma_stage_w<T, true, Args, false>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl)
-                   : launch_tma_stage_w<T, false, Args, false>(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl);
+    constexpr bool kW = sizeof(T) == 8;  // has a whole-tile instantiation (periodic)
+    const bool whole = kW && g.N2 % kTK == 0 && g.N1 % TmaCfg<T>::TJ == 0;
+    const auto f = wl.on  ? (stretch ? StagePart<T, true, true, false>::launch : StagePart<T, false, true, false>::launch)
+                   : whole ? (stretch ? StagePart<T, true, false, kW>::launch : StagePart<T, false, false, kW>::launch)
+                           : (stretch ? StagePart<T, true, false, false>::launch : StagePart<T, false, false, false>::launch);
+    return f(stage, g, co, ia, corr2, dt, visc, a, ef, err, st, wl, dpart);
 }
 
 }  // namespace
@@ -669,17 +703,14 @@ cudaError_t launch_stage_tma64(int stage, bool stretch, const Geo &g, const Wall
             (long long)((g.N2 + kTK - 1) / kTK) * ((g.N1 + Cf::TJ - 1) / Cf::TJ) * ((g.N0 + ch - 1) / ch);
         if (nb <= dg->cap) {
             const cudaError_t e =
-                stage == 0 ? launch_tma<double, 0, false, StageArgs64, true>(g, co, ia, corr2, dt, visc, a, a.Y, ef,
-                                                                             err, st, dg->part)
-                           : launch_tma<double, 4, false, StageArgs64, true>(g, co, ia, corr2, dt, visc, a, a.Y, ef,
-                                                                             err, st, dg->part);
+                launch_tma_stage<double>(stage, stretch, g, co, ia, corr2, dt, visc, a, ef, err, st, wl, dg->part);
             if (e != cudaSuccess) return e;
             launch_diag_final(dg->part, (int)nb, dg->fin, dg->row, dg->flag, st);
             if (dg_done) *dg_done = true;
             return cudaSuccess;
         }
     }
-    return launch_tma_stage<double>(stage, stretch, g, co, ia, corr2, dt, visc, a, ef, err, st, wl);
+    return launch_tma_stage<double>(stage, stretch, g, co, ia, corr2, dt, visc, a, ef, err, st, wl, nullptr);
 }
 
 cudaError_t launch_stage_tma32(int stage, bool stretch, const Geo &g, const Walls<float> &wl, const Coef<float> &co,
@@ -700,7 +731,8 @@ cudaError_t launch_stage_tma32(int stage, bool stretch, const Geo &g, const Wall
         ef[0] = a.U0hi;
         ef[1] = a.U0lo;
     }
-    return launch_tma_stage<float>(stage, stretch, g, co, ia, corr2, dt, visc, a, ef, err, st, wl);
+    return launch_tma_stage<float>(stage, stretch, g, co, ia, corr2, dt, visc, a, ef, err, st, wl, nullptr);
 }
+#endif
 
 }  // namespace nova
