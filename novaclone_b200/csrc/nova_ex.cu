@@ -24,7 +24,7 @@ struct OpArgs {
     const double *ia, *corr2, *a, *b;
     double nu, *out;
     int ngrp, ichunk;  // component groups in grid.y, planes per chunk
-    int nc, symm;
+    int symm;
 };
 
 // sum_l w[l] (v(l + 1) - v(-l - 1))
@@ -287,7 +287,6 @@ void launch_op(int op, int h, const Geo &g, const Walls<double> &wa, const Walls
     A.b = b ? b : a;
     A.nu = nu;
     A.out = out;
-    A.nc = nc;
     A.ngrp = 1;
     switch (op) {
     case OP_GRAD_S: launch_nf<OP_GRAD_S>(h, A, st); break;

@@ -98,19 +98,17 @@ __global__ void __launch_bounds__(kThreads, (stage_minb<T, PHYS>())) k_stage(Geo
         e1p = kSplit5 ? args.U0lo : args.A;
     }
     T e0[3] = {0, 0, 0}, e1[3] = {0, 0, 0}, e2[3] = {0, 0, 0};
-    T e0n[3] = {0, 0, 0}, e1n[3] = {0, 0, 0}, e2n[3] = {0, 0, 0};
+    T e0n[3] = {0, 0, 0}, e1n[3] = {0, 0, 0};
     auto pre = [&](long long nidx, bool load) {
         if constexpr (kAhead) {
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 e0[c] = e0n[c];
                 e1[c] = e1n[c];
-                e2[c] = e2n[c];
                 if (load) {
                     const long long o = (long long)c * g.N3 + nidx;
                     if constexpr (kE0) e0n[c] = e0p[o];
                     if constexpr (kE1) e1n[c] = e1p[o];
-                    if constexpr (kE2) e2n[c] = e2p[o];
                 }
             }
         }

@@ -312,19 +312,7 @@ __global__ void __launch_bounds__(MhdCfg<T>::kThreads, 1)
         idx += g.N12;
         return true;
     };
-    using I0 = std::integral_constant<int, 0>;
-    using I1 = std::integral_constant<int, 1>;
-    using I2 = std::integral_constant<int, 2>;
-    using I3 = std::integral_constant<int, 3>;
-    using I4 = std::integral_constant<int, 4>;
-    using I5 = std::integral_constant<int, 5>;
-    using I6 = std::integral_constant<int, 6>;
-    for (int m = 0, p = 0; ok && p < nout; m++, p += kRing) {
-        ok = step(I0{}, m, p) && (p + 1 >= nout || (step(I1{}, m, p + 1) && (p + 2 >= nout ||
-             (step(I2{}, m, p + 2) && (p + 3 >= nout || (step(I3{}, m, p + 3) && (p + 4 >= nout ||
-             (step(I4{}, m, p + 4) && (p + 5 >= nout || (step(I5{}, m, p + 5) && (p + 6 >= nout ||
-             step(I6{}, m, p + 6))))))))))));
-    }
+    if (ok) ok = march_unrolled<kRing>(nout, step);
 }
 
 // ------------------------------------------------------------------ host --

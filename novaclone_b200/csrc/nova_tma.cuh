@@ -10,6 +10,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <type_traits>
 
 #include "nova_regsplit.h"
 
@@ -123,6 +124,24 @@ cudaError_t reg_split_ok(RegSplit<CONSUMERS, INC, PRODUCERS, DEC>, Kern kern)
     const cudaError_t e = cudaFuncGetAttributes(&at, kern);
     if (e != cudaSuccess) return e;
     return reg_split_fits(at.numRegs, CONSUMERS, INC, PRODUCERS, DEC) ? cudaSuccess : cudaErrorInvalidConfiguration;
+}
+
+// step(R, m, p) for the planes p = PERIOD m + R < n in order (R an integral_constant,
+// so that ring slots and queue positions are compile-time constants), until one
+// returns false
+template <int PERIOD, int R, class Step> __device__ __forceinline__ bool march_period(int n, int m, int p, Step &step)
+{
+    if (!step(std::integral_constant<int, R>{}, m, p + R)) return false;
+    if constexpr (R + 1 < PERIOD)
+        return p + R + 1 >= n || march_period<PERIOD, R + 1>(n, m, p, step);
+    else
+        return true;
+}
+template <int PERIOD, class Step> __device__ __forceinline__ bool march_unrolled(int n, Step &step)
+{
+    bool ok = true;
+    for (int m = 0, p = 0; ok && p < n; m++, p += PERIOD) ok = march_period<PERIOD, 0>(n, m, p, step);
+    return ok;
 }
 
 // 3-D tiled load (a single component of a field: dims k, j, i)
