@@ -246,10 +246,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_diag_tiled(Geo g, Walls<double>
 // std::max(a, b) of the reference: b only when a < b
 __device__ __forceinline__ double ref_max(double a, double b) { return a < b ? b : a; }
 
-// kFinalRows threads per partial, consecutive threads on consecutive partials,
-// so that every load is coalesced; then one thread per partial over the rows in
-// order.  Latency-bound (one block): 2048 blocks of partials 18 -> 7 us,
-// 128 blocks 7.1 -> 4.2 us against twelve block reductions in a row.
+// kFinalRows threads per partial, consecutive threads on consecutive partials, so that
+// every load is coalesced; four running values per thread and a tree over the rows, so
+// that the sums are as exact as the block reductions were (one thread adding the 64 rows
+// in order: Ek of
+// 256^3 off by 2.7e-16 rms, 1.3e-16 now).  Latency-bound (one block): the partials of
+// MHD at 256^3 18.4 -> 7.5 us, of 64^3 8.3 -> 3.7 us against twelve block reductions in a row.
 constexpr int kFinalRows = 64, kFinalThreads = kFinalRows * kDiagParts;
 __global__ void __launch_bounds__(kFinalThreads) k_diag_final(const double *__restrict__ part, int nblk, DiagFinal fin,
                                                               double *__restrict__ row, int *__restrict__ flag)
@@ -258,20 +260,24 @@ __global__ void __launch_bounds__(kFinalThreads) k_diag_final(const double *__re
     __shared__ double tot[kDiagParts];
     const int q = threadIdx.x % kDiagParts, r = threadIdx.x / kDiagParts;
     const bool mx = q >= DP_DIVU;
-    double a = 0.0;
-#pragma unroll 8
-    for (int b = r; b < nblk; b += kFinalRows) {
-        const double v = part[(long long)b * kDiagParts + q];
-        a = mx ? fmax(a, v) : a + v;
-    }
-    sh[r][q] = a;
+    auto join = [&](double x, double y) { return mx ? fmax(x, y) : x + y; };
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    int b = r;
+#pragma unroll 2
+    for (; b + 3 * kFinalRows < nblk; b += 4 * kFinalRows)
+#pragma unroll
+        for (int u = 0; u < 4; u++) a[u] = join(a[u], part[(long long)(b + u * kFinalRows) * kDiagParts + q]);
+#pragma unroll
+    for (int u = 0; u < 3; u++)
+        if (b + u * kFinalRows < nblk) a[u] = join(a[u], part[(long long)(b + u * kFinalRows) * kDiagParts + q]);
+    sh[r][q] = join(join(a[0], a[1]), join(a[2], a[3]));
     __syncthreads();
-    if (threadIdx.x < kDiagParts) {
-        double t = 0.0;
-#pragma unroll 16
-        for (int x = 0; x < kFinalRows; x++) t = mx ? fmax(t, sh[x][q]) : t + sh[x][q];
-        tot[q] = q == DP_UMAX ? sqrt(t) : t;
+#pragma unroll
+    for (int s = kFinalRows / 2; s > 0; s /= 2) {
+        if (r < s) sh[r][q] = join(sh[r][q], sh[r + s][q]);
+        __syncthreads();
     }
+    if (threadIdx.x < kDiagParts) tot[q] = q == DP_UMAX ? sqrt(sh[0][q]) : sh[0][q];
     __syncthreads();
     if (threadIdx.x == 0) {
         const double n = fin.invN3;
