@@ -409,19 +409,21 @@ nova_status ensure_fft(nova_ctx *ctx, bool split)
     int cembed3[3] = {g.N0, ny, g.N2 / 2 + 1}, cembed2[2] = {ny, g.N2 / 2 + 1};
     int *n = pi ? n2d : n3d, *rembed = pi ? rembed2 : rembed3, *cembed = pi ? cembed2 : cembed3;
     const int rdist = (pi ? 1 : g.N0) * g.N1 * g.N2, cdist = (pi ? 1 : g.N0) * ny * (g.N2 / 2 + 1);
-    s = fft_plan(ctx, "cufftPlanMany D2Z", [&] {
-        return cufftPlanMany(&F.f, rank, n, rembed, 1, rdist, cembed, 1, cdist, CUFFT_D2Z, batch);
-    });
-    if (s != NOVA_OK)
-        return s;
-    s = fft_plan(ctx, "cufftPlanMany Z2D", [&] {
-        return cufftPlanMany(&F.b, rank, n, cembed, 1, cdist, rembed, 1, rdist, CUFFT_Z2D, batch);
-    });
-    if (s != NOVA_OK) {
-        cufftDestroy(F.f);
-        return s;
+    if (!F.plans) {
+        s = fft_plan(ctx, "cufftPlanMany D2Z", [&] {
+            return cufftPlanMany(&F.f, rank, n, rembed, 1, rdist, cembed, 1, cdist, CUFFT_D2Z, batch);
+        });
+        if (s != NOVA_OK)
+            return s;
+        s = fft_plan(ctx, "cufftPlanMany Z2D", [&] {
+            return cufftPlanMany(&F.b, rank, n, cembed, 1, cdist, rembed, 1, rdist, CUFFT_Z2D, batch);
+        });
+        if (s != NOVA_OK) {
+            cufftDestroy(F.f);
+            return s;
+        }
+        F.plans = true;
     }
-    F.plans = true;
     F.pois_i = pi;
     if ((s = dalloc(ctx, (double **)&ctx->d_spec, 2 * nspec)) != NOVA_OK) return s;
     if ((s = dalloc(ctx, &ctx->d_rhs, (size_t)g.N3)) != NOVA_OK) return s;
@@ -604,6 +606,8 @@ nova_status poisson_device_dct(nova_ctx *ctx, const double *rhs, double *p, bool
             return s;
         }
         ctx->dct_plans = true;
+    }
+    if (!ctx->d_ky2e || !ctx->d_spec2 || !ctx->d_ext) {  // (a call that ran out of memory here may be repeated)
         const size_t next = (size_t)g.N0 * 2 * ny * g.N2;
         if ((s = dalloc(ctx, &ctx->d_ext, next)) != NOVA_OK) return s;
         if ((s = dalloc(ctx, (double **)&ctx->d_spec2, 2 * (size_t)g.N0 * 2 * ny * (g.N2 / 2 + 1))) != NOVA_OK) return s;

@@ -66,3 +66,39 @@ def test_plan_work_area(nova):
         e.solve()
     assert np.array_equal(q.download_soa(), want)
     A.close()
+
+
+def test_wall_solve_repeated_after_running_out(nova):
+    """The even-extension solve's buffers follow its plans: a call that found no room for
+    them and is repeated allocates them then (the state is uploaded again: the stages
+    of the failed call have run)."""
+    N = (200, 250, 200)
+    U0 = 0.1 * np.random.default_rng(9).standard_normal((3, N[0], N[1] + 1, N[2]))
+
+    def setup():
+        M = nova.Mesh(N, walls=(0, 1, 0))
+        U, p = nova.Field(M, 3), nova.Field(M, 1).set_bc([1, 1] + [0] * 16)
+
+        def run(poisson):
+            U.upload_soa(U0)
+            nova.advance(M, nova.run_desc(dt=1e-4, nu=1e-2, poisson=poisson), U, p, nsteps=1, history=False)
+        run("fft")  # the kernels are loaded, the other buffers and plans are there
+        return M, U, run
+    M, U, run = setup()
+    run("dct")
+    want = U.download_soa()
+    U.close()
+    M.close()
+    M, U, run = setup()
+    short = 0
+    for mib in range(64, 1024, 96):  # two plans, then two buffers of 160 MB
+        with only(mib << 20):
+            try:
+                run("dct")
+                break
+            except nova.NovaError as e:
+                assert e.status in (nova.E_OOM, nova.E_CUDA)  # cuFFT reports its own as an internal error
+                short += 1
+    assert short > 2
+    run("dct")
+    assert np.array_equal(U.download_soa(), want)
