@@ -550,9 +550,9 @@ SHEAR_STEP_BYTES = {k: 4 * (v + 32 + 48 + 56) for k, v in SHEAR_STAGE_BYTES.item
 #   writing U*; projection; classical B loop with U frozen: 72, 96, 96, 144
 #   FP64 / 48, 72, 72, 84 split; cleaning projection)
 JET_STEP_BYTES = {"f64": 72 + 120 + 72 + 96 + 96 + 144 + 120, "f32split": 60 + 120 + 48 + 72 + 72 + 84 + 120}
-#   weakly compressible: 5 evolved components at 104 B each (RK stages
-#   16, 24, 24, 40)
-WC_STEP_BYTES = 5 * 104.0
+#   weakly compressible: U and rho without an accumulator, 104 B per component
+#   (RK stages 16, 24, 24, 40), T with one, 136 B
+WC_STEP_BYTES = 4 * 104.0 + 136.0
 
 
 def shear_leg(args, nova, torch, dist, world):
@@ -593,8 +593,7 @@ def shear_leg(args, nova, torch, dist, world):
                           "roofline": hbm_roof(SHEAR_STEP_BYTES[prec_name] * npts * steps, sec,
                                                "whole step, %g B/point-step" % SHEAR_STEP_BYTES[prec_name]),
                           "stage_kernel": hbm_roof(SHEAR_STAGE_BYTES[prec_name] * npts * st_n, st_ms / 1e3,
-                                                   "shear-loop stage kernel (walls; FP64 on the march, split on "
-                                                   "the TMA pipeline), %g B/point" % SHEAR_STAGE_BYTES[prec_name])}
+                                                   "shear-loop stage kernel (walls, TMA pipeline), %g B/point" % SHEAR_STAGE_BYTES[prec_name])}
         finals[prec_name] = U.download_soa()
         U.close()
         p.close()

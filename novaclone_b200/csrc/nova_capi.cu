@@ -69,7 +69,9 @@ struct nova_ctx {
     // the scale (k_pois_i) between transforms of the (j, k) planes, by the
     // library's own line kernels where N1 and N2/2 are such lengths too
     // (own_jk), else by batched 2-D cuFFT plans; other N0: 3-D cuFFT plans and
-    // k_scale.  Split: the plans only (batched 2-D around k_pois_i for N0 = 64
+    // k_scale.  (Line kernels: 1.1-1.8 times the plans' rate; the batched plans
+    // around k_pois_i against a 3-D plan on 28 meshes: 1.01-1.27 times, e.g.
+    // 240 x 250 x 260 566 -> 482 us, 96 x 77 x 110 78 -> 68.)  Split: the plans only (batched 2-D around k_pois_i for N0 = 64
     // and 256 on periodic meshes, else 3-D), so that a split run's results do
     // not depend on which transform the FP64 side uses: U is rounded to the
     // (hi, lo) pair after the correction, and a solve that rounds differently
@@ -445,7 +447,7 @@ nova_status stage_fail(nova_ctx *ctx, cudaError_t e)
 {
     if (e == cudaErrorNotSupported)
         return fail(ctx, NOVA_E_UNSUPPORTED,
-                    "NOVA_STAGE_IMPL=tma: the TMA stage kernel needs N2 >= 32 with whole 16-byte rows and no one or two columns beyond a 32-column tile, and N1 at least twice the tile height (16 rows FP64, 8 FP32) with, for periodic y, no one or two rows beyond a tile; walls in y only in FP32");
+                    "NOVA_STAGE_IMPL=tma: the TMA stage kernel needs N2 >= 32 with whole 16-byte rows and no one or two columns beyond a 32-column tile, and N1 at least twice the tile height (16 rows FP64, 8 FP32; MHD 8 and 16) with, for periodic y, no one or two rows beyond a tile; FP64 stages between walls run it by default only, forcing it is refused");
     if (e == cudaErrorInvalidValue) return fail(ctx, NOVA_E_CUDA, "stage kernel: cuTensorMapEncodeTiled failed");
     if (e == cudaErrorInvalidConfiguration)
         return fail(ctx, NOVA_E_CUDA, "stage kernel: compiled with too few registers for its register split");

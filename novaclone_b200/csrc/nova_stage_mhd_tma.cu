@@ -16,7 +16,7 @@
 //
 // FP64: TJ = 8 (a slot of the two fields is 24 KB, 209 KB with the epilogue
 // ring; one block per SM, 8 consumer warps of 232 registers); FP32:
-// TJ = 16 (20 KB slots, 195 KB; one block of 17 warps).
+// TJ = 16 (20 KB slots, 195 KB; one block of 20 warps, 16 consumers of 112 registers).
 #include "nova_internal.cuh"
 #include "nova_parts.h"
 #include "nova_stage_math.cuh"
