@@ -75,7 +75,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(r.stdout.decode())
             raise RuntimeError("nvcc failed: " + " ".join(cmd))
     jobs = list(_jobs(force))
-    with ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+    with ThreadPoolExecutor(min(os.cpu_count() or 1, 16)) as pool:  # about 1 GB each
         list(pool.map(compile, [cmd for _, cmd in jobs if cmd]))
     objs = [o for o, _ in jobs]
     if force or _newer(LIB, objs):

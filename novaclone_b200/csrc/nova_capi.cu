@@ -871,10 +871,8 @@ extern "C" nova_status nova_field_destroy(nova_ctx *ctx, nova_field *f)
     // a field that only its owner used has all its work on the owner's stream;
     // any other may have it on any stream, and the next field that gets the
     // buffer is ordered behind the owner's alone
-    if (ctx && ctx == f->owner && !__atomic_load_n(&f->shared, __ATOMIC_RELAXED))
-        cudaStreamSynchronize(ctx->stream);
-    else
-        cudaDeviceSynchronize();
+    const bool own = ctx && ctx == f->owner && !__atomic_load_n(&f->shared, __ATOMIC_RELAXED);
+    if (!own || cudaStreamSynchronize(ctx->stream) != cudaSuccess) cudaDeviceSynchronize();
     const size_t n = (size_t)f->nc * f->n3;
     f->home->put(f->d64, sizeof(double) * n);
     f->home->put(f->hi, sizeof(float) * n);
